@@ -185,6 +185,7 @@ struct NlData {
   std::vector<double> ch_vn;        // vnorm / vol per channel
   double2* dyp = nullptr;           // [nchan][npts] projector b(G) Ylm v_l(g)
   int *line_zneg = nullptr, *line_zpos = nullptr, *line_xy = nullptr;  // NL-grid lines
+  int grid_ready = 0;               // the NL-grid path's scratch below is allocated
   void *pen_a = nullptr, *pen_b = nullptr;  // [nstates][nkf][nlpad]
   void* tw = nullptr;               // [nkf] twiddles, working precision
   StateFftOps ops;
@@ -236,6 +237,12 @@ struct NlData {
   double* zt = nullptr;             // scaled Z of two types, [nstates][ldz] each
   size_t zt_slot = 0;               // doubles per type
   int gspace_ok = 0;                // every type has at most 4 channels
+  // FP64 contexts, the G-space pass of ees64.cu: atoms with projectors in type
+  // order, Z partials of the K splits, zs in both layouts, energy and atom-force
+  // partials
+  int gspace64 = 0, e64_na = 0, e64_split = 1, e64_nblk = 1;
+  int* e64_act = nullptr;
+  double *e64_part = nullptr, *e64_zs = nullptr, *e64_e = nullptr, *e64_f = nullptr;
 };
 
 // EES form of the Hartree + local + Ewald pass (cpstep_set_local_ees, the
@@ -392,8 +399,8 @@ struct cpstep_ctx {
     int plane_waves = 3;  // state plane passes: blocks ~ plane_waves x SMs
     int nl_blocks = 6;    // EES plane kernels: blocks ~ nl_blocks x SMs
     int pc_split = 1;     // PairCalc overlap split-K: CTAs ~ pc_split x SMs
-    int ees_gspace = 1;   // mixed contexts on the tensor cores: EES in G space (1) or
-                          // through the NL-grid FFTs (0)
+    int ees_gspace = 1;   // EES in G space where it is built and faster (1: FP64 contexts and
+                          // mixed ones on the tensor cores) or through the NL-grid FFTs (0)
   } tune;
   int use_graph = 1;
   int graph_warm = 0;              // a direct step with gkey ran
@@ -448,6 +455,12 @@ int sf_run(cpstep_ctx* c, const double* psi, const double* occ, double* fpsi, do
            double* fatm);
 int nl_run(cpstep_ctx* c, const double* psi, const double* occ, double* fpsi, double* energies,
            double* fatm);
+int nl_grid_reserve(cpstep_ctx* c);
+// ees64.cu: the same pass of an FP64 context in G space
+int ees64_set(cpstep_ctx* c, const std::vector<int>& order);
+bool ees64_faster(const cpstep_ctx* c);
+int ees64_run(cpstep_ctx* c, const double* psi, double* fpsi, const double* occ, double* energies,
+              double* fatm);
 int nl_grid_size(int kmax, double scale, int n_interp);
 int eext_grid_size(int kmax, double scale, int n_interp);
 // eesAtmBsplineRgrp's indices, Mn and dMn of every atom on an nkf grid

@@ -548,7 +548,55 @@ void nl_free(cpstep_ctx* c) {
   n.sep = nullptr; n.sv = nullptr; n.d_order = nullptr; n.d_tch = nullptr; n.d_vn = nullptr;
   n.csum = nullptr; n.zt = nullptr; n.gspace_ok = 0;
   cudaFree(n.plist); cudaFree(n.pcount);
+  cudaFree(n.e64_act); cudaFree(n.e64_part); cudaFree(n.e64_zs); cudaFree(n.e64_e);
+  cudaFree(n.e64_f);
   n = NlData();
+}
+
+// Scratch of the NL-grid path (pencils, twiddles, stencil tables), allocated
+// when that path is first chosen: an FP64 context whose pass runs in G space
+// never needs it.
+int nl_grid_reserve(cpstep_ctx* c) {
+  NlData& n = c->nl;
+  if (!n.on || n.grid_ready) return CPSTEP_OK;
+  const AtomData& at = c->atoms;
+  const int nkf = n.nkf;
+  const bool fp64 = c->precision == CPSTEP_PREC_FP64;
+  const size_t na = (size_t)n.natm, csz = fp64 ? sizeof(cplx<double>) : sizeof(cplx<float>);
+  const size_t pen = (size_t)c->nstates * nkf * c->nlpad * csz;
+  // stencil tables: 64 entries per atom of the type on each plane at most
+  n.tab_cap.assign(at.ntyp, 0);
+  n.tab_off.assign(at.ntyp, 0);
+  size_t tot = 0;
+  for (int t = 0; t < at.ntyp; ++t) {
+    n.tab_off[t] = tot;
+    n.tab_cap[t] = 64 * (at.tstart[t + 1] - at.tstart[t]);
+    tot += (size_t)nkf * n.tab_cap[t];
+  }
+  const size_t tot1 = std::max<size_t>(tot, 1);
+  auto get = [](auto** p, size_t bytes) -> int {  // kept from an earlier call that failed later
+    if (!*p) CPSTEP_CUDA_TRY(cudaMalloc(p, bytes));
+    return CPSTEP_OK;
+  };
+  int rc = CPSTEP_OK;
+  if (!n.tw) rc = fp64 ? upload_tw_n<double>(nkf, &n.tw) : upload_tw_n<float>(nkf, &n.tw);
+  if (rc || (rc = get(&n.pen_a, pen)) || (rc = get(&n.pen_b, pen)) ||
+      (rc = get(&n.plist, sizeof(int) * (size_t)at.ntyp * nkf * na)) ||
+      (rc = get(&n.pcount, sizeof(int) * (size_t)at.ntyp * nkf)) ||
+      (rc = get(&n.zpart, sizeof(double) * c->nstates * na * kNlInterp * 4)) ||
+      (rc = get(&n.zs, sizeof(double) * c->nstates * na)) ||
+      (rc = get(&n.tcell, sizeof(int) * tot1)) || (rc = get(&n.tval, sizeof(NlVal) * tot1)) ||
+      (rc = get(&n.gcell, sizeof(int) * tot1)) || (rc = get(&n.gent, sizeof(int) * tot1)) ||
+      (rc = get(&n.goff, sizeof(int) * (tot + (size_t)at.ntyp * nkf))) ||
+      (rc = get(&n.gcount, sizeof(int) * (size_t)at.ntyp * nkf)))
+    return rc;
+  n.grid_ready = 1;
+  return CPSTEP_OK;
+}
+
+// whether an FP64 context's pass runs in G space (ees64.cu)
+static bool nl_g64(const cpstep_ctx* c) {
+  return c->nl.gspace64 && c->tune.ees_gspace && ees64_faster(c);
 }
 
 int nl_set(cpstep_ctx* c, int nkf, int n_interp, int nchan, const int* ch_type, const int* ch_l,
@@ -691,37 +739,12 @@ int nl_set(cpstep_ctx* c, int nkf, int n_interp, int nchan, const int* ch_type, 
   CPSTEP_CUDA_TRY(cudaMemcpy(n.dyp, dyp.data(), sizeof(double2) * dyp.size(),
                              cudaMemcpyHostToDevice));
   const bool fp64 = c->precision == CPSTEP_PREC_FP64;
-  if ((rc = fp64 ? upload_tw_n<double>(nkf, &n.tw) : upload_tw_n<float>(nkf, &n.tw))) return rc;
-  const size_t csz = fp64 ? sizeof(cplx<double>) : sizeof(cplx<float>);
-  const size_t pen = (size_t)c->nstates * nkf * c->nlpad * csz;
-  CPSTEP_CUDA_TRY(cudaMalloc(&n.pen_a, pen));
-  CPSTEP_CUDA_TRY(cudaMalloc(&n.pen_b, pen));
   const size_t na = (size_t)at.natm;
   CPSTEP_CUDA_TRY(cudaMalloc(&n.ig, sizeof(int) * na * 3 * kNlInterp));
   CPSTEP_CUDA_TRY(cudaMalloc(&n.mn, sizeof(double) * na * 3 * kNlInterp));
   CPSTEP_CUDA_TRY(cudaMalloc(&n.dmn, sizeof(double) * na * 3 * kNlInterp));
-  CPSTEP_CUDA_TRY(cudaMalloc(&n.plist, sizeof(int) * (size_t)at.ntyp * nkf * na));
-  CPSTEP_CUDA_TRY(cudaMalloc(&n.pcount, sizeof(int) * (size_t)at.ntyp * nkf));
-  CPSTEP_CUDA_TRY(cudaMalloc(&n.zpart, sizeof(double) * c->nstates * na * kNlInterp * 4));
-  CPSTEP_CUDA_TRY(cudaMalloc(&n.zs, sizeof(double) * c->nstates * na));
   CPSTEP_CUDA_TRY(cudaMalloc(&n.enl_s, sizeof(double) * c->nstates));
   CPSTEP_CUDA_TRY(cudaMalloc(&n.fnl, sizeof(double) * c->nstates * na * 3));
-  // stencil tables: 64 entries per atom of the type on each plane at most
-  n.tab_cap.assign(at.ntyp, 0);
-  n.tab_off.assign(at.ntyp, 0);
-  size_t tot = 0;
-  for (int t = 0; t < at.ntyp; ++t) {
-    n.tab_off[t] = tot;
-    n.tab_cap[t] = 64 * (at.tstart[t + 1] - at.tstart[t]);
-    tot += (size_t)nkf * n.tab_cap[t];
-  }
-  const size_t tot1 = std::max<size_t>(tot, 1);
-  CPSTEP_CUDA_TRY(cudaMalloc(&n.tcell, sizeof(int) * tot1));
-  CPSTEP_CUDA_TRY(cudaMalloc(&n.tval, sizeof(NlVal) * tot1));
-  CPSTEP_CUDA_TRY(cudaMalloc(&n.gcell, sizeof(int) * tot1));
-  CPSTEP_CUDA_TRY(cudaMalloc(&n.gent, sizeof(int) * tot1));
-  CPSTEP_CUDA_TRY(cudaMalloc(&n.goff, sizeof(int) * (tot + (size_t)at.ntyp * nkf)));
-  CPSTEP_CUDA_TRY(cudaMalloc(&n.gcount, sizeof(int) * (size_t)at.ntyp * nkf));
   // G-space form (mixed contexts): channels per type, S matrices, scratch
   n.km = km;
   n.tch.assign(at.ntyp, {});
@@ -816,7 +839,25 @@ int nl_set(cpstep_ctx* c, int nkf, int n_interp, int nchan, const int* ch_type, 
     CPSTEP_CUDA_TRY(cudaMemcpy(n.d_order, horder.data(), sizeof(int) * na,
                                cudaMemcpyHostToDevice));
   }
+  if (fp64) {
+    std::vector<int> hrank(na), horder(na);
+    CPSTEP_CUDA_TRY(cudaMemcpy(hrank.data(), at.rank, sizeof(int) * na, cudaMemcpyDeviceToHost));
+    for (int a = 0; a < (int)na; ++a) horder[hrank[a]] = a;
+    if ((rc = ees64_set(c, horder))) return rc;
+  }
   n.on = 1;
+  if (!nl_g64(c) && (rc = nl_grid_reserve(c))) n.on = 0;
+  return rc;
+}
+
+// B-spline factors of the atoms and their separable transforms (n.sep)
+static int ees_sep_run(cpstep_ctx* c) {
+  NlData& n = c->nl;
+  if (int rc = ees_bspline_launch(c, c->atoms.frac, n.natm, n.nkf, n.ig, n.mn, n.dmn)) return rc;
+  const long long nsep = (long long)n.natm * 6 * (2 * n.km + 1);
+  ees::k_ees_sep<<<(unsigned)((nsep + 255) / 256), 256, 0, c->stream>>>(n.ig, n.mn, n.dmn, n.natm,
+                                                                         n.nkf, n.km, n.sep);
+  CPSTEP_LAUNCH_CHECK();
   return CPSTEP_OK;
 }
 
@@ -827,13 +868,7 @@ static int ees_gspace_run(cpstep_ctx* c, const double* psi, const double* occ, d
                           double* energies, double* fatm) {
   NlData& n = c->nl;
   const int S = c->nstates, natm = n.natm, ntyp = c->atoms.ntyp;
-  ees::k_nl_bspline<<<cdiv(natm, 128), 128, 0, c->stream>>>(c->atoms.frac, natm, n.nkf, n.ig,
-                                                            n.mn, n.dmn);
-  CPSTEP_LAUNCH_CHECK();
-  const long long nsep = (long long)natm * 6 * (2 * n.km + 1);
-  ees::k_ees_sep<<<(unsigned)((nsep + 255) / 256), 256, 0, c->stream>>>(n.ig, n.mn, n.dmn, natm,
-                                                                         n.nkf, n.km, n.sep);
-  CPSTEP_LAUNCH_CHECK();
+  if (int rc = ees_sep_run(c)) return rc;
   ees::TypeDims td{};
   for (int t = 0; t <= ntyp; ++t) td.tstart[t] = c->atoms.tstart[t];
   for (int t = 0; t < ntyp; ++t) {
@@ -919,6 +954,11 @@ int nl_run(cpstep_ctx* c, const double* psi, const double* occ, double* fpsi, do
   }
   if (n.gspace_ok && c->precision == CPSTEP_PREC_MIXED && c->tc_ok && c->tune.ees_gspace)
     return ees_gspace_run(c, psi, occ, fpsi, energies, fatm);
+  if (nl_g64(c)) {
+    if (int rc = ees_sep_run(c)) return rc;
+    return ees64_run(c, psi, fpsi, occ, energies, fatm);
+  }
+  if (int rc = nl_grid_reserve(c)) return rc;
   const int S = c->nstates, natm = n.natm;
   ees::k_nl_bspline<<<cdiv(natm, 128), 128, 0, c->stream>>>(c->atoms.frac, natm, n.nkf, n.ig,
                                                             n.mn, n.dmn);

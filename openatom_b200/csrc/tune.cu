@@ -99,7 +99,8 @@ int cpstep_tune_set(cpstep_ctx* c, const int* vals, int n) {
   c->tune.pc_split = vals[3];
   c->tc_ok = vals[4];
   c->tune.ees_gspace = vals[5];
-  return CPSTEP_OK;
+  // the NL-grid path may run from here on: its scratch before any capture
+  return vals[5] ? CPSTEP_OK : nl_grid_reserve(c);
 }
 
 int cpstep_autotune(cpstep_ctx* c, const double* d_psi, const double* d_occ, double* ms_out) {

@@ -150,3 +150,43 @@ def test_mixed_step_with_nonlocal(nlsys, nlstep):
     assert ok
     assert abs(e[8] - er["ETOT"]) / natm <= 1e-6
     assert np.max(np.abs(f - fr)) <= 1e-5
+
+
+@pytest.mark.parametrize("states,atoms,keep", [
+    (1, {"O": 1, "H": 2}, None), (31, {"O": 3, "H": 5}, None), (33, {"O": 11, "H": 22}, None),
+    (65, {"O": 2, "H": 3}, (1, 0)), (130, {"O": 9, "H": 0}, None), (64, {"O": 16, "H": 17}, (0, 0))])
+def test_fp64_gspace_matches_grid_form(states, atoms, keep):
+    """FP64 contexts: the G-space products against the NL-grid transforms at the
+    edges of their tiles (32, 64, 128 states; 32 atoms; a ragged last point
+    tile), with a type without channels or with one only, and forces added to
+    what is there.  Both are FP64 sums of the same terms: 1e-11 of the largest
+    entry."""
+    if not cuda_ok():
+        pytest.skip("no CUDA device")
+    import torch
+    from openatom_b200.context import StepContext
+    from openatom_b200.system import System
+    s = System(12.0, 25.0, states, {k: n for k, n in atoms.items() if n}, nfft=40, seed=5)
+    if keep is not None:  # (type, l) of the one channel kept
+        s.channels = [c for c in s.channels if (c["type"], c["l"]) == keep]
+    g = torch.Generator(device="cuda").manual_seed(states)
+    psi = torch.view_as_complex(torch.randn((states, s.layout.npts, 2), generator=g,
+                                            dtype=torch.float64, device="cuda"))
+    f0 = 0.1 * psi.flip(0).contiguous()
+    occ = 1.0 + torch.arange(states, dtype=torch.float64, device="cuda") % 2
+    out = []
+    for form in (1, 0):
+        ctx = StepContext(s.layout, states, precision="fp64")
+        try:
+            ctx.set_atoms(s)
+            ctx.set_nonlocal(s)
+            ctx.tune_set({"ees_gspace": form})
+            f, e, fa = ctx.ees_nonlocal(psi, occ, fpsi=f0.clone())
+            out.append((e[7:8].cpu().numpy(), f.cpu().numpy(), fa.cpu().numpy()))
+            f2, e2, _ = ctx.ees_nonlocal(psi, occ, fpsi=f0.clone(), forces=False)
+            assert bool((f2 == f).all()) and bool((e2[7] == e[7]).all())
+        finally:
+            ctx.close()
+    for a, b in zip(*out):
+        assert np.max(np.abs(b)) > 0.0
+        assert np.max(np.abs(a - b)) <= 1e-11 * np.max(np.abs(b))
