@@ -1,4 +1,4 @@
-// PairCalculator products (FP64 SIMT path; the mixed-precision context sends
+// PairCalculator products (FP64 path; the mixed-precision context sends
 // them to the tensor-core kernels of paircalc_tc.cu where those apply).
 //
 //   overlap:      C(i,j) = alpha * sum_p wpt_p Re(conj a_i(p) b_j(p)) (+ beta C)
@@ -12,13 +12,14 @@
 //   dgemm:        column-major BLAS semantics, the myGEMM wrapper
 //                 (ckPairCalculator.C:57-66).
 //
-// All three run on FP64 SIMT tiles; the overlap is split over K (the
+// The first two run on the FP64 tensor units, dgemm on FP64 SIMT tiles; the overlap is split over K (the
 // reference's numChunks K-split, pcCommManager.C:165-172) with a fixed-order
 // reduction of the partial tiles, so results are deterministic.
 #include <algorithm>
 #include <mutex>
 #include <cuda.h>
 #include "ctx.cuh"
+#include "dmma.cuh"
 
 namespace pcalc {
 
@@ -174,208 +175,227 @@ k_dgemm(int ta, int tb, int m, int n, int k, double alpha, const double* __restr
 }
 
 // ---------------------------------------------------------------------------
-// 128 x 128 block tiles: 256 threads, 8 x 8 outputs each (rows ty + 16 i,
-// columns tx + 16 j), K chunks of 16 staged through registers into two
-// shared buffers so the global loads of chunk k+1 overlap the FMAs of chunk k.
-constexpr int TB = 128, TK = 16, TLD = TB + 1;
-constexpr size_t T128_SMEM = sizeof(double) * 4 * TK * TLD;  // two operands, two buffers
+// FP64 products on the FP64 tensor units (dmma.cuh).  A block holds WM x WN
+// warps of 32 x 32 outputs; 32-real chunks of both operands come in by cp.async
+// into two stages, one barrier per chunk.  Blocks of 4 x 4 warps take one SM
+// each (164 KB); sizes that fit 64 rows run blocks of 2 x 2 (overlap) or 2 x 4
+// and 1 x 4 warps (back-multiply), whose padding costs less.  128 states, 65,736
+// points: lambda and S 281 us each on FP64 FMAs (15 TFLOP/s) -> 130 us (33
+// TFLOP/s; S's lower half is not formed), a back-multiply 293 -> 195 us (22
+// TFLOP/s: four chunks per tile, whose epilogue is not overlapped).
 
-// C_part[ks] = A[i0:i0+128, kslab] B[j0:j0+128, kslab]^T (A, B row-major [rows][K],
-// K in reals; w per complex point scales A).  Column-major partial tiles, ld = M.
-__global__ void __launch_bounds__(256, 1)
-k_overlap_t128(const double* __restrict__ A, int lda, const double* __restrict__ B, int ldb,
-               const double* __restrict__ w, int M, int N, int K, int kslab,
-               double* __restrict__ part) {
-  extern __shared__ __align__(16) double t128_smem[];
-  double (*As)[TK][TLD] = reinterpret_cast<double (*)[TK][TLD]>(t128_smem);
-  double (*Bs)[TK][TLD] = reinterpret_cast<double (*)[TK][TLD]>(t128_smem + 2 * TK * TLD);
-  const int i0 = blockIdx.x * TB, j0 = blockIdx.y * TB, ks = blockIdx.z;
-  const int kbeg = ks * kslab, kend = min(K, kbeg + kslab);
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  double acc[8][8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = 0.0;
-  // loader: 4 double2 of A and of B per thread (row = idx / 8, k pair = idx % 8)
-  double2 ra[4], rb[4];
-  auto load = [&](int k0) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int idx = threadIdx.x + 256 * q;
-      const int row = idx >> 3, kp = idx & 7;
-      const int k = k0 + 2 * kp;
-      double2 va = make_double2(0.0, 0.0), vb = make_double2(0.0, 0.0);
-      if (k < kend) {  // kend and k are even: the pair is inside
-        if (i0 + row < M) {
-          va = *reinterpret_cast<const double2*>(A + (size_t)(i0 + row) * lda + k);
-          if (w) {
-            const double sw = w[k >> 1];
-            va.x *= sw;
-            va.y *= sw;
-          }
-        }
-        if (j0 + row < N) vb = *reinterpret_cast<const double2*>(B + (size_t)(j0 + row) * ldb + k);
+template <int WM, int WN>
+struct OvlCfg {
+  static constexpr int TM = 32 * WM, TN = 32 * WN, THREADS = 32 * WM * WN;
+  static constexpr size_t SMEM = sizeof(double) * 2 * dm::LDK * (TM + TN);
+};
+
+// C_part[ks] = A B^T over the split's chunks of 32 reals (A, B row-major
+// [rows][K], K even; w per complex point scales A).  sym (A == B, M == N): only
+// the tiles and, in a diagonal tile, the warp blocks on and above the diagonal
+// are formed and written to both halves; a diagonal tile has one operand.
+template <int WM, int WN>
+__global__ void __launch_bounds__(OvlCfg<WM, WN>::THREADS)
+k_overlap(const double* __restrict__ A, const double* __restrict__ B,
+          const double* __restrict__ w, int M, int N, int K, int sym, int tn,
+          double* __restrict__ part) {
+  using C = OvlCfg<WM, WN>;
+  extern __shared__ __align__(16) double sm[];
+  double* As = sm;
+  double* Bs = sm + 2 * C::TM * dm::LDK;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  int ti, tj;
+  if (sym) {  // blockIdx.x counts the tiles ti <= tj by rows
+    int r = blockIdx.x;
+    ti = 0;
+    while (r >= tn - ti) {
+      r -= tn - ti;
+      ++ti;
+    }
+    tj = ti + r;
+  } else {
+    ti = blockIdx.x / tn;
+    tj = blockIdx.x % tn;
+  }
+  const int i0 = ti * C::TM, j0 = tj * C::TN;
+  const bool diag = sym && ti == tj;
+  int wm = warp / WN, wn = warp % WN;
+  bool work = true;
+  if (diag) {  // warps 0, 1, .. take the blocks wm <= wn: spread over the schedulers
+    int r = warp;
+    wm = 0;
+    while (wm < WM && r >= WN - wm) {
+      r -= WN - wm;
+      ++wm;
+    }
+    work = wm < WM;
+    wn = wm + r;
+    if (!work) wm = wn = 0;
+  }
+  const int nchunk = (K + 31) / 32;
+  const int c0 = (int)((long long)nchunk * blockIdx.y / gridDim.y);
+  const int c1 = (int)((long long)nchunk * (blockIdx.y + 1) / gridDim.y);
+  double acc[4][4][2];
+  dm::zero(acc);
+  auto load = [&](int st, int c) {
+    for (int q = tid; q < C::TM * 16; q += C::THREADS) {
+      const int row = q >> 4, k = c * 32 + 2 * (q & 15);
+      const bool ok = i0 + row < M && k < K;
+      tc::cp16(As + (st * C::TM + row) * dm::LDK + 2 * (q & 15),
+               A + (ok ? (size_t)(i0 + row) * K + k : 0), ok ? 16 : 0);
+    }
+    if (!diag)
+      for (int q = tid; q < C::TN * 16; q += C::THREADS) {
+        const int row = q >> 4, k = c * 32 + 2 * (q & 15);
+        const bool ok = j0 + row < N && k < K;
+        tc::cp16(Bs + (st * C::TN + row) * dm::LDK + 2 * (q & 15),
+                 B + (ok ? (size_t)(j0 + row) * K + k : 0), ok ? 16 : 0);
       }
-      ra[q] = va;
-      rb[q] = vb;
-    }
+    tc::cp_commit();
   };
-  auto store = [&](int buf) {
+  if (c0 < c1) load(0, c0);
+  const int g = lane >> 2, t = lane & 3;
+  for (int c = c0; c < c1; ++c) {
+    const int st = (c - c0) & 1;
+    double wv[4];  // the weight of this thread's point in each group of 8 reals
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int idx = threadIdx.x + 256 * q;
-      const int row = idx >> 3, kp = idx & 7;
-      As[buf][2 * kp][row] = ra[q].x;
-      As[buf][2 * kp + 1][row] = ra[q].y;
-      Bs[buf][2 * kp][row] = rb[q].x;
-      Bs[buf][2 * kp + 1][row] = rb[q].y;
+    for (int kk = 0; kk < 4; ++kk) {
+      const int p = c * 16 + kk * 4 + t;
+      wv[kk] = (w && 2 * p < K) ? w[p] : 1.0;
     }
-  };
-  int buf = 0;
-  if (kbeg < kend) {
-    load(kbeg);
-    store(0);
-  }
-  __syncthreads();
-  for (int k0 = kbeg; k0 < kend; k0 += TK) {
-    const bool more = k0 + TK < kend;
-    if (more) load(k0 + TK);
-#pragma unroll
-    for (int kk = 0; kk < TK; ++kk) {
-      double a[8], b[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) a[i] = As[buf][kk][ty + 16 * i];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) b[j] = Bs[buf][kk][tx + 16 * j];
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
-    }
-    if (more) store(buf ^ 1);
+    tc::cp_wait<0>();
     __syncthreads();
-    buf ^= 1;
-  }
-  double* P = part + (size_t)ks * M * N;
+    if (c + 1 < c1) load(st ^ 1, c + 1);
+    if (!work) continue;
+    const double* a0 = As + (st * C::TM + wm * 32 + g) * dm::LDK + 2 * t;
+    const double* b0 =
+        (diag ? As + (st * C::TM + wn * 32 + g) * dm::LDK : Bs + (st * C::TN + wn * 32 + g) * dm::LDK) +
+        2 * t;
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+    for (int kk = 0; kk < 4; ++kk) {
+      double2 a[4], b[4];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int r = i0 + ty + 16 * i, c = j0 + tx + 16 * j;
-      if (r < M && c < N) P[(size_t)c * M + r] = acc[i][j];
+      for (int i = 0; i < 4; ++i) {
+        a[i] = *reinterpret_cast<const double2*>(a0 + i * 8 * dm::LDK + kk * 8);
+        b[i] = *reinterpret_cast<const double2*>(b0 + i * 8 * dm::LDK + kk * 8);
+        a[i].x *= wv[kk];
+        a[i].y *= wv[kk];
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) dm::mma884(acc[i][j], a[i].x, b[j].x);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) dm::mma884(acc[i][j], a[i].y, b[j].y);
     }
+  }
+  if (!work) return;
+  double* P = part + (size_t)blockIdx.y * M * N;
+  const bool both = sym && (!diag || wm != wn);
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int r = i0 + wm * 32 + i * 8 + g, cc = j0 + wn * 32 + j * 8 + 2 * t + e;
+        if (r < M && cc < N) {
+          P[(size_t)cc * M + r] = acc[i][j][e];
+          if (both) P[(size_t)r * M + cc] = acc[i][j][e];
+        }
+      }
 }
 
+template <int WM>
+struct BmCfg {
+  static constexpr int TM = 32 * WM, THREADS = 128 * WM;
+  static constexpr size_t SMEM = sizeof(double) * 2 * (dm::LDK * TM + 32 * dm::LDN);
+};
+
 // out[i][p] = alpha w[p/2] sum_j Mcm[j + i ldm] in[j][p] + beta out[i][p] on
-// 128 (i) x 128 (p) tiles; the inner dimension j runs in chunks of 16.
-__global__ void __launch_bounds__(256, 1)
-k_backmul_t128(const double* __restrict__ Mcm, int ldm, const double* __restrict__ in, int ldi,
-               double* __restrict__ out, int ldo, int nout, int nin, int K, double alpha,
-               double beta, const double* __restrict__ w) {
-  extern __shared__ __align__(16) double t128_smem[];
-  double (*Ms)[TK][TLD] = reinterpret_cast<double (*)[TK][TLD]>(t128_smem);  // [j][i]
-  double (*Is)[TK][TLD] = reinterpret_cast<double (*)[TK][TLD]>(t128_smem + 2 * TK * TLD);
-  const int p0 = blockIdx.x * TB, i0 = blockIdx.y * TB;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  double acc[8][8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = 0.0;
-  double2 rm[4], ri[4];
-  // M tile: row i (128) x 16 j: idx -> i = idx / 8, j pair = idx % 8 (contiguous j)
-  // in tile: 16 j x 128 p: idx -> j = idx / 64, p pair = idx % 64
-  auto load = [&](int j0) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int idx = threadIdx.x + 256 * q;
-      const int i = idx >> 3, jp = idx & 7;
-      const int j = j0 + 2 * jp;
-      double2 vm = make_double2(0.0, 0.0);
-      if (i0 + i < nout) {
-        const double* mrow = Mcm + (size_t)(i0 + i) * ldm;
-        if (j + 1 < nin) vm = make_double2(mrow[j], mrow[j + 1]);
-        else if (j < nin) vm.x = mrow[j];
-      }
-      rm[q] = vm;
-      const int jj = idx >> 6, pp = idx & 63;
-      const int jr = j0 + jj, p = p0 + 2 * pp;
-      double2 vi = make_double2(0.0, 0.0);
-      if (jr < nin && p < K)  // K even, p even: the pair is inside
-        vi = *reinterpret_cast<const double2*>(in + (size_t)jr * ldi + p);
-      ri[q] = vi;
+// tiles of 32 WM rows x 128 reals; blocks walk the tiles (the row tiles of a
+// point tile one after the other: in read once from HBM) with the next chunk's
+// copies, the next tile's first one included, in flight behind the products.
+// vec: out rows are 16-byte aligned.
+template <int WM>
+__global__ void __launch_bounds__(BmCfg<WM>::THREADS)
+k_backmul(const double* __restrict__ Mcm, int ldm, const double* __restrict__ in, int ldi,
+          double* __restrict__ out, int ldo, int nout, int nin, int K, double alpha, double beta,
+          const double* __restrict__ w, int vec) {
+  using C = BmCfg<WM>;
+  extern __shared__ __align__(16) double sm[];
+  double* As = sm;                      // [2][TM][LDK]: M rows i, j contiguous
+  double* Bs = sm + 2 * C::TM * dm::LDK;  // [2][32][LDN]: in rows j
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int wm = warp >> 2, wn = warp & 3;
+  const int ni = (nout + C::TM - 1) / C::TM, nj = (nin + 31) / 32;
+  const int ntile = ((K + 127) / 128) * ni;
+  const int mine = (int)blockIdx.x < ntile ? (ntile - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+  const int total = mine * nj;
+  double acc[4][4][2];
+  dm::zero(acc);
+  auto load = [&](int st, int it) {
+    const int tile = (int)blockIdx.x + (it / nj) * (int)gridDim.x, j0 = (it % nj) * 32;
+    const int p0 = (tile / ni) * 128, i0 = (tile % ni) * C::TM;
+    for (int q = tid; q < C::TM * 32; q += C::THREADS) {
+      const int row = q >> 5, j = q & 31;
+      const bool ok = i0 + row < nout && j0 + j < nin;
+      tc::cp8(As + (st * C::TM + row) * dm::LDK + j,
+              Mcm + (ok ? (size_t)(i0 + row) * ldm + j0 + j : 0), ok ? 8 : 0);
     }
+    for (int q = tid; q < 32 * 64; q += C::THREADS) {
+      const int row = q >> 6, p = p0 + 2 * (q & 63);
+      const bool ok = j0 + row < nin && p < K;  // K and p even: the pair is inside
+      tc::cp16(Bs + (st * 32 + row) * dm::LDN + 2 * (q & 63),
+               in + (ok ? (size_t)(j0 + row) * ldi + p : 0), ok ? 16 : 0);
+    }
+    tc::cp_commit();
   };
-  auto store = [&](int buf) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int idx = threadIdx.x + 256 * q;
-      const int i = idx >> 3, jp = idx & 7;
-      Ms[buf][2 * jp][i] = rm[q].x;
-      Ms[buf][2 * jp + 1][i] = rm[q].y;
-      const int jj = idx >> 6, pp = idx & 63;
-      Is[buf][jj][2 * pp] = ri[q].x;
-      Is[buf][jj][2 * pp + 1] = ri[q].y;
-    }
-  };
-  int buf = 0;
-  load(0);
-  store(0);
-  __syncthreads();
-  for (int j0 = 0; j0 < nin; j0 += TK) {
-    const bool more = j0 + TK < nin;
-    if (more) load(j0 + TK);
-#pragma unroll
-    for (int kk = 0; kk < TK; ++kk) {
-      double a[8], b[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) a[i] = Ms[buf][kk][ty + 16 * i];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) b[j] = Is[buf][kk][tx + 16 * j];
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
-    }
-    if (more) store(buf ^ 1);
+  if (total > 0) load(0, 0);
+  for (int it = 0; it < total; ++it) {
+    const int st = it & 1;
+    tc::cp_wait<0>();
     __syncthreads();
-    buf ^= 1;
-  }
+    if (it + 1 < total) load(st ^ 1, it + 1);
+    dm::chunk_kn(acc, As + (st * C::TM + wm * 32) * dm::LDK, Bs + st * 32 * dm::LDN + wn * 32,
+                 lane);
+    if (it % nj != nj - 1) continue;
+    const int tile = (int)blockIdx.x + (it / nj) * (int)gridDim.x;
+    const int i0 = (tile % ni) * C::TM + wm * 32 + (lane >> 2);
+    const int q0 = (tile / ni) * 128 + wn * 32 + 2 * (lane & 3);
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+    for (int j = 0; j < 4; ++j) {
+      const int p = q0 + 8 * j;
+      const double a = (w && p < K) ? alpha * w[p >> 1] : alpha;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int r = i0 + ty + 16 * i, p = p0 + tx + 16 * j;
-      if (r < nout && p < K) {
+      for (int i = 0; i < 4; ++i) {
+        const int r = i0 + 8 * i;
+        double2 v = make_double2(a * acc[i][j][0], a * acc[i][j][1]);
+        acc[i][j][0] = acc[i][j][1] = 0.0;
+        if (r >= nout || p >= K) continue;
         double* o = out + (size_t)r * ldo + p;
-        const double a = w ? alpha * w[p >> 1] : alpha;
-        *o = a * acc[i][j] + (beta == 0.0 ? 0.0 : beta * (*o));
+        if (vec) {
+          if (beta != 0.0) {
+            const double2 u = *reinterpret_cast<const double2*>(o);
+            v.x += beta * u.x;
+            v.y += beta * u.y;
+          }
+          *reinterpret_cast<double2*>(o) = v;
+        } else {
+          o[0] = v.x + (beta == 0.0 ? 0.0 : beta * o[0]);
+          o[1] = v.y + (beta == 0.0 ? 0.0 : beta * o[1]);
+        }
       }
     }
+  }
 }
 
 }  // namespace pcalc
 
 // ---------------------------------------------------------------------------
 // host side
-
-static int t128_attr() {
-  static unsigned long long done = 0;  // one bit per device (the attribute is per device)
-  int dev = 0;
-  CPSTEP_CUDA_TRY(cudaGetDevice(&dev));
-  const unsigned long long bit = 1ull << (dev & 63);
-  if (!(__atomic_load_n(&done, __ATOMIC_ACQUIRE) & bit)) {
-    CPSTEP_CUDA_TRY(cudaFuncSetAttribute(pcalc::k_overlap_t128,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)pcalc::T128_SMEM));
-    CPSTEP_CUDA_TRY(cudaFuncSetAttribute(pcalc::k_backmul_t128,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)pcalc::T128_SMEM));
-    __atomic_or_fetch(&done, bit, __ATOMIC_RELEASE);
-  }
-  return CPSTEP_OK;
-}
 
 int pc_part_reserve(cpstep_ctx* c, size_t need) {
   if (need > c->pc_part_elems) {
@@ -445,36 +465,53 @@ int pc_splitk_reduce_launch(cpstep_ctx* c, int nsplit, int M, int N, double alph
   return CPSTEP_OK;
 }
 
+template <typename F>
+static int dyn_smem(F kernel, size_t bytes) {
+  CPSTEP_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)bytes));
+  return CPSTEP_OK;
+}
+
+template <int WM, int WN>
+static int overlap64(cpstep_ctx* c, const double* a, const double* b, int M, int N, int K,
+                     const double* w, double alpha, double beta, double* C, int ldc, bool sym,
+                     int per_sm) {
+  using Cfg = pcalc::OvlCfg<WM, WN>;
+  const int tm = cdiv(M, Cfg::TM), tn = cdiv(N, Cfg::TN);
+  const int tiles = sym ? tm * (tm + 1) / 2 : tm * tn;
+  const int nsplit = std::max(1, std::min(cdiv(K, 32), c->tune.pc_split * per_sm * c->num_sms / tiles));
+  if (int rc = pc_part_reserve(c, pc_part_need(nsplit, (size_t)M * N))) return rc;
+  if (int rc = dyn_smem(pcalc::k_overlap<WM, WN>, Cfg::SMEM)) return rc;
+  pcalc::k_overlap<WM, WN><<<dim3(tiles, nsplit), Cfg::THREADS, Cfg::SMEM, c->stream>>>(
+      a, b, w, M, N, K, sym ? 1 : 0, tn, c->d_pc_part);
+  CPSTEP_LAUNCH_CHECK();
+  return pc_splitk_reduce_launch(c, nsplit, M, N, alpha, beta, C, ldc, 0);
+}
+
 int pc_overlap_launch(cpstep_ctx* c, const double* a, const double* b, int M, int N, int K,
                       const double* w, double alpha, double beta, double* C, int ldc) {
   using namespace pcalc;
   bool used = false;
   if (int rc = pc_overlap_tc_launch(c, a, b, M, N, K, w, alpha, beta, C, ldc, &used)) return rc;
   if (used) return CPSTEP_OK;
-  if (int rc = t128_attr()) return rc;
-  int tm = cdiv(M, TB), tn = cdiv(N, TB);
-  int want = std::max(1, c->tune.pc_split * c->num_sms / (tm * tn));
-  int kslab = cdiv(cdiv(K, want), TK) * TK;
-  int nsplit = cdiv(K, kslab);
-  if (int rc = pc_part_reserve(c, pc_part_need(nsplit, (size_t)M * N))) return rc;
-  k_overlap_t128<<<dim3(tm, tn, nsplit), 256, T128_SMEM, c->stream>>>(a, K, b, K, w, M, N, K,
-                                                                     kslab, c->d_pc_part);
-  CPSTEP_LAUNCH_CHECK();
-  return pc_splitk_reduce_launch(c, nsplit, M, N, alpha, beta, C, ldc, 0);
+  // both sides within 64 rows: 2 x 2 warps, two blocks per SM
+  const bool sym = a == b && M == N;
+  return (M <= 64 && N <= 64)
+             ? overlap64<2, 2>(c, a, b, M, N, K, w, alpha, beta, C, ldc, sym, 2)
+             : overlap64<4, 4>(c, a, b, M, N, K, w, alpha, beta, C, ldc, sym, 1);
 }
 
-int pc_backmul_launch(cpstep_ctx* c, const double* Mcm, int ldm, const double* in, int ldi,
-                      double* out, int ldo, int nout, int nin, int K, double alpha, double beta) {
-  using namespace pcalc;
-  bool used = false;
-  if (int rc = pc_backmul_tc_launch(c, Mcm, ldm, in, ldi, out, ldo, nout, nin, K, alpha, beta,
-                                    nullptr, &used))
-    return rc;
-  if (used) return CPSTEP_OK;
-  if (int rc = t128_attr()) return rc;
-  dim3 grid(cdiv(K, TB), cdiv(nout, TB));
-  k_backmul_t128<<<grid, 256, T128_SMEM, c->stream>>>(Mcm, ldm, in, ldi, out, ldo, nout, nin, K,
-                                                      alpha, beta, nullptr);
+template <int WM>
+static int backmul64(cpstep_ctx* c, const double* Mcm, int ldm, const double* in, int ldi,
+                     double* out, int ldo, int nout, int nin, int K, double alpha, double beta,
+                     const double* w) {
+  using Cfg = pcalc::BmCfg<WM>;
+  if (int rc = dyn_smem(pcalc::k_backmul<WM>, Cfg::SMEM)) return rc;
+  const int tiles = cdiv(K, 128) * cdiv(nout, Cfg::TM);
+  const int per_sm = (int)std::max<size_t>(1, 227 * 1024 / (Cfg::SMEM + 1024));
+  const int vec = (reinterpret_cast<uintptr_t>(out) & 15) == 0 && (ldo & 1) == 0;
+  pcalc::k_backmul<WM><<<std::min(tiles, per_sm * c->num_sms), Cfg::THREADS, Cfg::SMEM, c->stream>>>(
+      Mcm, ldm, in, ldi, out, ldo, nout, nin, K, alpha, beta, w, vec);
   CPSTEP_LAUNCH_CHECK();
   return CPSTEP_OK;
 }
@@ -482,18 +519,20 @@ int pc_backmul_launch(cpstep_ctx* c, const double* Mcm, int ldm, const double* i
 int pc_backmul_w_launch(cpstep_ctx* c, const double* Mcm, int ldm, const double* in, int ldi,
                         double* out, int ldo, int nout, int nin, int K, double alpha, double beta,
                         const double* w) {
-  using namespace pcalc;
   bool used = false;
   if (int rc = pc_backmul_tc_launch(c, Mcm, ldm, in, ldi, out, ldo, nout, nin, K, alpha, beta, w,
                                     &used))
     return rc;
   if (used) return CPSTEP_OK;
-  if (int rc = t128_attr()) return rc;
-  dim3 grid(cdiv(K, TB), cdiv(nout, TB));
-  k_backmul_t128<<<grid, 256, T128_SMEM, c->stream>>>(Mcm, ldm, in, ldi, out, ldo, nout, nin, K,
-                                                      alpha, beta, w);
-  CPSTEP_LAUNCH_CHECK();
-  return CPSTEP_OK;
+  // the fewest rows per tile that hold all outputs: padded rows cost as much as real ones
+  if (nout <= 32) return backmul64<1>(c, Mcm, ldm, in, ldi, out, ldo, nout, nin, K, alpha, beta, w);
+  if (nout <= 64) return backmul64<2>(c, Mcm, ldm, in, ldi, out, ldo, nout, nin, K, alpha, beta, w);
+  return backmul64<4>(c, Mcm, ldm, in, ldi, out, ldo, nout, nin, K, alpha, beta, w);
+}
+
+int pc_backmul_launch(cpstep_ctx* c, const double* Mcm, int ldm, const double* in, int ldi,
+                      double* out, int ldo, int nout, int nin, int K, double alpha, double beta) {
+  return pc_backmul_w_launch(c, Mcm, ldm, in, ldi, out, ldo, nout, nin, K, alpha, beta, nullptr);
 }
 
 int dgemm_launch(cudaStream_t s, int ta, int tb, int m, int n, int k, double alpha,

@@ -200,6 +200,12 @@ __device__ __forceinline__ void cp16(void* dst, const void* src, int src_bytes) 
                "r"(src_bytes)
                : "memory");
 }
+// the same for 8 bytes (src_bytes 0 or 8), for sources that are only 8-byte aligned
+__device__ __forceinline__ void cp8(void* dst, const void* src, int src_bytes) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_u32(dst)), "l"(src),
+               "r"(src_bytes)
+               : "memory");
+}
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_wait() {

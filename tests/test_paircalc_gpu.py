@@ -128,3 +128,43 @@ def test_ortho_reports_non_convergence(pc):
     with pytest.raises(_lib.CpstepError) as e:
         pc["ctx"].ortho_tmat(S)
     assert e.value.code == _lib.CPSTEP_ERR_NOCONV
+
+
+@pytest.mark.parametrize("na,nb", [(1, 1), (32, 33), (64, 64), (65, 64), (64, 65), (128, 129), (200, 3)])
+def test_fp64_product_tile_edges(na, nb):
+    """The FP64 products at the edges of their tiles (32 rows per warp, 64 and 128
+    per block; ragged K), a operand equal to or other than b, an odd leading
+    dimension, an output that is only 8-byte aligned.  K = 2 npts terms of
+    order 1, so rounding stays below eps K = 2.6e-13 of the largest entry: 1e-12."""
+    if not cuda_ok():
+        pytest.skip("no CUDA device")
+    import torch
+    from openatom_b200.context import StepContext
+    from openatom_b200.layout import StateLayout
+    from oracle import ortho as OO
+    lay = StateLayout(9.0, 20.0, nfft=28)
+    g = torch.Generator(device="cuda").manual_seed(na * 1000 + nb)
+    mk = lambda n: torch.view_as_complex(torch.randn((n, lay.npts, 2), generator=g,
+                                                     dtype=torch.float64, device="cuda"))
+    a, b = mk(na), mk(nb)
+    ctx = StepContext(lay, max(na, nb), precision="fp64")
+    try:
+        out = ctx.pc_overlap(a, b)
+        ref = OO.pc_overlap(a.cpu().numpy(), b.cpu().numpy(), lay.kx)
+        assert np.max(np.abs(colmajor(out) - ref)) <= 1e-12 * np.max(np.abs(ref))
+        s = ctx.pc_overlap(a, a)
+        assert bool((s == s.t()).all())
+        refs = OO.pc_overlap(a.cpu().numpy(), a.cpu().numpy(), lay.kx)
+        assert np.max(np.abs(s.cpu().numpy() - refs)) <= 1e-12 * np.max(np.abs(refs))
+        M = torch.randn((nb, na + 1), generator=g, dtype=torch.float64, device="cuda")
+        want = (M[:, :na].cpu().numpy() @ a.cpu().numpy())
+        got = ctx.pc_backmultiply(M, a, nout=nb)
+        assert np.max(np.abs(got.cpu().numpy() - want)) <= 1e-12 * np.max(np.abs(want))
+        buf = torch.ones(2 * nb * lay.npts + 1, dtype=torch.float64, device="cuda")
+        odd = buf[1:]  # 8 bytes past a 16-byte boundary
+        ctx.pc_backmultiply(M, a, nout=nb, alpha=-2.0, beta=3.0, out=odd)
+        want2 = 3.0 * (1 + 1j) - 2.0 * want
+        got2 = odd.cpu().numpy().view(np.complex128).reshape(nb, -1)
+        assert np.max(np.abs(got2 - want2)) <= 1e-12 * np.max(np.abs(want2))
+    finally:
+        ctx.close()
