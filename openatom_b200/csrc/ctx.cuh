@@ -350,7 +350,8 @@ struct cpstep_ctx {
   double* d_rho_part;    // [ngroups_rho][nz*ny*nx], or the two-stage density's plane partials
   int ngroups_rho;
   size_t rho_part_elems = 0;  // doubles in d_rho_part
-  int p16_blocks_k2 = 0, p16_blocks_k3 = 0;  // resident blocks of the two-stage plane passes
+  int p16_blocks_k3 = 0;         // resident blocks of the FP32 N = 128 V.psi pass
+  int two_blocks[2] = {0, 0};    // the same of the P x Q two-stage passes (density, V.psi)
   void* d_vks_t;         // V_KS in working precision [nz][ny][nx]
   double* d_eke_part;    // [nstates][nblk_z]
   int nblk_z;
@@ -394,8 +395,9 @@ struct cpstep_ctx {
   // the fixed heuristics
   struct Tune {
     int shfl = 2;         // state plane passes (density, V.psi): register shuffle FFT (1),
-                          // shared-memory Stockham (0), or the two-stage form of
-                          // fft_p16.cuh (2: FP32 and N = 32, 64, 128; elsewhere as 1)
+                          // shared-memory Stockham (0), or the two-stage forms (2:
+                          // fft_two.cuh, fft_p16.cuh in FP32 where it is the faster one;
+                          // sizes without one run as 1)
     int plane_waves = 3;  // state plane passes: blocks ~ plane_waves x SMs
     int nl_blocks = 6;    // EES plane kernels: blocks ~ nl_blocks x SMs
     int pc_split = 1;     // PairCalc overlap split-K: CTAs ~ pc_split x SMs

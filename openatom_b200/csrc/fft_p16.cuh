@@ -38,17 +38,12 @@ __device__ __forceinline__ int p16_pad(int i) { return i + (i >> 4); }
 
 // Twiddles: s2b multiplies by W_N^{t k} and b2s by W_N^{(H t + h) a}.  The
 // b2s ones are kept factored, W_N^{H t a} in registers times W_N^{h a} read
-// from the shared table (the same word for every lane: a broadcast).  LEAN =
-// true factors the s2b ones too, W_N^{t (k % 4)} W_N^{4 t (k / 4)} (12
-// registers instead of 30, one more complex multiply per element), for
-// kernels that need their registers for accumulators.
-template <typename T, int N, bool LEAN = false>
+// from the shared table (the same word for every lane: a broadcast).
+template <typename T, int N>
 struct P16Fft {
   using C = P16Cfg<N>;
   static constexpr int R = C::R, H = C::H;
-  static constexpr int NW1 = LEAN ? 1 : 16;
-  cplx<T> w1[NW1];       // W_N^{t k'}   (s2b twiddles of this thread)
-  cplx<T> wa[4], wb[4];  // LEAN: W_N^{t j}, W_N^{4 t j}
+  cplx<T> w1[16];        // W_N^{t k'}   (s2b twiddles of this thread)
   cplx<T> w2[R];         // W_N^{H t a}  (b2s twiddles of this thread, before W_N^{h a})
   const cplx<T>* tws;    // the shared W_N^m table
   int t;                 // thread within the line group
@@ -56,23 +51,10 @@ struct P16Fft {
   __device__ __forceinline__ void init(const cplx<T>* tw) {
     t = (threadIdx.x & 31) % R;
     tws = tw;
-    if (LEAN) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        wa[j] = tw[(t * j) % N];
-        wb[j] = tw[(4 * t * j) % N];
-      }
-    } else {
-#pragma unroll
-      for (int k = 0; k < 16; ++k) w1[k] = tw[(t * k) % N];
-    }
+    for (int k = 0; k < 16; ++k) w1[k] = tw[(t * k) % N];
 #pragma unroll
     for (int a = 0; a < R; ++a) w2[a] = tw[(H * t * a) % N];
-  }
-
-  __device__ __forceinline__ cplx<T> tw1(int k) const {
-    if (LEAN) return (k & 3) ? ((k >> 2) ? cmul(wa[k & 3], wb[k >> 2]) : wa[k & 3]) : wb[k >> 2];
-    return w1[k];
   }
 
   template <bool INV>
@@ -87,7 +69,7 @@ struct P16Fft {
   __device__ __forceinline__ void s2b(cplx<T> (&v)[16], cplx<T>* scr) const {
     Dft<T, 16, INV>::template run<N>(v, nullptr);
 #pragma unroll
-    for (int k = 1; k < 16; ++k) v[k] = mulw<INV>(v[k], tw1(k));
+    for (int k = 1; k < 16; ++k) v[k] = mulw<INV>(v[k], w1[k]);
     __syncwarp();
 #pragma unroll
     for (int k = 0; k < 16; ++k) scr[p16_pad(k * R + t)] = v[k];

@@ -27,7 +27,7 @@
 #include "ctx.cuh"
 #include "fft_shfl.cuh"
 #include "fft_p16.cuh"
-#include "fft_t20.cuh"
+#include "fft_two.cuh"
 
 namespace sfft {
 
@@ -771,15 +771,15 @@ k_xy_bwd_s(const cplx<T>* __restrict__ pen, const double* __restrict__ freal,
 }
 
 // ---------------------------------------------------------------------------
-// Plane passes in the two-stage form (fft_p16.cuh), FP32, N = 32, 64, 128:
-// 256 threads, every warp 32 / R line groups of R threads, one line (a
-// column or a row pair) per group at a time.  The plane is [nplane_x][LDY]
-// with LDY = N + 3; every line group owns a scratch line of SCR = N + N/16
-// elements, the exchange buffer of its column and row transforms.  Row pairs
-// are built straight from the plane into stride layout (imag flip, Hermitian
-// extension), C2R'd by s2b into block layout where V_KS (K3) or the density
-// (K2) is applied, and (K3) R2C'd by b2s back into stride layout, where the
-// two real rows' spectra are split with one shuffle.
+// V.psi plane pass with a line per group of R = N / 16 lanes (fft_p16.cuh), FP32;
+// k_two runs the other sizes and the density.  256 threads at two blocks per SM,
+// every warp 32 / R line groups, one line (a column or a row pair) per group at a
+// time.  The plane is [nplane_x][LDY] with LDY = N + 3; every line group owns a
+// scratch line of SCR = N + N/16 elements, the exchange buffer of its column and
+// row transforms.  Row pairs are built straight from the plane into stride layout
+// (imag flip, Hermitian extension), C2R'd by s2b into block layout where V_KS is
+// applied, and R2C'd by b2s back into stride layout, where the two real rows'
+// spectra are split with one shuffle.
 // Bank layout (8-byte elements, a warp access served as two half-warp
 // phases): with LDY odd and LDY = N + 3 the column loads, the column stores in
 // block order and the row builds put the line groups of a half warp on
@@ -789,12 +789,10 @@ k_xy_bwd_s(const cplx<T>* __restrict__ pen, const double* __restrict__ freal,
 // The blocks split the (plane, state) items evenly, plane-major: block b
 // takes items [b I / B, (b + 1) I / B) of I = N S, so all B resident blocks
 // (B = blocks per SM x SMs) carry the same work whatever S is.
-// K2 runs 512 threads (for N = 128 every line group owns one row pair of the
-// plane, so its FP64 accumulators fit the registers), K3 256 threads at two
-// blocks per SM.
-template <int N, int THREADS_>
+constexpr int P16_THREADS = 256;
+template <int N>
 struct P16Shape {
-  static constexpr int THREADS = THREADS_, NW = THREADS / 32;
+  static constexpr int THREADS = P16_THREADS, NW = THREADS / 32;
   static constexpr int LPW = P16Cfg<N>::LPW, SLOTS = NW * LPW;
   static constexpr int LDY = N + 3;
   static constexpr int SL = P16Cfg<N>::SCR;  // scratch line stride
@@ -804,7 +802,6 @@ struct P16Shape {
            ((size_t)N + (size_t)nplx * LDY + (size_t)SLOTS * SL + (size_t)((nlines + 1) & ~1));
   }
 };
-constexpr int P16_K2_THREADS = 512, P16_K3_THREADS = 256;
 
 // the pencil row of one (state, z) into the shared staging buffer with
 // cp.async (8-byte copies, one group per call): issued while the previous
@@ -837,9 +834,9 @@ __device__ __forceinline__ void p16_scatter(const cplx<float>* stage, cplx<float
 // exchange through the line group's own scratch; a warp leaves as soon as no
 // column is left for any of its groups, and groups past the last column of a
 // round run on their scratch and store nothing.
-template <int N, bool INV, bool LEAN>
+template <int N, bool INV>
 __device__ __forceinline__ void p16_columns(cplx<float>* plane, int ldy, int nplx,
-                                            const P16Fft<float, N, LEAN>& F, cplx<float>* scr,
+                                            const P16Fft<float, N>& F, cplx<float>* scr,
                                             int slot, int nslots) {
   constexpr int R = P16Cfg<N>::R, LPW = P16Cfg<N>::LPW;
   const int wslot = slot - slot % LPW;  // first slot of this warp
@@ -917,12 +914,12 @@ __host__ __device__ __forceinline__ long long p16_item_start(long long items, in
 // K3 (two-stage form): pencils -> psi(r) -> psi V occ -> pencils_out, over
 // the block's (plane, state) items
 template <int N>
-__global__ void __launch_bounds__(P16_K3_THREADS, 2)
+__global__ void __launch_bounds__(P16_THREADS, 2)
 k_xy_bwd_p16(const cplx<float>* __restrict__ pen, const float* __restrict__ vks,
              cplx<float>* __restrict__ pen_out, StateGeom g,
              const cplx<float>* __restrict__ twx_g, const double* __restrict__ occ,
              int nstates) {
-  using S = P16Shape<N, P16_K3_THREADS>;
+  using S = P16Shape<N>;
   constexpr int LDY = S::LDY, SLOTS = S::SLOTS, R = P16Cfg<N>::R, LPW = S::LPW;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cplx<float>* tw = reinterpret_cast<cplx<float>*>(smem_raw);
@@ -1010,263 +1007,267 @@ k_xy_bwd_p16(const cplx<float>* __restrict__ pen, const float* __restrict__ vks,
   }
 }
 
-// K2 (two-stage form): planes -> occ psi^2 accumulated in FP64 registers over
-// the block's items of one plane; each plane the block touches (segment q of
-// its item range) gets its own partial density out[b segs + q][y][x].  Every
-// row pair of the plane belongs to one line group (PASSES = (N/2) / SLOTS of
-// them per group), the slots of its block layout to the group's threads.
-template <int N>
-__global__ void __launch_bounds__(P16_K2_THREADS, 1)
-k_xy_fwd_p16(const cplx<float>* __restrict__ pen, StateGeom g,
-             const cplx<float>* __restrict__ twx_g, const double* __restrict__ occ,
-             int nstates, int segs, double* __restrict__ out) {
-  using S = P16Shape<N, P16_K2_THREADS>;
-  constexpr int LDY = S::LDY, SLOTS = S::SLOTS, R = P16Cfg<N>::R, LPW = S::LPW;
-  constexpr int PASSES = (N / 2 + SLOTS - 1) / SLOTS;
+// ---------------------------------------------------------------------------
+// K2 (MODE 0) and K3 (MODE 1) in the two-stage P x Q form of fft_two.cuh, over
+// the block's (plane, state) items (p16_item_start); blockIdx.y: the row split
+// of MODE 0.  MODE 0 adds occ psi^2 in FP64 registers per plane and writes one
+// partial plane per (block, plane touched) as k_xy_fwd_p16; MODE 1 as
+// k_xy_bwd_p16.
+template <typename T, int N, int MODE>
+__global__ void __launch_bounds__(TwoShape<T, N, MODE == 0>::THREADS, TwoShape<T, N, MODE == 0>::minb())
+k_two(const cplx<T>* __restrict__ pen, const T* __restrict__ vks, cplx<T>* __restrict__ pen_out,
+      StateGeom g, const cplx<T>* __restrict__ twx_g, const double* __restrict__ occ,
+      int nstates, int segs, double* __restrict__ out) {
+  using S = TwoShape<T, N, MODE == 0>;
+  using Pos = TwoPos<N>;
+  constexpr int P = S::P, Q = S::Q, QS = S::QS, G = S::G, W = S::W, LC = S::LC, LS = S::LS;
+  constexpr int R1 = S::R1, R2 = S::R2, YS = MODE == 0 ? TwoCfg<N>::YS : 1;
+  constexpr int PASSES = S::passes(YS), NPAIR = N / 2;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  cplx<float>* tw = reinterpret_cast<cplx<float>*>(smem_raw);
-  cplx<float>* plane = tw + N;
+  cplx<T>* tw1 = reinterpret_cast<cplx<T>*>(smem_raw);  // [k][q] W_N^{q k}
+  cplx<T>* tw2 = tw1 + N;                               // [a][k] W_N^{k a}
+  cplx<T>* plane = tw2 + N;
   const int nplx = g.nplane_x;
-  const int slot = (threadIdx.x >> 5) * LPW + (threadIdx.x & 31) / R;
-  const int wslot = slot - slot % LPW;
-  cplx<float>* scr = plane + (size_t)nplx * LDY + (size_t)slot * S::SL;
-  cplx<float>* stage = plane + (size_t)nplx * LDY + (size_t)SLOTS * S::SL;
+  cplx<T>* scr0 = plane + (size_t)nplx * LC;
+  cplx<T>* stage = scr0 + (size_t)W * G * LS;
+  unsigned short* map = reinterpret_cast<unsigned short*>(stage + ((g.nlines + 1) & ~1));
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  cplx<T>* scr = scr0 + (size_t)warp * G * LS;
   const long long items = (long long)N * nstates;
   const long long i0 = p16_item_start(items, blockIdx.x, gridDim.x);
   const long long i1 = p16_item_start(items, blockIdx.x + 1, gridDim.x);
-  for (int i = threadIdx.x; i < N; i += blockDim.x) tw[i] = twx_g[i];
-  if (i0 < i1)
-    p16_prefetch(pen + ((size_t)(i0 % nstates) * N + (size_t)(i0 / nstates)) * g.nlpad, stage,
-                 g.nlines);
+  auto prefetch = [&](long long it) {
+    const cplx<T>* row = pen + ((size_t)(it % nstates) * N + (size_t)(it / nstates)) * g.nlpad;
+    for (int l = tid; l < g.nlines; l += S::THREADS)
+      asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(
+                       (unsigned)__cvta_generic_to_shared(stage + l)),
+                   "l"(row + l), "n"((int)sizeof(cplx<T>))
+                   : "memory");
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  if (i0 < i1) prefetch(i0);
+  for (int i = tid; i < N; i += S::THREADS) {
+    tw1[i] = twx_g[(i / Q) * (i % Q)];
+    tw2[i] = twx_g[(i / P) * (i % P)];
+  }
+  for (int i = tid; i < nplx * N; i += S::THREADS) map[i] = 0xffff;
   __syncthreads();
-  P16Fft<float, N, true> F;
-  F.init(tw);
-  double acc[PASSES][2][16];
+  for (int l = tid; l < g.nlines; l += S::THREADS) {
+    const int xy = __ldg(g.line_xy + l);
+    map[(xy & 0xffff) * N + (xy >> 16)] = (unsigned short)l;
+  }
+  constexpr int NACC = MODE == 0 ? PASSES * R2 : 1;
+  double acc[NACC][2][Q];
+  if (MODE == 0) {
 #pragma unroll
-  for (int q = 0; q < PASSES; ++q)
+    for (int i = 0; i < NACC; ++i)
 #pragma unroll
-    for (int h = 0; h < 2; ++h)
-#pragma unroll
-      for (int k = 0; k < 16; ++k) acc[q][h][k] = 0.0;
-  // the partial density of the current plane into its segment, then zero
+      for (int m = 0; m < Q; ++m) acc[i][0][m] = acc[i][1][m] = 0.0;
+  }
+  // first row pair of this warp's pass, and the last pair of the block's rows
+  const int ybeg = NPAIR * (int)blockIdx.y / YS, yend = NPAIR * ((int)blockIdx.y + 1) / YS;
   auto flush = [&](int seg) {
     double* o = out + ((size_t)blockIdx.x * segs + seg) * N * N;
 #pragma unroll
-    for (int q = 0; q < PASSES; ++q) {
-      const int pp = slot + SLOTS * q;
-      if (pp < N / 2) {
-        const int ya = 2 * pp;
+    for (int ps = 0; ps < PASSES; ++ps)
 #pragma unroll
-        for (int k = 0; k < 16; ++k) {
-          const int x = F.bpos(k);
-          o[(size_t)ya * N + x] = acc[q][0][k];
-          o[(size_t)(ya + 1) * N + x] = acc[q][1][k];
-          acc[q][0][k] = 0.0;
-          acc[q][1][k] = 0.0;
+      for (int rd = 0; rd < R2; ++rd) {
+        const int t = lane + 32 * rd, pair = ybeg + (ps * W + warp) * G + t / P;
+        if (t < G * P && pair < yend) {
+#pragma unroll
+          for (int m = 0; m < Q; ++m) {
+            double* q = o + (size_t)(2 * pair) * N + t % P + P * m;
+            q[0] = acc[ps * R2 + rd][0][m];
+            q[N] = acc[ps * R2 + rd][1][m];
+            acc[ps * R2 + rd][0][m] = acc[ps * R2 + rd][1][m] = 0.0;
+          }
         }
       }
-    }
   };
   int zc = (int)(i0 / nstates), seg = 0;
   for (long long it = i0; it < i1; ++it) {
     const int z = (int)(it / nstates), s = (int)(it % nstates);
-    if (z != zc) {  // block-uniform
+    if (MODE == 0 && z != zc) {  // block-uniform
       flush(seg);
       zc = z;
       ++seg;
     }
-    p16_scatter<N, LDY>(stage, plane, g);
-    if (it + 1 < i1)
-      p16_prefetch(pen + ((size_t)((it + 1) % nstates) * N + (size_t)((it + 1) / nstates)) *
-                             g.nlpad,
-                   stage, g.nlines);
-    p16_columns<N, false>(plane, LDY, nplx, F, scr, slot, SLOTS);  // FFTW_FORWARD y
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    // y pass (FFTW_FORWARD): columns, first stage from the pencil row
+    for (int t = tid; t < nplx * Q; t += S::THREADS) {
+      const int c = t / Q, q = t % Q;
+      const unsigned short* mp = map + c * N + q;
+      cplx<T> v[P];
+#pragma unroll
+      for (int r = 0; r < P; ++r) {
+        const int l = mp[Q * r];
+        v[r] = l != 0xffff ? stage[l] : mk<T>(0, 0);
+      }
+      rdft<T, P, false>(v);
+      cplx<T>* col = plane + c * LC + q;
+      col[0] = v[0];
+#pragma unroll
+      for (int k = 1; k < P; ++k) col[k * QS] = cmul(v[k], tw1[k * Q + q]);
+    }
+    __syncthreads();
+    if (it + 1 < i1) prefetch(it + 1);
+    for (int t = tid; t < nplx * P; t += S::THREADS) {
+      cplx<T>* col = plane + (t / P) * LC + (t % P) * QS;
+      cplx<T> v[Q];
+#pragma unroll
+      for (int q = 0; q < Q; ++q) v[q] = col[q];
+      rdft<T, Q, false>(v);
+#pragma unroll
+      for (int m = 0; m < Q; ++m) col[m] = v[m];
+    }
     __syncthreads();
     const double w = occ[s];
+    const T wt = (T)w;
+    const T* vplane = MODE == 1 ? vks + (size_t)z * N * N : nullptr;
 #pragma unroll
-    for (int q = 0; q < PASSES; ++q) {
-      if (SLOTS * q + wslot < N / 2) {  // warp-uniform
-        const int pp = slot + SLOTS * q;
-        const bool act = pp < N / 2;
-        const int ya = act ? 2 * pp : 0;
-        cplx<float> v[16];
-        p16_build_row<N>(plane, LDY, nplx, ya, F.t, v);
-        F.template s2b<true>(v, scr);  // C2R, +i sign
-        if (act) {
+    for (int ps = 0; ps < PASSES; ++ps) {
+      const int pbase = ybeg + (ps * W + warp) * G;
+      if (pbase >= yend) break;  // warp-uniform
+      const int np = min(G, yend - pbase);
+      // C2R (+i sign), first stage: Z = conj(Xa) + i conj(Xb) of rows (y, y + 1),
+      // Hermitian-extended to kx > N / 2
 #pragma unroll
-          for (int k = 0; k < 16; ++k) {
-            acc[q][0][k] += w * (double)v[k].x * (double)v[k].x;
-            acc[q][1][k] += w * (double)v[k].y * (double)v[k].y;
+      for (int rd = 0; rd < R1; ++rd) {
+        const int t = lane + 32 * rd, pi = t / Q, q = t % Q;
+        if (t < np * Q) {
+          const int y = 2 * (pbase + pi), ia = Pos::b(y), ib = Pos::b(y + 1);
+          cplx<T> v[P];
+#pragma unroll
+          for (int r = 0; r < P; ++r) {
+            const int x = q + Q * r;
+            cplx<T> zv = mk<T>(0, 0);
+            if (x == 0) {
+              zv = mk<T>(plane[ia].x, plane[ib].x);
+            } else if (x < nplx) {
+              const cplx<T> a = plane[x * LC + ia], b = plane[x * LC + ib];
+              zv = mk<T>(a.x + b.y, b.x - a.y);
+            } else if (N - x < nplx) {
+              const cplx<T> a = plane[(N - x) * LC + ia], b = plane[(N - x) * LC + ib];
+              zv = mk<T>(a.x - b.y, a.y + b.x);
+            }
+            v[r] = zv;
+          }
+          rdft<T, P, true>(v);
+          cplx<T>* o = scr + pi * LS + q;
+          o[0] = v[0];
+#pragma unroll
+          for (int k = 1; k < P; ++k) o[k * QS] = cmulc(v[k], tw1[k * Q + q]);
+        }
+      }
+      __syncwarp();
+#pragma unroll
+      for (int rd = 0; rd < R2; ++rd) {
+        const int t = lane + 32 * rd, pi = t / P, k = t % P;
+        if (t < np * P) {
+          cplx<T>* e = scr + pi * LS + k * QS;
+          const T* va = MODE == 1 ? vplane + (size_t)(2 * (pbase + pi)) * N + k : nullptr;
+          T ra[Q], rb[Q];
+          if (MODE == 1) {  // V_KS of the two rows, in flight behind the DFT
+#pragma unroll
+            for (int m = 0; m < Q; ++m) {
+              ra[m] = __ldg(va + P * m);
+              rb[m] = __ldg(va + N + P * m);
+            }
+          }
+          cplx<T> v[Q];
+#pragma unroll
+          for (int q = 0; q < Q; ++q) v[q] = e[q];
+          rdft<T, Q, true>(v);  // psi(r) of both rows at x = k + P m
+          if (MODE == 0) {
+#pragma unroll
+            for (int m = 0; m < Q; ++m) {
+              double* a0 = &acc[MODE == 0 ? ps * R2 + rd : 0][0][m];
+              double* a1 = &acc[MODE == 0 ? ps * R2 + rd : 0][1][m];
+              *a0 += w * (double)v[m].x * (double)v[m].x;
+              *a1 += w * (double)v[m].y * (double)v[m].y;
+            }
+          } else {
+#pragma unroll
+            for (int m = 0; m < Q; ++m) {
+              v[m].x *= ra[m] * wt;
+              v[m].y *= rb[m] * wt;
+            }
+            rdft<T, Q, false>(v);  // R2C (-i sign)
+            e[0] = v[0];
+#pragma unroll
+            for (int a = 1; a < Q; ++a) e[a] = cmul(v[a], tw2[a * P + k]);
           }
         }
       }
+      if (MODE == 1) {
+        __syncwarp();
+#pragma unroll
+        for (int rd = 0; rd < R1; ++rd) {
+          const int t = lane + 32 * rd, pi = t / Q, a = t % Q;
+          if (t < np * Q) {
+            cplx<T>* e = scr + pi * LS + a;
+            cplx<T> v[P];
+#pragma unroll
+            for (int k = 0; k < P; ++k) v[k] = e[k * QS];
+            rdft<T, P, false>(v);
+#pragma unroll
+            for (int b = 0; b < P; ++b) e[b * QS] = v[b];
+          }
+        }
+        __syncwarp();
+        // split the two rows' spectra, imag flip, kx < nplane_x into the plane
+        for (int pi = 0; pi < np; ++pi) {
+          const int y = 2 * (pbase + pi), ia = Pos::b(y), ib = Pos::b(y + 1);
+          const cplx<T>* e = scr + pi * LS;
+          for (int kx = lane; kx < nplx; kx += 32) {
+            const cplx<T> zk = e[Pos::s(kx)], zm = e[Pos::s(kx == 0 ? 0 : N - kx)];
+            plane[kx * LC + ia] = mk<T>((T)0.5 * (zk.x + zm.x), (T)0.5 * (zm.y - zk.y));
+            plane[kx * LC + ib] = mk<T>((T)0.5 * (zk.y + zm.y), (T)0.5 * (zk.x - zm.x));
+          }
+        }
+      }
+      __syncwarp();
     }
-    __syncthreads();
+    if (MODE == 1) {
+      __syncthreads();
+      // y pass back (FFTW_BACKWARD)
+      for (int t = tid; t < nplx * P; t += S::THREADS) {
+        const int k = t % P;
+        cplx<T>* col = plane + (t / P) * LC + k * QS;
+        cplx<T> v[Q];
+#pragma unroll
+        for (int m = 0; m < Q; ++m) v[m] = col[m];
+        rdft<T, Q, true>(v);
+        col[0] = v[0];
+#pragma unroll
+        for (int a = 1; a < Q; ++a) col[a] = cmulc(v[a], tw2[a * P + k]);
+      }
+      __syncthreads();
+      for (int t = tid; t < nplx * Q; t += S::THREADS) {
+        cplx<T>* col = plane + (t / Q) * LC + t % Q;
+        cplx<T> v[P];
+#pragma unroll
+        for (int k = 0; k < P; ++k) v[k] = col[k * QS];
+        rdft<T, P, true>(v);
+#pragma unroll
+        for (int b = 0; b < P; ++b) col[b * QS] = v[b];
+      }
+      __syncthreads();
+      cplx<T>* po = pen_out + ((size_t)s * N + z) * g.nlpad;
+      for (int l = tid; l < g.nlines; l += S::THREADS) {
+        const int xy = __ldg(g.line_xy + l);
+        po[l] = plane[(xy & 0xffff) * LC + Pos::s(xy >> 16)];
+      }
+    }
   }
-  if (i0 < i1) flush(seg);
+  if (MODE == 0 && i0 < i1) flush(seg);
 }
 
 // sum, for every plane z, the partial densities of the blocks whose item
 // range touched it (block order: deterministic), scaled
 __global__ void k_rho_reduce_items(const double* __restrict__ part, int n, int nstates,
                                    int nblocks, int segs, double scale, double* __restrict__ rho);
-
-// ---------------------------------------------------------------------------
-// K3 for N = 200 in the two-stage 20 x 10 form (fft_t20.cuh), FP32: the same
-// item split and plane passes as k_xy_bwd_p16, 512 threads (16 warps of three
-// 10-thread line groups; lanes 30 and 31 work on a scratch line of their own
-// and store nothing), one block per SM.  The plane is [nplane_x][N + 3];
-// every line group (and every warp's idle pair) owns a scratch line of
-// N + N / 20 elements.
-constexpr int T20_K3_THREADS = 512;
-struct T20Shape {
-  static constexpr int N = 200, R = 10, LPW = 3, NW = T20_K3_THREADS / 32;
-  static constexpr int SLOTS = NW * LPW;        // working line groups
-  static constexpr int SCRL = NW * (LPW + 1);   // scratch lines (idle pairs included)
-  static constexpr int LDY = N + 3;
-  static constexpr int SL = T20Cfg::SCR + 2;    // scratch line stride
-  static constexpr size_t bytes(int nplx, int nlines) {
-    return sizeof(cplx<float>) *
-           ((size_t)N + (size_t)nplx * LDY + (size_t)SCRL * SL + (size_t)((nlines + 1) & ~1));
-  }
-};
-
-template <int NN>
-__global__ void __launch_bounds__(T20_K3_THREADS, 1)
-k_xy_bwd_t20(const cplx<float>* __restrict__ pen, const float* __restrict__ vks,
-             cplx<float>* __restrict__ pen_out, StateGeom g,
-             const cplx<float>* __restrict__ twx_g, const double* __restrict__ occ,
-             int nstates) {
-  static_assert(NN == 200, "the 20 x 10 two-stage form");
-  using S = T20Shape;
-  constexpr int N = S::N, LDY = S::LDY, SLOTS = S::SLOTS, R = S::R, LPW = S::LPW, P = 20;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  cplx<float>* tw = reinterpret_cast<cplx<float>*>(smem_raw);
-  cplx<float>* plane = tw + N;
-  const int nplx = g.nplane_x;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int grp = lane / R;                 // 0..2 working, 3 idle
-  const bool idle = grp >= LPW;
-  const int slot = warp * LPW + (idle ? 0 : grp);
-  const int wslot = warp * LPW;
-  cplx<float>* scr = plane + (size_t)nplx * LDY + (size_t)(warp * (LPW + 1) + grp) * S::SL;
-  cplx<float>* stage = plane + (size_t)nplx * LDY + (size_t)S::SCRL * S::SL;
-  const long long items = (long long)N * nstates;
-  const long long i0 = p16_item_start(items, blockIdx.x, gridDim.x);
-  const long long i1 = p16_item_start(items, blockIdx.x + 1, gridDim.x);
-  for (int i = threadIdx.x; i < N; i += blockDim.x) tw[i] = twx_g[i];
-  if (i0 < i1)
-    p16_prefetch(pen + ((size_t)(i0 % nstates) * N + (size_t)(i0 / nstates)) * g.nlpad, stage,
-                 g.nlines);
-  __syncthreads();
-  T20Fft<float> F;
-  F.init(tw);
-  // partner lane of the R2C split (kx -> N - kx): thread (R - t) % R of the group
-  const int src = idle ? lane : grp * R + (R - F.t) % R;
-  for (long long it = i0; it < i1; ++it) {
-    const int z = (int)(it / nstates), s = (int)(it % nstates);
-    p16_scatter<N, LDY>(stage, plane, g);
-    if (it + 1 < i1)
-      p16_prefetch(pen + ((size_t)((it + 1) % nstates) * N + (size_t)((it + 1) / nstates)) *
-                             g.nlpad,
-                   stage, g.nlines);
-    // y pass, forward (FFTW_FORWARD y)
-    for (int c0 = 0; c0 < nplx; c0 += SLOTS) {
-      if (c0 + wslot >= nplx) break;  // warp-uniform
-      const int c = c0 + slot;
-      const bool act = !idle && c < nplx;
-      cplx<float>* col = plane + (size_t)(act ? c : 0) * LDY;
-      cplx<float> v[P];
-#pragma unroll
-      for (int k = 0; k < P; ++k) v[k] = act ? col[F.t + R * k] : mk<float>(0.f, 0.f);
-      F.template s2b<false>(v, scr);
-      if (act) {
-#pragma unroll
-        for (int q = 0; q < P; ++q) col[F.bpos(q)] = v[q];
-      }
-      __syncwarp();
-    }
-    __syncthreads();
-    const float* vplane = vks + (size_t)z * N * N;
-    const float w = (float)occ[s];
-    for (int p0 = 0; p0 < N / 2; p0 += SLOTS) {
-      if (p0 + wslot >= N / 2) break;  // warp-uniform
-      const int pp = p0 + slot;
-      const bool act = !idle && pp < N / 2;
-      const int ya = act ? 2 * pp : 0;
-      // C2R input of rows (ya, ya + 1): Z = conj(Xa) + i conj(Xb), Hermitian-
-      // extended to kx > N / 2
-      cplx<float> v[P];
-#pragma unroll
-      for (int k = 0; k < P; ++k) {
-        const int x = F.t + R * k;
-        cplx<float> zv = mk<float>(0, 0);
-        if (act) {
-          if (x == 0) {
-            zv = mk<float>(plane[ya].x, plane[ya + 1].x);
-          } else if (x < nplx) {
-            const cplx<float> a = plane[x * LDY + ya], b = plane[x * LDY + ya + 1];
-            zv = mk<float>(a.x + b.y, b.x - a.y);
-          } else if (N - x < nplx) {
-            const int m = N - x;
-            const cplx<float> a = plane[m * LDY + ya], b = plane[m * LDY + ya + 1];
-            zv = mk<float>(a.x - b.y, a.y + b.x);
-          }
-        }
-        v[k] = zv;
-      }
-      F.template s2b<true>(v, scr);  // C2R, +i sign
-#pragma unroll
-      for (int q = 0; q < P; ++q) {
-        const int x = F.bpos(q);
-        const float va = act ? __ldg(vplane + ya * N + x) : 0.f;
-        const float vb = act ? __ldg(vplane + (ya + 1) * N + x) : 0.f;
-        v[q].x *= va * w;
-        v[q].y *= vb * w;
-      }
-      F.template b2s<false>(v, scr);  // R2C, -i sign
-      // split the two real rows' spectra: partner N - kx in thread (R - t) % R,
-      // slot P - 1 - b (thread 0 keeps its own slot (P - b) % P); store kx < nplx
-#pragma unroll
-      for (int b = 0; b < P; ++b) {
-        cplx<float> zm;
-        zm.x = __shfl_sync(0xffffffffu, v[P - 1 - b].x, src);
-        zm.y = __shfl_sync(0xffffffffu, v[P - 1 - b].y, src);
-        if (F.t == 0) zm = v[(P - b) % P];
-        const int kx = F.t + R * b;
-        if (act && kx < nplx) {
-          const cplx<float> zk = v[b];
-          plane[kx * LDY + ya] = mk<float>(0.5f * (zk.x + zm.x), 0.5f * (zm.y - zk.y));
-          plane[kx * LDY + ya + 1] = mk<float>(0.5f * (zk.y + zm.y), 0.5f * (zk.x - zm.x));
-        }
-      }
-    }
-    __syncthreads();
-    // y pass, backward (FFTW_BACKWARD y)
-    for (int c0 = 0; c0 < nplx; c0 += SLOTS) {
-      if (c0 + wslot >= nplx) break;
-      const int c = c0 + slot;
-      const bool act = !idle && c < nplx;
-      cplx<float>* col = plane + (size_t)(act ? c : 0) * LDY;
-      cplx<float> v[P];
-#pragma unroll
-      for (int k = 0; k < P; ++k) v[k] = act ? col[F.t + R * k] : mk<float>(0.f, 0.f);
-      F.template s2b<true>(v, scr);
-      if (act) {
-#pragma unroll
-        for (int q = 0; q < P; ++q) col[F.bpos(q)] = v[q];
-      }
-      __syncwarp();
-    }
-    __syncthreads();
-    cplx<float>* po = pen_out + ((size_t)s * N + z) * g.nlpad;
-    for (int l = threadIdx.x; l < g.nlines; l += blockDim.x) {
-      const int xy = __ldg(g.line_xy + l);
-      po[l] = plane[(xy & 0xffff) * LDY + (xy >> 16)];
-    }
-    __syncthreads();
-  }
-}
 
 // ---------------------------------------------------------------------------
 // K4: pencils -> backward z-FFT -> pack -> scale.
@@ -1677,37 +1678,70 @@ struct StateFft {
     return CPSTEP_OK;
   }
 
+  // whether the two-stage P x Q plane passes (k_two) run this size
+  static constexpr bool two_built = TwoCfg<N>::ok && !(sizeof(T) == 8 && N == 200);
+  static bool two_fits(const cpstep_ctx* c, const FftJob& j) {
+    if constexpr (two_built)
+      return c->tune.shfl == 2 && j.g.nlines < 0xffff &&
+             std::max(TwoShape<T, N>::bytes(j.g.nplane_x, j.g.nlines),
+                      TwoShape<T, N, true>::bytes(j.g.nplane_x, j.g.nlines)) <= 227 * 1024;
+    return false;
+  }
+
+  // blocks of the density pass: the resident ones, at least four items each
+  // (a block writes a partial plane per plane it touches), within the partial
+  // buffer and the partials per plane that the reduction lists
+  static int two_density(cpstep_ctx* c, const FftJob& j, const double* occ, double* rho) {
+    if constexpr (two_built) {
+      constexpr int YS = TwoCfg<N>::YS;
+      const size_t smem = TwoShape<T, N, true>::bytes(j.g.nplane_x, j.g.nlines), n2 = (size_t)N * N;
+      if (int rc = set_smem(k_two<T, N, 0>, smem)) return rc;
+      if (int rc = resident_blocks(c, k_two<T, N, 0>, TwoShape<T, N, true>::THREADS, smem,
+                                   &c->two_blocks[0]))
+        return rc;
+      const long long items = (long long)N * c->nstates;
+      int nb = std::max(1, c->two_blocks[0] / YS);
+      nb = (int)std::min<long long>(std::min(nb, 48 * N), std::max(1LL, items / 4));
+      auto segs = [&](int b) {
+        return (int)(((items + b - 1) / b + c->nstates - 1) / c->nstates) + 1;
+      };
+      while (nb > 1 && (size_t)nb * segs(nb) * n2 > c->rho_part_elems) nb = nb * 3 / 4;
+      if ((size_t)nb * segs(nb) * n2 > c->rho_part_elems) {
+        cpstep_set_error("state FFT: density partials need %zu doubles, %zu allocated",
+                         (size_t)nb * segs(nb) * n2, c->rho_part_elems);
+        return CPSTEP_ERR_CUDA;
+      }
+      k_two<T, N, 0><<<dim3(nb, YS), TwoShape<T, N, true>::THREADS, smem, c->stream>>>(
+          reinterpret_cast<const cplx<T>*>(j.pen_a), nullptr, nullptr, j.g, tws<T>(c).x, occ,
+          c->nstates, segs(nb), c->d_rho_part);
+      CPSTEP_LAUNCH_CHECK();
+      k_rho_reduce_items<<<dim3(N, cdiv(4 * c->num_sms, N)), 256, 0, c->stream>>>(
+          c->d_rho_part, N, c->nstates, nb, segs(nb), 1.0 / c->vol, rho);
+      CPSTEP_LAUNCH_CHECK();
+    }
+    return CPSTEP_OK;
+  }
+
+  static int two_vpsi(cpstep_ctx* c, const FftJob& j, const T* vt, const double* occ) {
+    if constexpr (two_built) {
+      const size_t smem = TwoShape<T, N>::bytes(j.g.nplane_x, j.g.nlines);
+      if (int rc = set_smem(k_two<T, N, 1>, smem)) return rc;
+      if (int rc = resident_blocks(c, k_two<T, N, 1>, TwoShape<T, N>::THREADS, smem,
+                                   &c->two_blocks[1]))
+        return rc;
+      const long long items = (long long)N * c->nstates;
+      k_two<T, N, 1><<<(int)std::min<long long>(c->two_blocks[1], items), TwoShape<T, N>::THREADS,
+                       smem, c->stream>>>(
+          reinterpret_cast<const cplx<T>*>(j.pen_a), vt, reinterpret_cast<cplx<T>*>(j.pen_b), j.g,
+          tws<T>(c).x, occ, c->nstates, 0, nullptr);
+    }
+    return CPSTEP_OK;
+  }
+
   static int density(cpstep_ctx* c, const double* psi, const double* occ, double* rho) {
     const FftJob j = c->state_job();
     if (int rc = zfft_fwd(c, j, psi, c->nstates)) return rc;
-    if constexpr (P16Cfg<N>::ok && sizeof(T) == 4) {
-      if (c->tune.shfl == 2) {
-        const size_t smem = P16Shape<N, P16_K2_THREADS>::bytes(j.g.nplane_x, j.g.nlines);
-        if (int rc = set_smem(k_xy_fwd_p16<N>, smem)) return rc;
-        if (int rc = resident_blocks(c, k_xy_fwd_p16<N>, P16_K2_THREADS, smem, &c->p16_blocks_k2))
-          return rc;
-        const int nb = c->p16_blocks_k2;
-        const long long items = (long long)N * c->nstates;
-        const int segs = (int)(((items + nb - 1) / nb + c->nstates - 1) / c->nstates) + 1;
-        if ((size_t)nb * segs * N * N > c->rho_part_elems) {
-          cpstep_set_error("state FFT: density partials need %zu doubles, %zu allocated",
-                           (size_t)nb * segs * N * N, c->rho_part_elems);
-          return CPSTEP_ERR_CUDA;
-        }
-        k_xy_fwd_p16<N><<<nb, P16_K2_THREADS, smem, c->stream>>>(
-            reinterpret_cast<const cplx<float>*>(j.pen_a), j.g, tws<float>(c).x, occ,
-            c->nstates, segs, c->d_rho_part);
-        CPSTEP_LAUNCH_CHECK();
-        if ((long long)nb > 62LL * N) {  // more blocks on one plane than the reduction lists
-          cpstep_set_error("state FFT: %d density blocks over %d planes", nb, N);
-          return CPSTEP_ERR_CUDA;
-        }
-        k_rho_reduce_items<<<dim3(N, cdiv(4 * c->num_sms, N)), 256, 0, c->stream>>>(
-            c->d_rho_part, N, c->nstates, nb, segs, 1.0 / c->vol, rho);
-        CPSTEP_LAUNCH_CHECK();
-        return CPSTEP_OK;
-      }
-    }
+    if (two_fits(c, j)) return two_density(c, j, occ, rho);
     if constexpr (ShflCfg<N>::ok) {
       if (c->tune.shfl) {
         const size_t smem = SShape<T, N>::bytes(j.g.nplane_x);
@@ -1842,29 +1876,23 @@ struct StateFft {
     int spg = cdiv(c->nstates, ng);
     ng = cdiv(c->nstates, spg);
     bool shfl_done = false;
-    if constexpr (P16Cfg<N>::ok && sizeof(T) == 4) {
-      if (c->tune.shfl == 2) {
-        const size_t smem = P16Shape<N, P16_K3_THREADS>::bytes(j.g.nplane_x, j.g.nlines);
+    // N = 128 in FP32: the lane-group form of fft_p16.cuh, with V_KS in vector loads
+    // (64 states: 492 us against 498 us)
+    if constexpr (N == 128 && sizeof(T) == 4) {
+      const size_t smem = P16Shape<N>::bytes(j.g.nplane_x, j.g.nlines);
+      if (c->tune.shfl == 2 && smem <= 227 * 1024) {
         if (int rc = set_smem(k_xy_bwd_p16<N>, smem)) return rc;
-        if (int rc = resident_blocks(c, k_xy_bwd_p16<N>, P16_K3_THREADS, smem, &c->p16_blocks_k3))
+        if (int rc = resident_blocks(c, k_xy_bwd_p16<N>, P16_THREADS, smem, &c->p16_blocks_k3))
           return rc;
-        k_xy_bwd_p16<N><<<c->p16_blocks_k3, P16_K3_THREADS, smem, c->stream>>>(
+        k_xy_bwd_p16<N><<<c->p16_blocks_k3, P16_THREADS, smem, c->stream>>>(
             reinterpret_cast<const cplx<float>*>(j.pen_a), reinterpret_cast<const float*>(vt),
             reinterpret_cast<cplx<float>*>(j.pen_b), j.g, tws<float>(c).x, occ, c->nstates);
         shfl_done = true;
       }
     }
-    if constexpr (N == 200 && sizeof(T) == 4) {
-      const size_t smem = T20Shape::bytes(j.g.nplane_x, j.g.nlines);
-      if (c->tune.shfl == 2 && smem <= 227 * 1024) {  // else the Stockham form below
-        if (int rc = set_smem(k_xy_bwd_t20<N>, smem)) return rc;
-        if (int rc = resident_blocks(c, k_xy_bwd_t20<N>, T20_K3_THREADS, smem, &c->p16_blocks_k3))
-          return rc;
-        k_xy_bwd_t20<N><<<c->p16_blocks_k3, T20_K3_THREADS, smem, c->stream>>>(
-            reinterpret_cast<const cplx<float>*>(j.pen_a), reinterpret_cast<const float*>(vt),
-            reinterpret_cast<cplx<float>*>(j.pen_b), j.g, tws<float>(c).x, occ, c->nstates);
-        shfl_done = true;
-      }
+    if (!shfl_done && two_fits(c, j)) {
+      if (int rc = two_vpsi(c, j, vt, occ)) return rc;
+      shfl_done = true;
     }
     if constexpr (ShflCfg<N>::ok) {
       if (c->tune.shfl && !shfl_done) {

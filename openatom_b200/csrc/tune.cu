@@ -126,7 +126,7 @@ int cpstep_autotune(cpstep_ctx* c, const double* d_psi, const double* d_occ, dou
     return statefft_vpsi(c, d_psi, rho, d_occ, force, eke, 1);
   };
   // plane-pass form: 1 register shuffles, 0 shared-memory Stockham, 2 the
-  // two-stage form (FP32, N = 32, 64, 128; elsewhere it runs as 1)
+  // two-stage forms (elsewhere it runs as 1)
   if (!rc) {
     std::vector<int> forms = {1, 0};
     if (c->precision == CPSTEP_PREC_MIXED) forms.push_back(2);

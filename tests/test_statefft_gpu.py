@@ -201,3 +201,38 @@ def test_plane_pass_forms_n200(form):
         assert ctx.device_errors() == 0
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("grid,box,states", [
+    (28, 9.0, 1), (32, 9.0, 7), (40, 9.0, 33), (42, 9.0, 5), (48, 9.0, 150), (60, 9.0, 3),
+    (64, 12.0, 9), (80, 12.0, 4), (96, 12.0, 2), (120, 12.0, 5), (128, 12.0, 3), (200, 12.0, 2)])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_two_stage_planes_match_stockham(grid, box, states, precision):
+    """Every grid of the two-stage P x Q passes (form 2) against the shared-memory
+    Stockham passes (form 0): one state and many (blocks over several planes and
+    several blocks per plane), empty and ragged rounds of line tasks.  Both are
+    transforms of the same rounding order: the oracle tests' tolerances."""
+    if not cuda_ok():
+        pytest.skip("no CUDA device")
+    import torch
+    from openatom_b200.context import StepContext
+    from openatom_b200.layout import StateLayout
+    lay = StateLayout(box, 20.0, nfft=grid)
+    g = torch.Generator(device="cuda").manual_seed(grid)
+    psi = torch.view_as_complex(torch.randn((states, lay.npts, 2), generator=g,
+                                            dtype=torch.float64, device="cuda"))
+    occ = 0.5 + torch.arange(states, dtype=torch.float64, device="cuda") % 3
+    vks = torch.randn((grid, grid, grid), generator=g, dtype=torch.float64, device="cuda")
+    ctx = StepContext(lay, states, precision=precision)
+    out = []
+    try:
+        for form in (2, 0):
+            ctx.tune_set({"plane_shfl": form})
+            rho = ctx.density(psi, occ).clone()
+            force, eke = ctx.vks_psi(psi, vks, occ)
+            out.append((rho, torch.view_as_real(force), eke))
+        for a, b in zip(*out):
+            assert bool(torch.isfinite(a).all())
+            assert relerr(a.cpu().numpy(), b.cpu().numpy()) < TOL[precision]
+    finally:
+        ctx.close()
