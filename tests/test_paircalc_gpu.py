@@ -168,3 +168,20 @@ def test_fp64_product_tile_edges(na, nb):
         assert np.max(np.abs(got2 - want2)) <= 1e-12 * np.max(np.abs(want2))
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("n", [1, 16, 17, 63, 64, 65, 96, 127, 128, 129, 200])
+@pytest.mark.parametrize("mixed", [False, True])
+def test_ortho_tile_edges(pc, n, mixed):
+    """One block (64 states at most), one K chunk (128) and more, odd and even row
+    strides: T (S/2) T = I.  The products have n terms of order 1, rounding
+    below n eps = 5e-14 each over four of them: 1e-12."""
+    import torch
+    rng = np.random.default_rng(n)
+    Q, _ = np.linalg.qr(rng.standard_normal((n, n)))
+    S = (Q * rng.uniform(1.7, 2.3, n)) @ Q.T
+    S = 0.5 * (S + S.T)
+    T, it, rms = pc["ctx"].ortho_tmat(torch.from_numpy(S).cuda(), mixed=mixed,
+                                      tol=2e-6 if mixed else 1e-13, max_iter=12)
+    T = T.cpu().numpy()
+    assert np.max(np.abs(T.T @ (S / 2) @ T - np.eye(n))) < 1e-12
