@@ -94,6 +94,7 @@ struct StateFftOps {
   int (*gtor)(cpstep_ctx*, const double*, double*, int);
   int (*rtog)(cpstep_ctx*, const double*, double*, int);
   int (*g2r)(cpstep_ctx*, const FftJob&, const double*, double*, int);
+  int (*g2r_add)(cpstep_ctx*, const FftJob&, const double*, double*, double, bool*);
   int (*r2g)(cpstep_ctx*, const FftJob&, const double*, double*, int, double);
   // EES on this grid size: conj(dyp psi) -> NL grid -> per-plane atom sums
   // zpart[s][atom][8][4]; scatter of zs[s][atom] -> NL grid -> fpsi +=

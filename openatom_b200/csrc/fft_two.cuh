@@ -152,6 +152,23 @@ struct TwoShape {
   }
 };
 
+// Real-space passes of single arrays (the density sphere): one block of 16 warps
+// per plane; G row pairs per warp and round, fewer where the plane leaves less
+// shared memory.
+template <typename T, int N>
+struct TwoReal {
+  using S = TwoShape<T, N>;
+  static constexpr int THREADS = 512, W = THREADS / 32;
+  static constexpr size_t bytes_g(int nplx, int G) {
+    return sizeof(cplx<T>) * (2 * (size_t)N + (size_t)nplx * S::LC + (size_t)W * G * S::LL);
+  }
+  static constexpr int g_fit(int G) {
+    return G > 1 && bytes_g(N / 2, G) > 225 * 1024 ? g_fit(G - 1) : G;
+  }
+  static constexpr int G = g_fit((N / 2 + W - 1) / W);
+  static constexpr size_t bytes(int nplx) { return bytes_g(nplx, G); }
+};
+
 template <int N>
 struct TwoPos {
   static constexpr int P = TwoCfg<N>::P, Q = TwoCfg<N>::Q, QS = Q | 1;

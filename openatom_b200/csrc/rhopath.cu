@@ -665,10 +665,10 @@ __global__ void k_sum_cols(const double* __restrict__ part, int nrow, int ncol,
   if (threadIdx.x == 0) out[c] = s * scale;
 }
 
-__global__ void k_add(double* __restrict__ a, const double* __restrict__ b, size_t n) {
+__global__ void k_add(double* __restrict__ a, const double* __restrict__ b, double sign, size_t n) {
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (size_t)gridDim.x * blockDim.x)
-    a[i] += b[i];
+    a[i] += sign * b[i];
 }
 
 __global__ void k_conj_scale(const double2* __restrict__ in, double2* __restrict__ out, int n,
@@ -832,12 +832,6 @@ __global__ void k_div_g(const double2* __restrict__ u, const int* __restrict__ k
     sy += g[d] * v.y;
   }
   w[p] = make_double2(sy, -sx);
-}
-
-__global__ void k_sub(double* __restrict__ a, const double* __restrict__ b, size_t n) {
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (size_t)gridDim.x * blockDim.x)
-    a[i] -= b[i];
 }
 
 }  // namespace rho
@@ -1106,6 +1100,20 @@ int rho_gga_functional(cpstep_ctx* c, const double* rho_r, double* gx, double* g
   return CPSTEP_OK;
 }
 
+// out(r) += sign sum_G vg e^{iGr}
+static int rho_g2r_add(cpstep_ctx* c, const double2* vg, double* out, double sign) {
+  const FftJob j = rho_job(c);
+  const size_t nr = (size_t)c->nx * c->ny * c->nz;
+  bool done = false;
+  if (int rc = c->ops64.g2r_add(c, j, reinterpret_cast<const double*>(vg), out, sign, &done))
+    return rc;
+  if (done) return CPSTEP_OK;
+  if (int rc = c->ops64.g2r(c, j, reinterpret_cast<const double*>(vg), c->rg.vhl, 1)) return rc;
+  rho::k_add<<<2 * c->num_sms, 256, 0, c->stream>>>(out, c->rg.vhl, sign, nr);
+  CPSTEP_LAUNCH_CHECK();
+  return CPSTEP_OK;
+}
+
 // BLYP gradient correction after rho_r2g (r.rhog holds the transformed
 // density): gradients, the functional, the White-Bird term subtracted from vks
 int rho_gga(cpstep_ctx* c, const double* rho_r, double* vks_r, double* energies) {
@@ -1135,11 +1143,7 @@ int rho_gga(cpstep_ctx* c, const double* rho_r, double* vks_r, double* energies)
   rho::k_div_g<<<cdiv(np, 256), 256, 0, c->stream>>>(gg, r.kx, r.ky, r.kz, np, c->d_hmati,
                                                      gg + 3 * (size_t)np);
   CPSTEP_LAUNCH_CHECK();
-  if (int rc = c->ops64.g2r(c, j, reinterpret_cast<const double*>(gg + 3 * (size_t)np), r.vhl, 1))
-    return rc;
-  rho::k_sub<<<2 * c->num_sms, 256, 0, c->stream>>>(vks_r, r.vhl, nr);
-  CPSTEP_LAUNCH_CHECK();
-  return CPSTEP_OK;
+  return rho_g2r_add(c, gg + 3 * (size_t)np, vks_r, -1.0);
 }
 
 void eesloc_free(cpstep_ctx* c) {
@@ -1321,15 +1325,7 @@ int rho_hart(cpstep_ctx* c, double* energies, double* force) {
 }
 
 // V_KS(r) = vxc (already in vks_r) + sum_G vks(G) e^{iGr}
-int rho_vks_r(cpstep_ctx* c, double* vks_r) {
-  FftJob j = rho_job(c);
-  size_t nr = (size_t)c->nx * c->ny * c->nz;
-  if (int rc = c->ops64.g2r(c, j, reinterpret_cast<const double*>(c->rg.vg), c->rg.vhl, 1))
-    return rc;
-  rho::k_add<<<2 * c->num_sms, 256, 0, c->stream>>>(vks_r, c->rg.vhl, nr);
-  CPSTEP_LAUNCH_CHECK();
-  return CPSTEP_OK;
-}
+int rho_vks_r(cpstep_ctx* c, double* vks_r) { return rho_g2r_add(c, c->rg.vg, vks_r, 1.0); }
 
 // helpers for the ABI entries that exchange reference-convention arrays
 int rho_conj_scale(cpstep_ctx* c, const double* in, double* out, int n, double s) {

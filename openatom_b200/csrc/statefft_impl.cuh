@@ -54,7 +54,10 @@ struct PlaneLd;
 
 template <int N>
 struct ZShape {
-  static constexpr int LB = std::min(64, std::max(8, 4096 / N));  // lines per block
+  // lines per block; whole 128-byte pieces of a pencil row (16 FP32 pairs) where a
+  // block's lines allow it
+  static constexpr int LB0 = std::min(64, std::max(8, 4096 / N));
+  static constexpr int LB = LB0 >= 16 ? LB0 / 16 * 16 : LB0;
   static constexpr int LD = PlaneLd<N>::value;
   template <typename T>
   static constexpr size_t bytes() {
@@ -1264,6 +1267,347 @@ k_two(const cplx<T>* __restrict__ pen, const T* __restrict__ vks, cplx<T>* __res
   if (MODE == 0 && i0 < i1) flush(seg);
 }
 
+// ---------------------------------------------------------------------------
+// The z passes in the two-stage form: a first-stage task of K1 reads its P
+// elements of a line straight from the packed coefficients (z -> run position;
+// lanes on consecutive z), a last-stage task of K4 writes its P elements
+// straight to them, so neither zero-fills, searches nor reorders a line buffer;
+// one exchange and the line -> pencil transposition go through shared memory.
+
+// z passes: LB lines per block (ZShape), line tables of LL | 1 elements; as many
+// threads as leave the fewest idle in the rounds of the two stages' LB Q and LB P
+// tasks (160 for 200 points: 16 lines of 10 and 20 tasks, of which 256 threads
+// idled through 0.38).  Forward: latency of the loads, most warps (256 threads, 48
+// registers: 105 us for 128 states of 128^3 FP32, 20 warps of 94: 137).  Backward:
+// blocks of 128 with the registers for four elements' loads in flight (226 -> 130
+// us, FP64 448 -> 239; the bytes take 72 and 104).
+template <typename T, int N>
+struct TwoZ {
+  using S = TwoShape<T, N>;
+  static constexpr int LD = S::LL | 1;
+  static constexpr int LB = ZShape<N>::LB;
+  static constexpr size_t bytes() { return sizeof(cplx<T>) * (N + (size_t)LB * LD); }
+  static constexpr int slots(int t) {
+    return (LB * S::Q + t - 1) / t * t + (LB * S::P + t - 1) / t * t;
+  }
+  static constexpr int FWD = slots(160) < slots(256) ? 160 : 256;
+  static constexpr int BWD = slots(160) < slots(128) ? 160 : 128;
+  static constexpr int MINB = (sizeof(T) == 4 ? 640 : 512) / BWD;  // 102 or 128 registers
+};
+
+// packed offset of element z of a line, -1 outside its two runs
+__device__ __forceinline__ int z_point(int z, int off, int nneg, int zneg, int npos, int zpos) {
+  if ((unsigned)(z - zneg) < (unsigned)nneg) return off + z - zneg;
+  if ((unsigned)(z - zpos) < (unsigned)npos) return off + nneg + z - zpos;
+  return -1;
+}
+
+template <typename T, int N>
+__global__ void __launch_bounds__(TwoZ<T, N>::FWD)
+k_z2_fwd(const double2* __restrict__ psi, cplx<T>* __restrict__ pen, StateGeom g,
+         const cplx<T>* __restrict__ twz) {
+  using S = TwoShape<T, N>;
+  constexpr int P = S::P, Q = S::Q, QS = S::QS, LD = TwoZ<T, N>::LD, LB = TwoZ<T, N>::LB;
+  constexpr int NTHR = TwoZ<T, N>::FWD;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  cplx<T>* tw1 = reinterpret_cast<cplx<T>*>(smem_raw);
+  cplx<T>* buf = tw1 + N;
+  const int l0 = blockIdx.x * LB, nl = min(LB, g.nlines - l0);
+  for (int i = threadIdx.x; i < N; i += NTHR) tw1[i] = twz[(i / Q) * (i % Q)];
+  __syncthreads();
+  const double2* ps = psi + (size_t)blockIdx.y * g.npts;
+  for (int t = threadIdx.x; t < nl * Q; t += NTHR) {
+    const int li = t / Q, q = t % Q, l = l0 + li;
+    const int off = g.line_off[l], nneg = g.line_nneg[l], zneg = g.line_zneg[l];
+    const int npos = g.line_npos[l], zpos = g.line_zpos[l];
+    cplx<T> v[P];
+#pragma unroll
+    for (int r = 0; r < P; ++r) {
+      const int i = z_point(q + Q * r, off, nneg, zneg, npos, zpos);
+      const double2 x = i >= 0 ? ps[i] : make_double2(0.0, 0.0);
+      v[r] = mk<T>((T)x.x, (T)x.y);
+    }
+    rdft<T, P, false>(v);  // FFTW_FORWARD along z
+    cplx<T>* e = buf + li * LD + q;
+    e[0] = v[0];
+#pragma unroll
+    for (int k = 1; k < P; ++k) e[k * QS] = cmul(v[k], tw1[k * Q + q]);
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < nl * P; t += NTHR) {
+    cplx<T>* e = buf + (t / P) * LD + (t % P) * QS;
+    cplx<T> v[Q];
+#pragma unroll
+    for (int q = 0; q < Q; ++q) v[q] = e[q];
+    rdft<T, Q, false>(v);
+#pragma unroll
+    for (int m = 0; m < Q; ++m) e[m] = v[m];
+  }
+  __syncthreads();
+  cplx<T>* po = pen + (size_t)blockIdx.y * N * g.nlpad + l0;
+  for (int i = threadIdx.x; i < LB * N; i += NTHR) {
+    const int z = i / LB, li = i % LB;
+    if (li < nl) po[(size_t)z * g.nlpad + li] = buf[li * LD + TwoPos<N>::b(z)];
+  }
+}
+
+// MODE 0 and 1 as k_zfft_bwd
+template <typename T, int N, int MODE>
+__global__ void __launch_bounds__(TwoZ<T, N>::BWD, TwoZ<T, N>::MINB)
+k_z2_bwd(const cplx<T>* __restrict__ pen, double2* __restrict__ fout,
+         const double2* __restrict__ psi, const double* __restrict__ occ, StateGeom g,
+         const cplx<T>* __restrict__ twz, double scale, double ecut,
+         double* __restrict__ eke_part) {
+  using S = TwoShape<T, N>;
+  constexpr int P = S::P, Q = S::Q, QS = S::QS, LD = TwoZ<T, N>::LD, LB = TwoZ<T, N>::LB;
+  constexpr int NTHR = TwoZ<T, N>::BWD;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ double red[32];
+  cplx<T>* tw2 = reinterpret_cast<cplx<T>*>(smem_raw);
+  cplx<T>* buf = tw2 + N;
+  const int s = blockIdx.y, l0 = blockIdx.x * LB, nl = min(LB, g.nlines - l0);
+  for (int i = threadIdx.x; i < N; i += NTHR) tw2[i] = twz[(i / P) * (i % P)];
+  const cplx<T>* pi = pen + (size_t)s * N * g.nlpad + l0;
+#pragma unroll 8
+  for (int i = threadIdx.x; i < LB * N; i += NTHR) {
+    const int z = i / LB, li = i % LB;
+    if (li < nl) buf[li * LD + TwoPos<N>::b(z)] = pi[(size_t)z * g.nlpad + li];
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < nl * P; t += NTHR) {
+    const int k = t % P;
+    cplx<T>* e = buf + (t / P) * LD + k * QS;
+    cplx<T> v[Q];
+#pragma unroll
+    for (int m = 0; m < Q; ++m) v[m] = e[m];
+    rdft<T, Q, true>(v);  // FFTW_BACKWARD along z
+    e[0] = v[0];
+#pragma unroll
+    for (int a = 1; a < Q; ++a) e[a] = cmulc(v[a], tw2[a * P + k]);
+  }
+  __syncthreads();
+  double e_kin = 0.0;
+  const double wocc = (MODE == 0 && occ) ? occ[s] : 0.0;
+  for (int t = threadIdx.x; t < nl * Q; t += NTHR) {
+    const int li = t / Q, a = t % Q, l = l0 + li;
+    const int off = g.line_off[l], nneg = g.line_nneg[l], zneg = g.line_zneg[l];
+    const int npos = g.line_npos[l], zpos = g.line_zpos[l];
+    const cplx<T>* e = buf + li * LD + a;
+    cplx<T> v[P];
+#pragma unroll
+    for (int k = 0; k < P; ++k) v[k] = e[k * QS];
+    rdft<T, P, true>(v);
+    constexpr int NB = 4;  // elements whose loads are in flight together
+#pragma unroll
+    for (int b0 = 0; b0 < P; b0 += NB) {
+      int pt[NB];
+      double2 ps[NB];
+      double wp[NB], g2[NB];
+#pragma unroll
+      for (int b = 0; b < NB; ++b) {
+        pt[b] = b0 + b < P ? z_point(a + Q * (b0 + b), off, nneg, zneg, npos, zpos) : -1;
+        const bool in = MODE == 0 && pt[b] >= 0, kin = in && occ;
+        wp[b] = in ? __ldg(g.wpt + pt[b]) : 0.0;
+        g2[b] = kin ? __ldg(g.g2 + pt[b]) : 0.0;
+        ps[b] = kin ? psi[(size_t)s * g.npts + pt[b]] : make_double2(0.0, 0.0);
+      }
+#pragma unroll
+      for (int b = 0; b < NB; ++b) {
+        if (b0 + b >= P) break;
+        double fx = (double)v[b0 + b].x * scale, fy = (double)v[b0 + b].y * scale;
+        if (MODE == 0) {
+          fx *= wp[b];
+          fy *= wp[b];
+          if (occ) {
+            const bool in = g2[b] <= ecut;
+            const double wt = in ? wocc * wp[b] * g2[b] : 0.0;
+            fx = in ? fx - wt * ps[b].x : 0.0;
+            fy = in ? fy - wt * ps[b].y : 0.0;
+            e_kin += in ? wt * (ps[b].x * ps[b].x + ps[b].y * ps[b].y) : 0.0;
+          }
+        }
+        if (pt[b] >= 0) fout[(size_t)s * g.npts + pt[b]] = make_double2(fx, fy);
+      }
+    }
+  }
+  if (MODE == 0 && occ) {
+    const double t = block_sum(e_kin, red);
+    if (threadIdx.x == 0) eke_part[(size_t)s * gridDim.x + blockIdx.x] = 0.5 * t;
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Plane passes between pencils and a real array (FP64, [s][z][y][x]): one block
+// per (plane, array).  G2R: pencils -> real (ADD: sign times it added to what is
+// there); else real -> pencils.
+template <typename T, int N, bool G2R, bool ADD = false>
+__global__ void __launch_bounds__(512, 1)
+k_two_real(const cplx<T>* __restrict__ pen, cplx<T>* __restrict__ pen_out,
+           const double* __restrict__ fin, double* __restrict__ fout, double sign, StateGeom g,
+           const cplx<T>* __restrict__ twx_g) {
+  using S = TwoShape<T, N>;
+  using R = TwoReal<T, N>;
+  using Pos = TwoPos<N>;
+  constexpr int P = S::P, Q = S::Q, QS = S::QS, LC = S::LC, LL = S::LL, G = R::G, NPAIR = N / 2;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  cplx<T>* tw1 = reinterpret_cast<cplx<T>*>(smem_raw);
+  cplx<T>* tw2 = tw1 + N;
+  cplx<T>* plane = tw2 + N;
+  const int nplx = g.nplane_x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  cplx<T>* scr = plane + (size_t)nplx * LC + (size_t)warp * G * LL;
+  const int z = blockIdx.x, s = blockIdx.y;
+  for (int i = tid; i < N; i += R::THREADS) {
+    tw1[i] = twx_g[(i / Q) * (i % Q)];
+    tw2[i] = twx_g[(i / P) * (i % P)];
+  }
+  if (G2R) {
+    for (int i = tid; i < nplx * LC; i += R::THREADS) plane[i] = mk<T>(0, 0);
+    __syncthreads();
+    const cplx<T>* row = pen + ((size_t)s * N + z) * g.nlpad;
+    for (int l = tid; l < g.nlines; l += R::THREADS) {
+      const int xy = __ldg(g.line_xy + l);
+      plane[(xy & 0xffff) * LC + Pos::s(xy >> 16)] = row[l];
+    }
+    __syncthreads();
+    for (int t = tid; t < nplx * Q; t += R::THREADS) {  // FFTW_FORWARD y
+      const int q = t % Q;
+      cplx<T>* col = plane + (t / Q) * LC + q;
+      cplx<T> v[P];
+#pragma unroll
+      for (int r = 0; r < P; ++r) v[r] = col[r * QS];
+      rdft<T, P, false>(v);
+      col[0] = v[0];
+#pragma unroll
+      for (int k = 1; k < P; ++k) col[k * QS] = cmul(v[k], tw1[k * Q + q]);
+    }
+    __syncthreads();
+    for (int t = tid; t < nplx * P; t += R::THREADS) {
+      cplx<T>* col = plane + (t / P) * LC + (t % P) * QS;
+      cplx<T> v[Q];
+#pragma unroll
+      for (int q = 0; q < Q; ++q) v[q] = col[q];
+      rdft<T, Q, false>(v);
+#pragma unroll
+      for (int m = 0; m < Q; ++m) col[m] = v[m];
+    }
+  }
+  __syncthreads();
+  for (int p0 = warp * G; p0 < NPAIR; p0 += R::W * G) {
+    const int np = min(G, NPAIR - p0);
+    const size_t base = (((size_t)s * N + z) * N + 2 * p0) * N;
+    if (G2R) {
+      for (int t = lane; t < np * Q; t += 32) {  // C2R, first stage (as k_two)
+        const int pi = t / Q, q = t % Q, y = 2 * (p0 + pi), ia = Pos::b(y), ib = Pos::b(y + 1);
+        cplx<T> v[P];
+#pragma unroll
+        for (int r = 0; r < P; ++r) {
+          const int x = q + Q * r;
+          cplx<T> zv = mk<T>(0, 0);
+          if (x == 0) {
+            zv = mk<T>(plane[ia].x, plane[ib].x);
+          } else if (x < nplx) {
+            const cplx<T> a = plane[x * LC + ia], b = plane[x * LC + ib];
+            zv = mk<T>(a.x + b.y, b.x - a.y);
+          } else if (N - x < nplx) {
+            const cplx<T> a = plane[(N - x) * LC + ia], b = plane[(N - x) * LC + ib];
+            zv = mk<T>(a.x - b.y, a.y + b.x);
+          }
+          v[r] = zv;
+        }
+        rdft<T, P, true>(v);
+        cplx<T>* o = scr + pi * LL + q;
+        o[0] = v[0];
+#pragma unroll
+        for (int k = 1; k < P; ++k) o[k * QS] = cmulc(v[k], tw1[k * Q + q]);
+      }
+      __syncwarp();
+      for (int t = lane; t < np * P; t += 32) {
+        const int pi = t / P, k = t % P;
+        const cplx<T>* e = scr + pi * LL + k * QS;
+        double* o = fout + base + (size_t)(2 * pi) * N + k;
+        double oa[Q], ob[Q];
+#pragma unroll
+        for (int m = 0; m < Q; ++m) {
+          oa[m] = ADD ? o[P * m] : 0.0;
+          ob[m] = ADD ? o[N + P * m] : 0.0;
+        }
+        cplx<T> v[Q];
+#pragma unroll
+        for (int q = 0; q < Q; ++q) v[q] = e[q];
+        rdft<T, Q, true>(v);
+#pragma unroll
+        for (int m = 0; m < Q; ++m) {
+          o[P * m] = ADD ? oa[m] + sign * (double)v[m].x : (double)v[m].x;
+          o[N + P * m] = ADD ? ob[m] + sign * (double)v[m].y : (double)v[m].y;
+        }
+      }
+    } else {
+      for (int t = lane; t < np * P; t += 32) {  // R2C (-i sign), first stage
+        const int pi = t / P, k = t % P;
+        const double* f = fin + base + (size_t)(2 * pi) * N + k;
+        cplx<T> v[Q];
+#pragma unroll
+        for (int m = 0; m < Q; ++m) v[m] = mk<T>((T)f[P * m], (T)f[N + P * m]);
+        rdft<T, Q, false>(v);
+        cplx<T>* e = scr + pi * LL + k * QS;
+        e[0] = v[0];
+#pragma unroll
+        for (int a = 1; a < Q; ++a) e[a] = cmul(v[a], tw2[a * P + k]);
+      }
+      __syncwarp();
+      for (int t = lane; t < np * Q; t += 32) {
+        cplx<T>* e = scr + (t / Q) * LL + t % Q;
+        cplx<T> v[P];
+#pragma unroll
+        for (int k = 0; k < P; ++k) v[k] = e[k * QS];
+        rdft<T, P, false>(v);
+#pragma unroll
+        for (int b = 0; b < P; ++b) e[b * QS] = v[b];
+      }
+      __syncwarp();
+      for (int pi = 0; pi < np; ++pi) {
+        const int y = 2 * (p0 + pi), ia = Pos::b(y), ib = Pos::b(y + 1);
+        const cplx<T>* e = scr + pi * LL;
+        for (int kx = lane; kx < nplx; kx += 32) {
+          const cplx<T> zk = e[Pos::s(kx)], zm = e[Pos::s(kx == 0 ? 0 : N - kx)];
+          plane[kx * LC + ia] = mk<T>((T)0.5 * (zk.x + zm.x), (T)0.5 * (zm.y - zk.y));
+          plane[kx * LC + ib] = mk<T>((T)0.5 * (zk.y + zm.y), (T)0.5 * (zk.x - zm.x));
+        }
+      }
+    }
+    __syncwarp();
+  }
+  if (G2R) return;
+  __syncthreads();
+  for (int t = tid; t < nplx * P; t += R::THREADS) {  // FFTW_BACKWARD y
+    const int k = t % P;
+    cplx<T>* col = plane + (t / P) * LC + k * QS;
+    cplx<T> v[Q];
+#pragma unroll
+    for (int m = 0; m < Q; ++m) v[m] = col[m];
+    rdft<T, Q, true>(v);
+    col[0] = v[0];
+#pragma unroll
+    for (int a = 1; a < Q; ++a) col[a] = cmulc(v[a], tw2[a * P + k]);
+  }
+  __syncthreads();
+  for (int t = tid; t < nplx * Q; t += R::THREADS) {
+    cplx<T>* col = plane + (t / Q) * LC + t % Q;
+    cplx<T> v[P];
+#pragma unroll
+    for (int k = 0; k < P; ++k) v[k] = col[k * QS];
+    rdft<T, P, true>(v);
+#pragma unroll
+    for (int b = 0; b < P; ++b) col[b * QS] = v[b];
+  }
+  __syncthreads();
+  cplx<T>* po = pen_out + ((size_t)s * N + z) * g.nlpad;
+  for (int l = tid; l < g.nlines; l += R::THREADS) {
+    const int xy = __ldg(g.line_xy + l);
+    po[l] = plane[(xy & 0xffff) * LC + Pos::s(xy >> 16)];
+  }
+}
+
 // sum, for every plane z, the partial densities of the blocks whose item
 // range touched it (block order: deterministic), scaled
 __global__ void k_rho_reduce_items(const double* __restrict__ part, int n, int nstates,
@@ -1669,6 +2013,17 @@ struct StateFft {
   static int zfft_fwd(cpstep_ctx* c, const FftJob& j, const double* psi, int nstates,
                       const cplx<T>* twz = nullptr, const double2* mul = nullptr) {
     dim3 grid(cdiv(j.g.nlines, ZShape<N>::LB), nstates);
+    if constexpr (TwoCfg<N>::ok) {
+      if (!mul) {
+        const size_t zs = TwoZ<T, N>::bytes();
+        if (int rc = set_smem(k_z2_fwd<T, N>, zs)) return rc;
+        k_z2_fwd<T, N><<<grid, TwoZ<T, N>::FWD, zs, c->stream>>>(
+            reinterpret_cast<const double2*>(psi), reinterpret_cast<cplx<T>*>(j.pen_a), j.g,
+            twz ? twz : tws<T>(c).z);
+        CPSTEP_LAUNCH_CHECK();
+        return CPSTEP_OK;
+      }
+    }
     const size_t smem = ZShape<N>::template bytes<T>();
     if (int rc = set_smem(k_zfft_fwd<T, N>, smem)) return rc;
     k_zfft_fwd<T, N><<<grid, ZTHREADS, smem, c->stream>>>(
@@ -1780,13 +2135,15 @@ struct StateFft {
   // packed G -> real r for nstates arrays of the job's geometry
   static int g2r(cpstep_ctx* c, const FftJob& j, const double* packed, double* real, int nstates) {
     if (int rc = zfft_fwd(c, j, packed, nstates)) return rc;
-    if constexpr (ShflCfg<N>::ok) {
-      const size_t smem = SShape<T, N>::bytes(j.g.nplane_x);
-      if (int rc = set_smem(k_xy_fwd_s<T, N, 1>, smem)) return rc;
-      k_xy_fwd_s<T, N, 1><<<dim3(N, nstates), PTHREADS, smem, c->stream>>>(
-          reinterpret_cast<const cplx<T>*>(j.pen_a), j.g, tws<T>(c).x, nullptr, nstates, 1, real);
-      CPSTEP_LAUNCH_CHECK();
-      return CPSTEP_OK;
+    if constexpr (TwoCfg<N>::ok) {
+      const size_t sm = TwoReal<T, N>::bytes(j.g.nplane_x);
+      if (sm <= PShape<T, N>::LIMIT) {
+        if (int rc = set_smem(k_two_real<T, N, true>, sm)) return rc;
+        k_two_real<T, N, true><<<dim3(N, nstates), TwoReal<T, N>::THREADS, sm, c->stream>>>(
+            reinterpret_cast<const cplx<T>*>(j.pen_a), nullptr, nullptr, real, 0.0, j.g, tws<T>(c).x);
+        CPSTEP_LAUNCH_CHECK();
+        return CPSTEP_OK;
+      }
     }
     const size_t smem = PShape<T, N>::bytes(j.g.nplane_x);
     if (smem > PShape<T, N>::LIMIT) return split_g2r(c, j, real, nstates);
@@ -1795,6 +2152,25 @@ struct StateFft {
         reinterpret_cast<const cplx<T>*>(j.pen_a), j.g, tws<T>(c).x, nullptr, nstates, 1, N,
         real);
     CPSTEP_LAUNCH_CHECK();
+    return CPSTEP_OK;
+  }
+
+  // real += sign (packed G -> real r) for one array; *done = false where only the
+  // storing form is built
+  static int g2r_add(cpstep_ctx* c, const FftJob& j, const double* packed, double* real,
+                     double sign, bool* done) {
+    *done = false;
+    if constexpr (TwoCfg<N>::ok && sizeof(T) == 8) {
+      const size_t sm = TwoReal<T, N>::bytes(j.g.nplane_x);
+      if (sm > PShape<T, N>::LIMIT) return CPSTEP_OK;
+      if (int rc = zfft_fwd(c, j, packed, 1)) return rc;
+      if (int rc = set_smem(k_two_real<T, N, true, true>, sm)) return rc;
+      k_two_real<T, N, true, true><<<dim3(N, 1), TwoReal<T, N>::THREADS, sm, c->stream>>>(
+          reinterpret_cast<const cplx<T>*>(j.pen_a), nullptr, nullptr, real, sign, j.g,
+          tws<T>(c).x);
+      CPSTEP_LAUNCH_CHECK();
+      *done = true;
+    }
     return CPSTEP_OK;
   }
 
@@ -1840,6 +2216,17 @@ struct StateFft {
   static int zfft_bwd(cpstep_ctx* c, const FftJob& j, double* out, const double* psi,
                       const double* occ, int nstates, double scale, int mode) {
     dim3 grid(cdiv(j.g.nlines, ZShape<N>::LB), nstates);
+    if constexpr (TwoCfg<N>::ok) {
+      const size_t zs = TwoZ<T, N>::bytes();
+      auto kern = mode == 0 ? k_z2_bwd<T, N, 0> : k_z2_bwd<T, N, 1>;
+      if (int rc = set_smem(kern, zs)) return rc;
+      kern<<<grid, TwoZ<T, N>::BWD, zs, c->stream>>>(
+          reinterpret_cast<const cplx<T>*>(j.pen_b), reinterpret_cast<double2*>(out),
+          reinterpret_cast<const double2*>(psi), occ, j.g, tws<T>(c).z, scale, c->ecut_ry,
+          c->d_eke_part);
+      CPSTEP_LAUNCH_CHECK();
+      return CPSTEP_OK;
+    }
     const size_t smem = ZShape<N>::template bytes<T>();
     if (mode == 0) {
       if (int rc = set_smem(k_zfft_bwd<T, N, 0>, smem)) return rc;
@@ -1925,23 +2312,25 @@ struct StateFft {
   // real r -> packed G (sum_r f(r) e^{+iG.r}) times scale, for the job's geometry
   static int r2g(cpstep_ctx* c, const FftJob& j, const double* f_r, double* fg, int nstates,
                  double scale) {
-    if constexpr (ShflCfg<N>::ok) {
-      const size_t smem = SShape<T, N>::bytes(j.g.nplane_x);
-      if (int rc = set_smem(k_xy_bwd_s<T, N, 1>, smem)) return rc;
-      k_xy_bwd_s<T, N, 1><<<dim3(N, nstates), PTHREADS, smem, c->stream>>>(
-          nullptr, f_r, nullptr, reinterpret_cast<cplx<T>*>(j.pen_b), j.g, tws<T>(c).x, nullptr,
-          nstates, 1);
-    } else {
-      const size_t smem = PShape<T, N>::bytes(j.g.nplane_x);
-      if (smem > PShape<T, N>::LIMIT) {
-        if (int rc = split_r2g(c, j, f_r, nstates)) return rc;
+    if constexpr (TwoCfg<N>::ok) {
+      const size_t sm = TwoReal<T, N>::bytes(j.g.nplane_x);
+      if (sm <= PShape<T, N>::LIMIT) {
+        if (int rc = set_smem(k_two_real<T, N, false>, sm)) return rc;
+        k_two_real<T, N, false><<<dim3(N, nstates), TwoReal<T, N>::THREADS, sm, c->stream>>>(
+            nullptr, reinterpret_cast<cplx<T>*>(j.pen_b), f_r, nullptr, 0.0, j.g, tws<T>(c).x);
+        CPSTEP_LAUNCH_CHECK();
         return zfft_bwd(c, j, fg, nullptr, nullptr, nstates, scale, 1);
       }
-      if (int rc = set_smem(k_xy_bwd<T, N, 1>, smem)) return rc;
-      k_xy_bwd<T, N, 1><<<dim3(N, nstates), PTHREADS, smem, c->stream>>>(
-          nullptr, f_r, nullptr, reinterpret_cast<cplx<T>*>(j.pen_b), j.g, tws<T>(c).x, nullptr,
-          nstates, 1);
     }
+    const size_t smem = PShape<T, N>::bytes(j.g.nplane_x);
+    if (smem > PShape<T, N>::LIMIT) {
+      if (int rc = split_r2g(c, j, f_r, nstates)) return rc;
+      return zfft_bwd(c, j, fg, nullptr, nullptr, nstates, scale, 1);
+    }
+    if (int rc = set_smem(k_xy_bwd<T, N, 1>, smem)) return rc;
+    k_xy_bwd<T, N, 1><<<dim3(N, nstates), PTHREADS, smem, c->stream>>>(
+        nullptr, f_r, nullptr, reinterpret_cast<cplx<T>*>(j.pen_b), j.g, tws<T>(c).x, nullptr,
+        nstates, 1);
     CPSTEP_LAUNCH_CHECK();
     return zfft_bwd(c, j, fg, nullptr, nullptr, nstates, scale, 1);
   }
@@ -2009,6 +2398,7 @@ struct StateFft {
     o.gtor = &gtor;
     o.rtog = &rtog;
     o.g2r = &g2r;
+    o.g2r_add = &g2r_add;
     o.r2g = &r2g;
     o.lb = ZShape<N>::LB;
     return o;

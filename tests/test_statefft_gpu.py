@@ -236,3 +236,34 @@ def test_two_stage_planes_match_stockham(grid, box, states, precision):
             assert relerr(a.cpu().numpy(), b.cpu().numpy()) < TOL[precision]
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("grid,box,states", [
+    (28, 9.0, 3), (32, 9.0, 1), (40, 12.0, 2), (42, 9.0, 7), (48, 12.0, 2), (60, 12.0, 3),
+    (64, 12.0, 1), (80, 12.0, 2), (96, 12.0, 1), (120, 12.0, 2), (128, 12.0, 1), (200, 12.0, 1)])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_line_and_real_passes_match_oracle(grid, box, states, precision):
+    """The z passes and the passes to and from a real array on every grid of the
+    two-stage form, with a ragged last block of lines.  The oracle tests'
+    tolerances."""
+    if not cuda_ok():
+        pytest.skip("no CUDA device")
+    import torch
+    from oracle import fftpath as OF
+    from oracle import layout as OL
+    from openatom_b200.context import StepContext
+    from openatom_b200.layout import StateLayout
+    lay = StateLayout(box, 20.0, nfft=grid)
+    olay = OL.Layout(box, 20.0, grid=grid)
+    g = torch.Generator(device="cuda").manual_seed(grid)
+    psi = torch.view_as_complex(torch.randn((states, lay.npts, 2), generator=g,
+                                            dtype=torch.float64, device="cuda"))
+    f = torch.randn((states, grid, grid, grid), generator=g, dtype=torch.float64, device="cuda")
+    ctx = StepContext(lay, states, precision=precision)
+    try:
+        pr = ctx.fft_g_to_r(psi).cpu().numpy()
+        assert relerr(pr, OF.state_g_to_r(psi.cpu().numpy(), olay)) < TOL[precision]
+        out = ctx.fft_r_to_g(f).cpu().numpy()
+        assert relerr(out, OF.state_r_to_g(f.cpu().numpy(), olay)) < TOL[precision]
+    finally:
+        ctx.close()
