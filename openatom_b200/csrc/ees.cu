@@ -442,11 +442,13 @@ __global__ void k_nl_zmat(const double* __restrict__ zpart, NlAtoms A, int ctype
 __global__ void k_nl_finish(const double* __restrict__ enl_s, const double* __restrict__ fnl,
                             int nstates, int natm, double* __restrict__ energies,
                             double* __restrict__ fatm) {
+  __shared__ double red[32];
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i == 0 && energies) {
+  if (blockIdx.x == 0 && energies) {
     double e = 0.0;
-    for (int s = 0; s < nstates; ++s) e += enl_s[s];
-    energies[CPSTEP_E_NL] = e;
+    for (int s = threadIdx.x; s < nstates; s += blockDim.x) e += enl_s[s];
+    e = block_sum(e, red);
+    if (i == 0) energies[CPSTEP_E_NL] = e;
   }
   if (fatm && i < 3 * natm) {
     double f = 0.0;

@@ -12,7 +12,7 @@
 //   dgemm:        column-major BLAS semantics, the myGEMM wrapper
 //                 (ckPairCalculator.C:57-66).
 //
-// The first two run on the FP64 tensor units, dgemm on FP64 SIMT tiles; the overlap is split over K (the
+// All three run on the FP64 tensor units; the overlap is split over K (the
 // reference's numChunks K-split, pcCommManager.C:165-172) with a fixed-order
 // reduction of the partial tiles, so results are deterministic.
 #include <algorithm>
@@ -79,99 +79,150 @@ k_overlap_part(const double* __restrict__ A, int lda, const double* __restrict__
     }
 }
 
-// sym (M == N): C = alpha (P + P^T) / 2 + beta C, summed in the same order for
-// (i,j) and (j,i) so the result is exactly symmetric.
-__global__ void k_splitk_reduce(const double* __restrict__ part, int nsplit, int M, int N,
-                                double alpha, double beta, double* __restrict__ C, int ldc,
-                                int sym, const double* __restrict__ diag) {
-  int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= M * N) return;
-  int j = e / M, i = e - j * M;
-  double s = 0.0;
-  if (diag && i == j) {  // the diagonal summed in FP64 elsewhere
-    s = diag[i];
-  } else if (sym) {
-    const size_t e1 = (size_t)min(i, j) * M + max(i, j), e2 = (size_t)max(i, j) * M + min(i, j);
-    double s1 = 0.0, s2 = 0.0;
-    for (int k = 0; k < nsplit; ++k) {
-      s1 += part[(size_t)k * M * N + e1];
-      s2 += part[(size_t)k * M * N + e2];
-    }
-    s = 0.5 * (s1 + s2);
-  } else {
-    for (int k = 0; k < nsplit; ++k) s += part[(size_t)k * M * N + e];
+// C = alpha sum_k part[k] + beta C; sym (M == N): the sum averaged with its
+// transpose, taken in the same order for (i,j) and (j,i) so the result is exactly
+// symmetric.  With G = 8 the partials of an element are added in eight groups by
+// eight threads, then the groups in order: one thread per element over ~150
+// partials is bound by the latency of its loads (two passes over them, groups
+// first, took 18 us for 148 partials of 128 x 128, this one 5).
+template <int G>
+__global__ void __launch_bounds__(256)
+k_splitk_reduce(const double* __restrict__ part, int nsplit, int M, int N, double alpha,
+                double beta, double* __restrict__ C, int ldc, int sym,
+                const double* __restrict__ diag) {
+  constexpr int E = 256 / G;  // elements per block
+  __shared__ double sh[2][G][E];
+  const int tx = threadIdx.x % E, g = threadIdx.x / E;
+  const long long e = (long long)blockIdx.x * E + tx;
+  const bool in = e < (long long)M * N;
+  const int j = in ? (int)(e / M) : 0, i = in ? (int)(e - (long long)j * M) : 0;
+  const bool onlyd = diag && i == j;  // the diagonal summed in FP64 elsewhere
+  double s1 = 0.0, s2 = 0.0;
+  if (in && !onlyd) {
+    const size_t mn = (size_t)M * N;
+    const int k0 = nsplit * g / G, k1 = nsplit * (g + 1) / G;
+    const size_t e1 = sym ? (size_t)min(i, j) * M + max(i, j) : (size_t)e;
+    const size_t e2 = (size_t)max(i, j) * M + min(i, j);
+#pragma unroll 8
+    for (int k = k0; k < k1; ++k) s1 += part[(size_t)k * mn + e1];
+    if (sym)
+#pragma unroll 8
+      for (int k = k0; k < k1; ++k) s2 += part[(size_t)k * mn + e2];
   }
+  if (G > 1) {
+    sh[0][g][tx] = s1;
+    sh[1][g][tx] = s2;
+    __syncthreads();
+    if (g) return;
+#pragma unroll
+    for (int q = 1; q < G; ++q) {
+      s1 += sh[0][q][tx];
+      s2 += sh[1][q][tx];
+    }
+  }
+  if (!in) return;
+  const double s = onlyd ? diag[i] : (sym ? 0.5 * (s1 + s2) : s1);
   double* c = C + (size_t)j * ldc + i;
   *c = alpha * s + (beta == 0.0 ? 0.0 : beta * (*c));
 }
 
-// First pass of a long split-K reduction (many partial tiles): group g of
-// the nsplit partials summed in order, part2[g][e] (G groups).  The second
-// pass is k_splitk_reduce over the G group sums; both orders are fixed.
-__global__ void k_splitk_group(const double* __restrict__ part, int nsplit, int G, size_t mn,
-                               double* __restrict__ part2) {
-  const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= mn) return;
-  const int g = blockIdx.y;
-  const int k0 = (int)((long long)nsplit * g / G), k1 = (int)((long long)nsplit * (g + 1) / G);
-  double s = 0.0;
-#pragma unroll 8
-  for (int k = k0; k < k1; ++k) s += part[(size_t)k * mn + e];
-  part2[(size_t)g * mn + e] = s;
+template <typename... A>
+static void splitk_reduce(cudaStream_t st, const double* part, int nsplit, int M, int N, A... a) {
+  const long long mn = (long long)M * N;
+  if (nsplit > 16)
+    k_splitk_reduce<8><<<(unsigned)((mn + 31) / 32), 256, 0, st>>>(part, nsplit, M, N, a...);
+  else
+    k_splitk_reduce<1><<<(unsigned)((mn + 255) / 256), 256, 0, st>>>(part, nsplit, M, N, a...);
 }
 
-// column-major C = alpha op(A) op(B) + beta C (reference DGEMM semantics)
-__global__ void __launch_bounds__(NT)
-k_dgemm(int ta, int tb, int m, int n, int k, double alpha, const double* __restrict__ A, int lda,
-        const double* __restrict__ B, int ldb, double beta, double* __restrict__ C, int ldc) {
-  __shared__ double As[BK][BM + 1];
-  __shared__ double Bs[BK][BN + 1];
-  const int i0 = blockIdx.x * BM, j0 = blockIdx.y * BN;
-  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-  double acc[4][4] = {};
-  for (int l0 = 0; l0 < k; l0 += BK) {
-    for (int e = threadIdx.x; e < BM * BK; e += NT) {
-      int r, c;
-      if (ta) { r = e / BK; c = e % BK; } else { c = e / BM; r = e % BM; }
-      int i = i0 + r, l = l0 + c;
-      double v = 0.0;
-      if (i < m && l < k) v = ta ? A[(size_t)i * lda + l] : A[(size_t)l * lda + i];
-      As[c][r] = v;
-    }
-    for (int e = threadIdx.x; e < BN * BK; e += NT) {
-      int r, c;
-      if (tb) { c = e / BN; r = e % BN; } else { r = e / BK; c = e % BK; }
-      int j = j0 + r, l = l0 + c;
-      double v = 0.0;
-      if (j < n && l < k) v = tb ? B[(size_t)l * ldb + j] : B[(size_t)j * ldb + l];
-      Bs[c][r] = v;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < BK; ++kk) {
-      double a[4], b[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        a[q] = As[kk][ty + 16 * q];
-        b[q] = Bs[kk][tx + 16 * q];
-      }
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-#pragma unroll
-        for (int r = 0; r < 4; ++r) acc[q][r] += a[q] * b[r];
-    }
-    __syncthreads();
+// column-major C = alpha op(A) op(B) + beta C (reference DGEMM semantics) on the
+// FP64 tensor units: a 32 x 32 tile per block, its eight warps sharing out each
+// 128-long K chunk (16 each) so that the S x S products of the step, 16 blocks at
+// 128 states, still keep eight warps per tile busy; the warps' tiles are added in
+// order.  An operand is kept as it lies: [x][k] where k is contiguous (op(A) = A^T,
+// op(B) = B), [k][x] otherwise, both with strides that spread the fragment
+// reads over the banks.  Sizes 128, 512, 2048: 27, 94, 1217 us on scalar FMAs in 64 x 64 tiles -> 14, 25, 1027.
+constexpr int DT = 32, DK = 128, DLK = DK + 8, DLX = DT + 2;
+constexpr int DOPND = DT * DLK;  // = DK * DLX doubles
+static_assert(DOPND == DK * DLX, "one operand size for both layouts");
+
+template <bool KC>  // k contiguous
+__device__ __forceinline__ void dg_load(const double* __restrict__ X, int ldx, int x0, int nx,
+                                        int k0, int k, double* s) {
+  for (int q = threadIdx.x; q < DT * DK; q += NT) {
+    const int x = KC ? q / DK : q % DT, l = KC ? q % DK : q / DT;
+    const bool ok = x0 + x < nx && k0 + l < k;
+    const size_t off = KC ? (size_t)(x0 + x) * ldx + k0 + l : (size_t)(k0 + l) * ldx + x0 + x;
+    tc::cp8(s + (KC ? x * DLK + l : l * DLX + x), X + (ok ? off : 0), ok ? 8 : 0);
   }
+}
+template <bool KC>
+__device__ __forceinline__ double2 dg_frag(const double* s, int x, int l) {
+  if (KC) return *reinterpret_cast<const double2*>(s + x * DLK + l);
+  return make_double2(s[l * DLX + x], s[(l + 1) * DLX + x]);
+}
+
+template <bool TA, bool TB>
+__global__ void __launch_bounds__(NT)
+k_dgemm(int m, int n, int k, double alpha, const double* __restrict__ A, int lda,
+        const double* __restrict__ B, int ldb, double beta, double* __restrict__ C, int ldc) {
+  extern __shared__ __align__(16) double sm[];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  const int tm = (m + DT - 1) / DT, nc = (k + DK - 1) / DK;
+  const int i0 = (int)(blockIdx.x % tm) * DT, j0 = (int)(blockIdx.x / tm) * DT;
+  double acc[4][4][2];
+  dm::zero(acc);
+  auto load = [&](int st, int c) {
+    double* s = sm + st * 2 * DOPND;
+    dg_load<TA>(A, lda, i0, m, c * DK, k, s);
+    dg_load<!TB>(B, ldb, j0, n, c * DK, k, s + DOPND);
+    tc::cp_commit();
+  };
+  if (nc > 0) load(0, 0);
+  for (int c = 0; c < nc; ++c) {
+    tc::cp_wait<0>();
+    __syncthreads();
+    if (c + 1 < nc) load((c + 1) & 1, c + 1);
+    if (c * DK + warp * 16 >= k) continue;
+    const double* s = sm + (c & 1) * 2 * DOPND;
 #pragma unroll
-  for (int q = 0; q < 4; ++q)
+    for (int kk = 0; kk < 2; ++kk) {
+      const int l = warp * 16 + kk * 8 + 2 * t;
+      double2 a[4], b[4];
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      int i = i0 + ty + 16 * q, j = j0 + tx + 16 * r;
-      if (i < m && j < n) {
-        double* c = C + (size_t)j * ldc + i;
-        *c = alpha * acc[q][r] + (beta == 0.0 ? 0.0 : beta * (*c));
+      for (int i = 0; i < 4; ++i) {
+        a[i] = dg_frag<TA>(s, i * 8 + g, l);
+        b[i] = dg_frag<!TB>(s + DOPND, i * 8 + g, l);
       }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) dm::mma884(acc[i][j], a[i].x, b[j].x);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) dm::mma884(acc[i][j], a[i].y, b[j].y);
     }
+  }
+  __syncthreads();  // the stages become the eight partial tiles, column-major
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+        sm[warp * DT * DT + (j * 8 + 2 * t + e) * DT + i * 8 + g] = acc[i][j][e];
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < DT * DT / NT; ++q) {
+    const int e = tid + NT * q, i = i0 + e % DT, j = j0 + e / DT;
+    if (i >= m || j >= n) continue;
+    double v = 0.0;
+#pragma unroll
+    for (int w = 0; w < NT / 32; ++w) v += sm[w * DT * DT + e];
+    double* o = C + (size_t)j * ldc + i;
+    *o = alpha * v + (beta == 0.0 ? 0.0 : beta * (*o));
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -433,34 +484,11 @@ int split_reserve(cpstep_ctx* c, size_t bytes) {
   return CPSTEP_OK;
 }
 
-// Partials beyond 32 are first summed in 16 groups (k_splitk_group) into the
-// tail of the partial buffer: one thread per element over ~150 partials is
-// bound by the latency of its loads.
-static int splitk_groups(int nsplit) { return nsplit > 32 ? 16 : 0; }
-
-size_t pc_part_need(int nsplit, size_t mn) {
-  return (size_t)(nsplit + splitk_groups(nsplit)) * mn;
-}
+size_t pc_part_need(int nsplit, size_t mn) { return (size_t)nsplit * mn; }
 
 int pc_splitk_reduce_launch(cpstep_ctx* c, int nsplit, int M, int N, double alpha, double beta,
                             double* C, int ldc, int sym, const double* diag) {
-  const size_t mn = (size_t)M * N;
-  const int G = splitk_groups(nsplit);
-  const double* part = c->d_pc_part;
-  if (G) {
-    if (c->pc_part_elems < pc_part_need(nsplit, mn)) {
-      cpstep_set_error("split-K reduction: partial buffer reserved without its group sums");
-      return CPSTEP_ERR_STATE;
-    }
-    double* part2 = c->d_pc_part + (size_t)nsplit * mn;
-    pcalc::k_splitk_group<<<dim3((unsigned)((mn + 255) / 256), G), 256, 0, c->stream>>>(
-        c->d_pc_part, nsplit, G, mn, part2);
-    CPSTEP_LAUNCH_CHECK();
-    part = part2;
-    nsplit = G;
-  }
-  pcalc::k_splitk_reduce<<<cdiv(M * N, 256), 256, 0, c->stream>>>(part, nsplit, M, N, alpha,
-                                                                   beta, C, ldc, sym, diag);
+  pcalc::splitk_reduce(c->stream, c->d_pc_part, nsplit, M, N, alpha, beta, C, ldc, sym, diag);
   CPSTEP_LAUNCH_CHECK();
   return CPSTEP_OK;
 }
@@ -539,8 +567,13 @@ int dgemm_launch(cudaStream_t s, int ta, int tb, int m, int n, int k, double alp
                  const double* A, int lda, const double* B, int ldb, double beta, double* C,
                  int ldc) {
   using namespace pcalc;
-  dim3 grid(cdiv(m, BM), cdiv(n, BN));
-  k_dgemm<<<grid, NT, 0, s>>>(ta, tb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc);
+  auto kern = ta ? (tb ? k_dgemm<true, true> : k_dgemm<true, false>)
+                 : (tb ? k_dgemm<false, true> : k_dgemm<false, false>);
+  const size_t smem = sizeof(double) * 2 * DOPND * (k > DK ? 2 : 1);
+  if (int rc = dyn_smem(kern, sizeof(double) * 4 * DOPND)) return rc;
+  const long long tiles = (long long)cdiv(m, DT) * cdiv(n, DT);
+  kern<<<(unsigned)tiles, NT, smem, s>>>(m, n, k, alpha, A, lda, B, ldb, beta, C,
+                                                        ldc);
   CPSTEP_LAUNCH_CHECK();
   return CPSTEP_OK;
 }
@@ -646,8 +679,7 @@ extern "C" int cpstep_pc_overlap_noalloc(const double* d_a, const double* d_b, i
   // every partial the reduction reads is written by this call: nothing to clear
   k_overlap_part<<<dim3(tm, tn, nsplit), NT, 0, s>>>(d_a, K, d_b, K, d_w, M, N, K, kslab, part);
   CPSTEP_LAUNCH_CHECK();
-  k_splitk_reduce<<<cdiv(M * N, 256), 256, 0, s>>>(part, nsplit, M, N, alpha, beta, d_c, ldc, 0,
-                                                    nullptr);
+  splitk_reduce(s, part, nsplit, M, N, alpha, beta, d_c, ldc, 0, (const double*)nullptr);
   CPSTEP_LAUNCH_CHECK();
   return CPSTEP_OK;
 }

@@ -377,11 +377,13 @@ k_hart_lines_rec(const double2* __restrict__ rhog_t, const int* __restrict__ lin
   }
 }
 
-// G = 0 (cp_hart_ext.C:345-368); single thread
+// G = 0 (cp_hart_ext.C:345-368); one warp
 __global__ void k_hart_g0(const double2* __restrict__ rhog_t, int izero, double vol, Atoms A,
                           double2* __restrict__ vg_t, double* __restrict__ eext) {
   double v = 0.0;
-  for (int i = 0; i < A.natm; ++i) v += A.gzvps[A.typ[i]];
+  for (int i = threadIdx.x; i < A.natm; i += 32) v += A.gzvps[A.typ[i]];
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if (threadIdx.x) return;
   v /= vol;
   vg_t[izero] = make_double2(v, 0.0);
   *eext += v * rhog_t[izero].x;
@@ -1237,7 +1239,7 @@ static int eesloc_hart(cpstep_ctx* c, double* energies, double* force) {
       r.rhog, r.line_off, r.nlines, r.kx, r.ky, r.kz, r.npts, c->d_hmati, c->vol, ecut4,
       ad.alp_ewd, A, r.vg, r.fterm, hp);
   CPSTEP_LAUNCH_CHECK();
-  rho::k_sum_cols<<<3, 256, 0, c->stream>>>(hp, r.nlines, 3, energies + CPSTEP_E_HART, 1.0);
+  rho::k_sum_cols<<<3, 1024, 0, c->stream>>>(hp, r.nlines, 3, energies + CPSTEP_E_HART, 1.0);
   CPSTEP_LAUNCH_CHECK();
   if (c->rho_izero >= 0) {
     rho::k_eloc_g0<<<1, 1, 0, c->stream>>>(r.rhog, c->rho_izero, c->vol, A, r.vg,
@@ -1296,10 +1298,10 @@ int rho_hart(cpstep_ctx* c, double* energies, double* force) {
         c->atoms.alp_ewd, A, r.vg, r.fterm, hp);
   }
   CPSTEP_LAUNCH_CHECK();
-  rho::k_sum_cols<<<3, 256, 0, c->stream>>>(hp, r.nlines, 3, energies + CPSTEP_E_HART, 1.0);
+  rho::k_sum_cols<<<3, 1024, 0, c->stream>>>(hp, r.nlines, 3, energies + CPSTEP_E_HART, 1.0);
   CPSTEP_LAUNCH_CHECK();
   if (c->rho_izero >= 0) {
-    rho::k_hart_g0<<<1, 1, 0, c->stream>>>(r.rhog, c->rho_izero, c->vol, A, r.vg,
+    rho::k_hart_g0<<<1, 32, 0, c->stream>>>(r.rhog, c->rho_izero, c->vol, A, r.vg,
                                            energies + CPSTEP_E_EXT);
     CPSTEP_LAUNCH_CHECK();
   }

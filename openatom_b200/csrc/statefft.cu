@@ -56,15 +56,15 @@ __global__ void k_rho_reduce_items(const double* __restrict__ part, int n, int n
   }
 }
 
-// per-state sum of block partials in a fixed order (deterministic)
+// per-state sum of block partials in a fixed order (deterministic), a warp each
 __global__ void k_rowsum(const double* __restrict__ part, int ncol, int nrow,
                          double* __restrict__ out) {
-  int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r < nrow) {
-    double a = 0.0;
-    for (int c = 0; c < ncol; ++c) a += part[(size_t)r * ncol + c];
-    out[r] = a;
-  }
+  const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (r >= nrow) return;
+  double a = 0.0;
+  for (int c = lane; c < ncol; c += 32) a += part[(size_t)r * ncol + c];
+  for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+  if (lane == 0) out[r] = a;
 }
 
 __global__ void k_to_float(const double* __restrict__ in, float* __restrict__ out, size_t n) {

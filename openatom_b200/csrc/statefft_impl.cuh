@@ -2303,7 +2303,7 @@ struct StateFft {
     if (int rc = zfft_bwd(c, j, force, psi, eke ? occ : nullptr, c->nstates, scale, 0)) return rc;
     if (eke) {
       int nblk = cdiv(j.g.nlines, ZShape<N>::LB);
-      k_rowsum<<<cdiv(c->nstates, 128), 128, 0, c->stream>>>(c->d_eke_part, nblk, c->nstates, eke);
+      k_rowsum<<<cdiv(c->nstates, 4), 128, 0, c->stream>>>(c->d_eke_part, nblk, c->nstates, eke);
       CPSTEP_LAUNCH_CHECK();
     }
     return CPSTEP_OK;

@@ -111,9 +111,11 @@ __global__ void k_sum(const double* __restrict__ part, int n, double* __restrict
 // energies[KE] = sum eke[s]; energies[TOT] = KE + NL + HART + EXT + EXC
 __global__ void k_energy_tot(const double* __restrict__ eke, int nstates,
                              double* __restrict__ e) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    double k = 0.0;
-    for (int s = 0; s < nstates; ++s) k += eke[s];
+  __shared__ double red[32];
+  double k = 0.0;
+  for (int s = threadIdx.x; s < nstates; s += blockDim.x) k += eke[s];
+  k = block_sum(k, red);
+  if (threadIdx.x == 0) {
     e[CPSTEP_E_KE] = k;
     e[CPSTEP_E_TOT] = k + e[CPSTEP_E_NL] + e[CPSTEP_E_HART] + e[CPSTEP_E_EXT] + e[CPSTEP_E_EXC];
   }
@@ -127,10 +129,13 @@ __global__ void k_norb_check(const double* __restrict__ S, int n, double tol, in
                              int* __restrict__ flags, double* __restrict__ dev) {
   __shared__ double red[32];
   double m = 0.0;
-  const int nn = n * n;
-  for (int i = threadIdx.x; i < nn; i += blockDim.x) {
-    const double a = fabs(S[i] - ((i % n) == (i / n) ? 2.0 : 0.0));
-    m = (a > m || a != a) ? a : m;
+  const int w0 = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  for (int i = threadIdx.x & 31; i < n; i += 32) {  // a warp walks columns w0, w0 + nw, ..
+#pragma unroll 8
+    for (int j = w0; j < n; j += nw) {
+      const double a = fabs(S[(size_t)j * n + i] - (i == j ? 2.0 : 0.0));
+      m = (a > m || a != a) ? a : m;
+    }
   }
   for (int o = 16; o > 0; o >>= 1) {
     const double b = __shfl_xor_sync(0xffffffffu, m, o);
@@ -366,7 +371,7 @@ int step_run(cpstep_ctx* c, double* psi, double* vpsi, const double* occ, double
   } else {
     CPSTEP_CUDA_TRY(cudaMemsetAsync(energies + CPSTEP_E_NL, 0, sizeof(double), c->stream));
   }
-  stp::k_energy_tot<<<1, 32, 0, c->stream>>>(c->d_eke, S, energies);
+  stp::k_energy_tot<<<1, 256, 0, c->stream>>>(c->d_eke, S, energies);
   CPSTEP_LAUNCH_CHECK();
   mark(4);
   const int K = 2 * c->npts;

@@ -185,3 +185,25 @@ def test_ortho_tile_edges(pc, n, mixed):
                                       tol=2e-6 if mixed else 1e-13, max_iter=12)
     T = T.cpu().numpy()
     assert np.max(np.abs(T.T @ (S / 2) @ T - np.eye(n))) < 1e-12
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 1, 1), (32, 33, 15), (31, 32, 128), (64, 1, 129), (97, 65, 16),
+                                   (128, 128, 300)])
+def test_dgemm_tile_edges(pc, m, n, k):
+    """Edges of the 32 x 32 tiles, of a warp's 16 and a chunk's 128 of K, leading
+    dimensions beyond the matrices, beta = 0 over NaN.  At most 300 terms of
+    order 1: rounding below 300 eps times a few: 1e-12."""
+    import torch
+    rng = np.random.default_rng(m * 1000 + n)
+    for ta in "NT":
+        for tb in "NT":
+            A = rng.standard_normal((m + 3, k) if ta == "N" else (k + 3, m))
+            B = rng.standard_normal((k + 5, n) if tb == "N" else (n + 5, k))
+            opA = A[:m] if ta == "N" else A[:k].T
+            opB = B[:k] if tb == "N" else B[:n].T
+            dA, dB = (torch.from_numpy(np.ascontiguousarray(x.T)).cuda() for x in (A, B))
+            dC = torch.full((n, m + 1), float("nan"), dtype=torch.float64, device="cuda")
+            pc["ctx"].dgemm(ta, tb, m, n, k, -0.5, dA, A.shape[0], dB, B.shape[0], 0.0, dC, m + 1)
+            got = dC.cpu().numpy()
+            assert np.max(np.abs(got[:, :m].T + 0.5 * opA @ opB)) < 1e-12
+            assert np.isnan(got[:, m]).all()
