@@ -178,7 +178,7 @@ struct PreArgs {
   const double* w;    // weight per complex point k / 2 (a power of two), or none
   int zero_diag;      // element (i, i) taken as zero
   uint8_t* dst;       // [row tile][step][level][4 KB]
-  uint8_t* dst2;      // the unweighted levels as well (the B operand of S), or none
+  uint8_t* dst2;      // k_presplit_s: the unweighted levels (the B operand of S)
 };
 
 // One warp = 16 rows x 16 reals of one K step and row tile: lane -> row
@@ -228,11 +228,6 @@ __global__ void __launch_bounds__(256) k_presplit(const PreArgs a) {
   }
   float f[8];
   const size_t off = ((size_t)rt * a.nsp + s) * STEP_B + core_off(rl, 8 * kh);
-  if (a.dst2) {
-    const float one[4] = {1.f, 1.f, 1.f, 1.f};
-    to_f32(x, one, f);
-    split_store(a.dst2 + off, f);
-  }
   to_f32(x, ws, f);
   split_store(a.dst + off, f);
 }
@@ -1228,21 +1223,59 @@ __global__ void __launch_bounds__(PP_NTHR, 1) k_pp_tc(const PPArgs p) {
   if (failed && tid == 0) atomicOr(p.err, 1);
 }
 
-// The diagonal of S = overlap(psi, psi) for the many-state overlap: the
-// FP64 row sums of w x^2, one block per row (fixed order).
-__global__ void __launch_bounds__(256) k_rowdot(const double* __restrict__ src, long long ldr,
-                                                int K, const double* __restrict__ w,
-                                                double* __restrict__ diag) {
-  __shared__ double red[32];
-  const double* x = src + (size_t)blockIdx.x * ldr;
+// The images of S = overlap(psi, psi) for many states, w psi and psi, and the
+// FP64 row sums of w x^2 (S's diagonal) from one read of psi: k_presplit's
+// mapping, a warp walking RD_STEPS K steps of its 16 rows with the rows' sums in
+// registers; part[range][row], added in range order by k_rowdot_sum.  (As a
+// pass of its own the diagonal took 139 us for 512 states x 60,000 points, a
+// second read of psi at 3.5 TB/s.)
+constexpr int RD_STEPS = 32;
+__global__ void __launch_bounds__(256) k_presplit_s(const PreArgs a, double* __restrict__ part) {
+  const int lane = threadIdx.x & 31, gp = threadIdx.x >> 5;  // 8 warps: the 8 row pairs of a tile
+  const int nr = (a.nsp + RD_STEPS - 1) / RD_STEPS;
+  const int rg = blockIdx.x % nr;
+  const long long rt = blockIdx.x / nr;
+  const int rl = (lane & 7) + 8 * (lane >> 4) + 16 * gp;
+  const int kh = (lane >> 3) & 1;
+  const long long row = rt * ROWS + rl;
+  const bool live = row < a.rows;
+  const int s1 = min(a.nsp, (rg + 1) * RD_STEPS);
   double d = 0.0;
-  for (int k2 = threadIdx.x; 2 * k2 < K; k2 += blockDim.x) {  // point k2: reals 2 k2, 2 k2 + 1
-    const double2 v = *reinterpret_cast<const double2*>(x + 2 * k2);
-    const double ww = w ? w[k2] : 1.0;
-    d = fma(ww * v.x, v.x, fma(ww * v.y, v.y, d));
+#pragma unroll 2
+  for (int s = rg * RD_STEPS; s < s1; ++s) {
+    const int k0 = 16 * s + 8 * kh;
+    double x[8];
+    float ws[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {  // K even: points are inside or outside
+      const bool ok = live && k0 + 2 * e < a.K;
+      const double2 v = ok ? *reinterpret_cast<const double2*>(a.src + row * a.ldr + k0 + 2 * e)
+                           : make_double2(0.0, 0.0);
+      const double w = ok ? (a.w ? a.w[(k0 >> 1) + e] : 1.0) : 1.0;
+      x[2 * e] = v.x;
+      x[2 * e + 1] = v.y;
+      ws[e] = (float)w;
+      d = fma(w * v.x, v.x, fma(w * v.y, v.y, d));
+    }
+    float f[8];
+    const float one[4] = {1.f, 1.f, 1.f, 1.f};
+    const size_t off = ((size_t)rt * a.nsp + s) * STEP_B + core_off(rl, 8 * kh);
+    to_f32(x, one, f);
+    split_store(a.dst2 + off, f);
+    to_f32(x, ws, f);
+    split_store(a.dst + off, f);
   }
-  d = block_sum(d, red);
-  if (threadIdx.x == 0) diag[blockIdx.x] = d;
+  d += __shfl_xor_sync(0xffffffffu, d, 8);  // the two K halves of a row
+  if (kh == 0 && live) part[(size_t)rg * a.rows + row] = d;
+}
+__global__ void k_rowdot_sum(const double* __restrict__ part, int nr, int rows,
+                             double* __restrict__ diag) {
+  const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (r >= rows) return;
+  double d = 0.0;
+  for (int q = lane; q < nr; q += 32) d += part[(size_t)q * rows + r];
+  for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+  if (lane == 0) diag[r] = d;
 }
 
 // A of a many-state back-multiply: in^T (rows = the points' reals p, K =
@@ -1674,9 +1707,9 @@ static int hlv_reserve(cpstep_ctx* c, int i, size_t bytes) {
 
 // C = alpha overlap(a, b) + beta C for many states (M, N >= 256): both
 // operands split once in global memory into their three BF16 levels
-// (k_presplit; S's two images, w psi and psi, from one read of psi), the
+// (k_presplit; S's two images, w psi and psi, by k_presplit_s), the
 // product streamed by k_pp_tc<3> (six level products, FP64 folds every 128
-// reals), S's diagonal summed in FP64 (k_rowdot).  The in-CTA split of
+// reals), S's diagonal summed in FP64 with the split (k_presplit_s).  The in-CTA split of
 // k_pc_tc re-reads and re-splits each operand once per tile row or column of
 // the output.
 static int overlap_stream(cpstep_ctx* c, const double* a, const double* b, int M, int N, int K,
@@ -1686,23 +1719,25 @@ static int overlap_stream(cpstep_ctx* c, const double* a, const double* b, int M
   const int nsp = pre_nsp(K);
   if (int rc = hlv_reserve(c, 0, pre_bytes(M, K))) return rc;
   if (int rc = hlv_reserve(c, 1, pre_bytes(N, K))) return rc;
-  if (same && (size_t)M > c->pdiag_elems) {
+  const int nr = cdiv(nsp, RD_STEPS);
+  if (same && (size_t)M * (nr + 1) > c->pdiag_elems) {
     graph_drop(c);
     cudaFree(c->d_pdiag);
     c->d_pdiag = nullptr;
     c->pdiag_elems = 0;
-    CPSTEP_CUDA_TRY(cudaMalloc(&c->d_pdiag, sizeof(double) * M));
-    c->pdiag_elems = M;
-  }
-  if (same) {
-    k_rowdot<<<M, 256, 0, c->stream>>>(a, K, K, w, c->d_pdiag);
-    CPSTEP_LAUNCH_CHECK();
+    CPSTEP_CUDA_TRY(cudaMalloc(&c->d_pdiag, sizeof(double) * M * (nr + 1)));
+    c->pdiag_elems = (size_t)M * (nr + 1);
   }
   PreArgs pa{a, K, M, K, nsp, w, 0, c->d_hlv[0], same ? c->d_hlv[1] : nullptr};
-  const long long ta = (long long)cdiv(M, ROWS) * nsp * 8 * 32;
-  k_presplit<<<(unsigned)((ta + 255) / 256), 256, 0, c->stream>>>(pa);
-  CPSTEP_LAUNCH_CHECK();
-  if (!same) {
+  if (same) {
+    k_presplit_s<<<(unsigned)(cdiv(M, ROWS) * nr), 256, 0, c->stream>>>(pa, c->d_pdiag + M);
+    CPSTEP_LAUNCH_CHECK();
+    k_rowdot_sum<<<cdiv(M, 8), 256, 0, c->stream>>>(c->d_pdiag + M, nr, M, c->d_pdiag);
+    CPSTEP_LAUNCH_CHECK();
+  } else {
+    const long long ta = (long long)cdiv(M, ROWS) * nsp * 8 * 32;
+    k_presplit<<<(unsigned)((ta + 255) / 256), 256, 0, c->stream>>>(pa);
+    CPSTEP_LAUNCH_CHECK();
     PreArgs pb{b, K, N, K, nsp, nullptr, 0, c->d_hlv[1], nullptr};
     const long long tb = (long long)cdiv(N, ROWS) * nsp * 8 * 32;
     k_presplit<<<(unsigned)((tb + 255) / 256), 256, 0, c->stream>>>(pb);
