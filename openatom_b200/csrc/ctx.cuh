@@ -206,9 +206,13 @@ struct NlData {
   std::vector<int> tab_cap;
   // G-space evaluation of the same sums (mixed contexts on the tensor cores,
   // ees_gspace_run): per atom separable transforms, S matrices (FP32) of each
-  // type [v][atom of type][ld_s], each type's channels with contiguous dyp
+  // type [atom of type][ld_s], each type's channels with contiguous dyp
   int km = 0;                       // largest |k| of the state sphere on an axis
   double2* sep = nullptr;           // [natm][3][2][2 km + 1]
+  float2* sepf = nullptr;           // the same in FP32, [axis][m][k][rank] (atom forces)
+  int2* kw = nullptr;               // [npts, padded to 64] kx | ky << 16, kz
+  uint8_t *psi_t = nullptr, *af_z = nullptr;  // atom forces: levels of psi and zs, transposed
+  double* af_part = nullptr;        // their partial sums [blocks][atoms of two types][3]
   float* sv = nullptr;              // per type at sv_off[t]
   long long ld_s = 0;               // floats per S row (2 npts rounded up to 4)
   std::vector<long long> sv_off;
@@ -217,8 +221,9 @@ struct NlData {
   std::vector<float> tdmax;         // largest |dyp| of each type's channels (FP16 scales)
   std::vector<std::vector<float>> tdmax_c;  // the same per channel of the type
   float* d_hmax = nullptr;          // [2][ntyp] bound of |S| (Mn rows) and largest |Z| entry
-                                    // per type (float bits, atomicMax), written every pass
-  // FP16 levels of the S rows of every type (rows v natm_t + a, the pre-split
+                                    // per type, then the largest |component| of psi (float
+                                    // bits, atomicMax), written every pass
+  // FP16 levels of the S rows of every type (row a, the pre-split
   // image) at blv + blv_off[t], their scales and inverses at tsc / tinv +
   // tsoff[t]; the A operand of the sums (w psi dyp_c) at alv
   uint8_t* blv = nullptr;
@@ -234,7 +239,7 @@ struct NlData {
   int* d_order = nullptr;           // atom of each type-order rank
   int* d_tch = nullptr;             // [ntyp][4] channel indices (-1 unused)
   double* d_vn = nullptr;           // [nchan] vnorm / vol
-  double* csum = nullptr;           // sums of one type [nch 4 natm_t][nstates]
+  double* csum = nullptr;           // sums of one type [nch natm_t][nstates]
   double* zt = nullptr;             // scaled Z of two types, [nstates][ldz] each
   size_t zt_slot = 0;               // doubles per type
   int gspace_ok = 0;                // every type has at most 4 channels
@@ -522,12 +527,19 @@ struct EesForceType {
 };
 int ees_tc_force_pre(cpstep_ctx* c, int ntyp, const EesForceType* ty, int ld_d, double alpha,
                      double* fpsi, size_t zlv_bytes, size_t stlv_bytes);
+int ees_tc_atom_force(cpstep_ctx* c, int ntyp, const EesForceType* ty, const int* rank0,
+                      const double* psi, const float* pmax, bool split_psi,
+                      const float2* sep, int km, const int2* kw, int ld_d, uint8_t* psi_t,
+                      uint8_t* zlv, double* fpart, int* nblk);
+int ees_af_blocks(const cpstep_ctx* c, int na);
+size_t ees_psit_bytes(int nstates, int npts);
+size_t ees_ztlv_bytes(int nstates, int na);
 size_t ees_pf_zbytes(int nstates, int natm_t);
 size_t ees_pf_stbytes(int npts, int natm_t);
 size_t ees_lv_bytes(int rows, int K);
 int ees_tc_presplit_a(cpstep_ctx* c, const double* psi, int ntyp, const float2* const* dyp,
                       int ld_d, const int* nch, const float* const* dmax, uint8_t* const* alv,
-                      size_t alv_bytes);
+                      size_t alv_bytes, float* pmax);
 int ees_tc_sums_pre(cpstep_ctx* c, int nch, const float* dmax, const uint8_t* blv, int jp,
                     const float* cinv, const uint8_t* alv, double* C);
 int pc_splitk_reduce_launch(cpstep_ctx* c, int nsplit, int M, int N, double alpha, double beta,

@@ -17,6 +17,7 @@
 // scatters Z Mn and starts the R->G transform, and K4 adding the psi force.
 // The projector dyp depends on the cell only and is formed once at set-up.
 #include <algorithm>
+#include <cstring>
 #include <cmath>
 #include <vector>
 #include "ctx.cuh"
@@ -218,7 +219,8 @@ k_nl_table(NlAtoms A, int nkf, TabDims d, int* __restrict__ tcell, NlVal* __rest
 // separable transforms [atom][axis][Mn, dMn][k + km], k in [-km, km]
 __global__ void k_ees_sep(const int* __restrict__ ig, const double* __restrict__ mn,
                           const double* __restrict__ dmn, int natm, int nkf, int km,
-                          double2* __restrict__ sep) {
+                          double2* __restrict__ sep, const int* __restrict__ rank,
+                          float2* __restrict__ sepf) {
   const int nk = 2 * km + 1;
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (long long)natm * 6 * nk) return;
@@ -239,6 +241,8 @@ __global__ void k_ees_sep(const int* __restrict__ ig, const double* __restrict__
     im -= f[j] * sn;
   }
   sep[i] = make_double2(re, im);
+  if (sepf)  // [axis][m][k][rank]
+    sepf[((long long)(2 * d + m) * nk + kk) * natm + rank[a]] = make_float2((float)re, (float)im);
 }
 
 struct TypeDims {
@@ -252,157 +256,122 @@ __device__ __forceinline__ double2 cm(double2 a, double2 b) {
   return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
 
-// Bounds of |S| of the rows (v, a) of every atom from the per-axis maxima of
-// its separable transforms: |S| is their product, the gradient rows are
-// bounded by the triangle inequality.  tsc = pow2_scale(bound) scales the
-// row's FP16 levels, tinv = 1 / tsc; smax[t] gets the largest Mn-row bound of
-// the type (float bits of a non-negative value, atomicMax).  One warp per atom.
+// Bounds of |S| of the Mn rows from the per-axis maxima of the atoms' separable
+// transforms (|S| is their product).  tsc = pow2_scale(bound) scales the row's
+// FP16 levels, tinv = 1 / tsc; smax[t] gets the largest bound of the type (float
+// bits of a non-negative value, atomicMax).  One warp per atom.
 __global__ void k_ees_bound(const double2* __restrict__ sep, int natm, int km,
                             const int* __restrict__ typ, const int* __restrict__ rank,
-                            TypeDims td, NlAtoms A, float* __restrict__ tsc,
-                            float* __restrict__ tinv, unsigned int* __restrict__ smax) {
+                            TypeDims td, float* __restrict__ tsc, float* __restrict__ tinv,
+                            unsigned int* __restrict__ smax) {
   const int a = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (a >= natm) return;
   const int nk = 2 * km + 1;
   const double2* T = sep + (size_t)a * 6 * nk;
-  double m[6];
+  double b = 1.0;
 #pragma unroll
-  for (int q = 0; q < 6; ++q) {
+  for (int d = 0; d < 3; ++d) {
     double mx = 0.0;
     for (int k = lane; k < nk; k += 32) {
-      const double2 v = T[q * nk + k];
+      const double2 v = T[2 * d * nk + k];
       mx = fmax(mx, hypot(v.x, v.y));
     }
     for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    m[q] = mx;
+    b *= mx;
   }
   if (lane == 0) {
-    const int t = typ[a];
-    const int nt = td.tstart[t + 1] - td.tstart[t], al = rank[a] - td.tstart[t];
-    double b[4];
-    b[0] = m[0] * m[2] * m[4];
-    const double* h = A.hmati;
-    for (int v = 0; v < 3; ++v) {
-      const double h0 = fabs(h[3 * v] * A.grid), h1 = fabs(h[3 * v + 1] * A.grid),
-                   h2 = fabs(h[3 * v + 2] * A.grid);
-      b[v + 1] = m[1] * m[2] * m[4] * h0 + m[0] * m[3] * m[4] * h1 + m[0] * m[2] * m[5] * h2;
-    }
-    for (int v = 0; v < 4; ++v) {
-      const float sc = tc::pow2_scale((float)b[v]);
-      tsc[td.tsoff[t] + v * nt + al] = sc;
-      tinv[td.tsoff[t] + v * nt + al] = 1.f / sc;
-    }
-    atomicMax(smax + t, __float_as_uint((float)b[0]));
+    const int t = typ[a], al = rank[a] - td.tstart[t];
+    const float sc = tc::pow2_scale((float)b);
+    tsc[td.tsoff[t] + al] = sc;
+    tinv[td.tsoff[t] + al] = 1.f / sc;
+    atomicMax(smax + t, __float_as_uint((float)b));
   }
 }
 
-// S matrices, 4 points per thread: the Mn rows in FP32 (row a of the type, for
-// the psi force) and every row (v natm_t + a, v = Mn, d/dx, d/dy, d/dz) as
-// scaled FP16 levels in the pre-split image (nsp K steps per 128-row tile)
-// for the sums.  Lane i of a warp is the atom of type-order rank 8 y + (i & 7)
-// (y = blockIdx.y) at point quad (i >> 3) of the warp: the 8 atoms' 16-byte
-// pieces of a K half are one 128-byte core matrix when their rows are 8-aligned.
+// S matrices, 4 points per thread: the Mn rows (row a of the type) in FP32 for
+// the psi force and as scaled FP16 levels in the pre-split image (nsp K steps
+// per 128-row tile) for the sums.  Lane i of a warp is the atom of type-order
+// rank 8 y + (i & 7) (y = blockIdx.y) at point quad (i >> 3) of the warp: the 8
+// atoms' 16-byte pieces of a K half are one 128-byte core matrix when their
+// rows are 8-aligned.
 __global__ void __launch_bounds__(256) k_ees_smat(
     const double2* __restrict__ sep, const int* __restrict__ kx, const int* __restrict__ ky,
     const int* __restrict__ kz, int npts, int km, const int* __restrict__ typ,
-    const int* __restrict__ order, int natm, TypeDims td, NlAtoms A, long long ld_s,
+    const int* __restrict__ order, int natm, TypeDims td, long long ld_s,
     float* __restrict__ sv, const float* __restrict__ tsc, uint8_t* __restrict__ blv, int nsp) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int ra = blockIdx.y * 8 + (lane & 7);
   const int p0 = 4 * ((blockIdx.x * 8 + warp) * 4 + (lane >> 3));
   if (ra >= natm || p0 >= npts) return;
   const int a = order[ra];
-  const int t = typ[a];
-  const int nt = td.tstart[t + 1] - td.tstart[t], al = ra - td.tstart[t];
+  const int t = typ[a], al = ra - td.tstart[t];
   const int nk = 2 * km + 1;
-  const double2* T = sep + (size_t)a * 6 * nk;
-  const double* h = A.hmati;
-  const double g = A.grid;
-  float lv[4][8];
+  const double2* T = sep + (size_t)a * 6 * nk + km;
+  float lv[8];
   float* base = sv + td.svoff[t] + (size_t)al * ld_s;
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
     const int p = p0 + e;
-    if (p < npts) {
-      const int ix = kx[p] + km, iy = ky[p] + km, iz = kz[p] + km;
-      const double2 sa = T[0 * nk + ix], da = T[1 * nk + ix];
-      const double2 sb = T[2 * nk + iy], db = T[3 * nk + iy];
-      const double2 sc = T[4 * nk + iz], dc = T[5 * nk + iz];
-      const double2 sbc = cm(sb, sc);
-      const double2 S = cm(sa, sbc);
-      const double2 at = cm(da, sbc), bt = cm(sa, cm(db, sc)), ct = cm(cm(sa, sb), dc);
-      lv[0][2 * e] = (float)S.x;
-      lv[0][2 * e + 1] = (float)S.y;
-#pragma unroll
-      for (int v = 0; v < 3; ++v) {
-        const double h0 = h[3 * v] * g, h1 = h[3 * v + 1] * g, h2 = h[3 * v + 2] * g;
-        lv[v + 1][2 * e] = (float)(at.x * h0 + bt.x * h1 + ct.x * h2);
-        lv[v + 1][2 * e + 1] = (float)(at.y * h0 + bt.y * h1 + ct.y * h2);
-      }
-    } else {
-#pragma unroll
-      for (int v = 0; v < 4; ++v) lv[v][2 * e] = lv[v][2 * e + 1] = 0.f;
-    }
+    double2 S = make_double2(0.0, 0.0);
+    if (p < npts) S = cm(T[kx[p]], cm(T[2 * nk + ky[p]], T[4 * nk + kz[p]]));
+    lv[2 * e] = (float)S.x;
+    lv[2 * e + 1] = (float)S.y;
   }
   if (p0 + 3 < npts) {
-    *reinterpret_cast<float4*>(base + 2 * p0) = make_float4(lv[0][0], lv[0][1], lv[0][2], lv[0][3]);
-    *reinterpret_cast<float4*>(base + 2 * p0 + 4) =
-        make_float4(lv[0][4], lv[0][5], lv[0][6], lv[0][7]);
+    *reinterpret_cast<float4*>(base + 2 * p0) = make_float4(lv[0], lv[1], lv[2], lv[3]);
+    *reinterpret_cast<float4*>(base + 2 * p0 + 4) = make_float4(lv[4], lv[5], lv[6], lv[7]);
   } else {
     for (int e = 0; p0 + e < npts; ++e)
-      reinterpret_cast<float2*>(base)[p0 + e] = make_float2(lv[0][2 * e], lv[0][2 * e + 1]);
+      reinterpret_cast<float2*>(base)[p0 + e] = make_float2(lv[2 * e], lv[2 * e + 1]);
   }
   // reals 2 p0 .. 2 p0 + 7: K step p0 / 8, half (p0 / 4) & 1
-  uint8_t* bt0 = blv + td.bloff[t];
-#pragma unroll
-  for (int v = 0; v < 4; ++v) {
-    const int j = v * nt + al;
-    tc::split_store_h(bt0 + ((size_t)(j >> 7) * nsp + (p0 >> 3)) * (2 * tc::CM_TILE) +
-                          tc::core_off(j & 127, 8 * ((p0 >> 2) & 1)),
-                      lv[v], tsc[td.tsoff[t] + j]);
-  }
+  tc::split_store_h(blv + td.bloff[t] + ((size_t)(al >> 7) * nsp + (p0 >> 3)) * (2 * tc::CM_TILE) +
+                        tc::core_off(al & 127, 8 * ((p0 >> 2) & 1)),
+                    lv, tsc[td.tsoff[t] + al]);
 }
 
-// Z, E_NL, scaled Z and atom forces of one type from its G-space sums
-// C(s, ch jp + v nt + a) (column-major, ld = nstates): as k_nl_zmat.
+// Z, E_NL and scaled Z of one type from its G-space sums C(s, ch nt + a)
+// (column-major, ld = nstates): as k_nl_zmat.
 __global__ void k_ees_zglue(const double* __restrict__ C, int nstates, int nt, int nch,
                             const int* __restrict__ chan, const double* __restrict__ vnc,
-                            const int* __restrict__ order, int t0, int natm,
                             const double* __restrict__ occ, double* __restrict__ zt, int ldz,
-                            double* __restrict__ enl_s, double* __restrict__ fnl,
-                            unsigned int* __restrict__ zmax) {
+                            double* __restrict__ enl_s, unsigned int* __restrict__ zmax) {
   __shared__ double red[32];
   const int s = blockIdx.x;
   const double w = occ[s];
-  const int jp = 4 * nt;
   double e = 0.0;
   float zm = 0.f;  // largest |scaled Z| (float bits into *zmax, as k_ees_smat)
-  for (int al = threadIdx.x; al < nt; al += blockDim.x) {
-    const int atom = order[t0 + al];
-    double f0 = 0.0, f1 = 0.0, f2 = 0.0;
-    for (int ch = 0; ch < nch; ++ch) {
-      const double vn = vnc[chan[ch]];
-      const double* cc = C + ((size_t)ch * jp + al) * nstates + s;
-      const double z = cc[0];
-      const double dx = cc[(size_t)nt * nstates], dy = cc[(size_t)2 * nt * nstates];
-      const double dz = cc[(size_t)3 * nt * nstates];
-      e += z * z * vn * w;
-      const double zsc = z * (2.0 * vn * w);
-      zt[(size_t)s * ldz + ch * nt + al] = zsc;
-      zm = fmaxf(zm, (float)fabs(zsc));
-      f0 -= dx * zsc;
-      f1 -= dy * zsc;
-      f2 -= dz * zsc;
-    }
-    double* f = fnl + ((size_t)s * natm + atom) * 3;
-    f[0] += f0;
-    f[1] += f1;
-    f[2] += f2;
+  for (int i = threadIdx.x; i < nch * nt; i += blockDim.x) {
+    const double vn = vnc[chan[i / nt]];
+    const double z = C[(size_t)i * nstates + s];
+    e += z * z * vn * w;
+    const double zsc = z * (2.0 * vn * w);
+    zt[(size_t)s * ldz + i] = zsc;
+    zm = fmaxf(zm, (float)fabs(zsc));
   }
   for (int o = 16; o > 0; o >>= 1) zm = fmaxf(zm, __shfl_xor_sync(0xffffffffu, zm, o));
   if ((threadIdx.x & 31) == 0 && zm > 0.f) atomicMax(zmax, __float_as_uint(zm));
   e = block_sum(e, red);
   if (threadIdx.x == 0) enl_s[s] += e;
+}
+
+// fatm -= the Cartesian sums of a pair's atoms from their lattice-axis partials;
+// one warp per atom, lanes over the blocks
+__global__ void k_ees_atoms(const double* __restrict__ part, int nblk, int nat0, int na, int rank0,
+                            int rank1, const int* __restrict__ order, NlAtoms A,
+                            double* __restrict__ fatm) {
+  const int al = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (al >= na) return;
+  double f[3] = {0.0, 0.0, 0.0};
+  for (int b = lane; b < nblk; b += 32)
+#pragma unroll
+    for (int d = 0; d < 3; ++d) f[d] += part[((size_t)b * na + al) * 3 + d];
+#pragma unroll
+  for (int d = 0; d < 3; ++d)
+    for (int o = 16; o > 0; o >>= 1) f[d] += __shfl_xor_sync(0xffffffffu, f[d], o);
+  if (lane >= 3) return;
+  fatm[3 * (size_t)order[al < nat0 ? rank0 + al : rank1 + al - nat0] + lane] -=
+      A.grid * (f[0] * A.hmati[3 * lane] + f[1] * A.hmati[3 * lane + 1] + f[2] * A.hmati[3 * lane + 2]);
 }
 
 // Z_a = sum over the atom's planes, E_NL += Z^2 vn occ, Z <- 2 vn occ Z,
@@ -550,6 +519,7 @@ void nl_free(cpstep_ctx* c) {
   n.sep = nullptr; n.sv = nullptr; n.d_order = nullptr; n.d_tch = nullptr; n.d_vn = nullptr;
   n.csum = nullptr; n.zt = nullptr; n.gspace_ok = 0;
   cudaFree(n.plist); cudaFree(n.pcount);
+  cudaFree(n.sepf); cudaFree(n.kw); cudaFree(n.psi_t); cudaFree(n.af_z); cudaFree(n.af_part);
   cudaFree(n.e64_act); cudaFree(n.e64_part); cudaFree(n.e64_zs); cudaFree(n.e64_e);
   cudaFree(n.e64_f);
   n = NlData();
@@ -761,13 +731,34 @@ int nl_set(cpstep_ctx* c, int nkf, int n_interp, int nchan, const int* ch_type, 
     for (int t = 0; t < at.ntyp; ++t) {
       const int nt = at.tstart[t + 1] - at.tstart[t];
       n.sv_off[t] = tot;
-      tot += 4LL * nt * n.ld_s;
-      csz = std::max(csz, (size_t)n.tch[t].size() * 4 * nt * c->nstates);
+      tot += (long long)nt * n.ld_s;
+      csz = std::max(csz, (size_t)n.tch[t].size() * nt * c->nstates);
       zsz = std::max(zsz, (size_t)c->nstates * (((size_t)n.tch[t].size() * nt + 1) / 2 * 2));
     }
     CPSTEP_CUDA_TRY(cudaMalloc(&n.sv, sizeof(float) * (size_t)std::max(tot, 4LL)));
     CPSTEP_CUDA_TRY(cudaMemset(n.sv, 0, sizeof(float) * (size_t)std::max(tot, 4LL)));
     CPSTEP_CUDA_TRY(cudaMalloc(&n.sep, sizeof(double2) * na * 6 * (2 * (size_t)km + 1)));
+    CPSTEP_CUDA_TRY(cudaMalloc(&n.sepf, sizeof(float2) * na * 6 * (2 * (size_t)km + 1)));
+    {
+      std::vector<int2> kw((c->npts + 63) / 64 * 64, make_int2(0, 0));
+      for (int p = 0; p < c->npts; ++p)
+        kw[p] = make_int2((int)((unsigned)(c->h_kx[p] & 0xffff) | (unsigned)c->h_ky[p] << 16),
+                          c->h_kz[p]);
+      CPSTEP_CUDA_TRY(cudaMalloc(&n.kw, sizeof(int2) * kw.size()));
+      CPSTEP_CUDA_TRY(cudaMemcpy(n.kw, kw.data(), sizeof(int2) * kw.size(), cudaMemcpyHostToDevice));
+      int two = 1;  // atoms of two types at most, and their partials' rows
+      size_t rows = 1;
+      for (int t = 0; t < at.ntyp; ++t)
+        for (int u = 0; u <= t; ++u) {
+          const int a2 = at.tstart[t + 1] - at.tstart[t] + (u < t ? at.tstart[u + 1] - at.tstart[u] : 0);
+          if (a2 < 1) continue;
+          two = std::max(two, a2);
+          rows = std::max(rows, (size_t)ees_af_blocks(c, a2) * a2);
+        }
+      CPSTEP_CUDA_TRY(cudaMalloc(&n.psi_t, ees_psit_bytes(c->nstates, c->npts)));
+      CPSTEP_CUDA_TRY(cudaMalloc(&n.af_z, ees_ztlv_bytes(c->nstates, two)));
+      CPSTEP_CUDA_TRY(cudaMalloc(&n.af_part, sizeof(double) * 3 * rows));
+    }
     CPSTEP_CUDA_TRY(cudaMalloc(&n.csum, sizeof(double) * csz));
     n.zt_slot = zsz;  // two types at a time
     CPSTEP_CUDA_TRY(cudaMalloc(&n.zt, sizeof(double) * 2 * zsz));
@@ -775,7 +766,7 @@ int nl_set(cpstep_ctx* c, int nkf, int n_interp, int nchan, const int* ch_type, 
     n.tdmax.assign(at.ntyp, 0.f);
     n.tdmax_c.assign(at.ntyp, std::vector<float>(4, 0.f));
     n.ld_d32 = (c->npts + 1) / 2 * 2;
-    CPSTEP_CUDA_TRY(cudaMalloc(&n.d_hmax, sizeof(float) * 2 * std::max(1, at.ntyp)));
+    CPSTEP_CUDA_TRY(cudaMalloc(&n.d_hmax, sizeof(float) * (2 * std::max(1, at.ntyp) + 1)));
     std::vector<int> htch((size_t)at.ntyp * 4, -1);
     for (int t = 0; t < at.ntyp; ++t) {
       const size_t nc = n.tch[t].size();
@@ -811,8 +802,8 @@ int nl_set(cpstep_ctx* c, int nkf, int n_interp, int nchan, const int* ch_type, 
         const int nt = at.tstart[t + 1] - at.tstart[t];
         n.blv_off[t] = bl;
         n.tsoff[t] = ts;
-        bl += ees_lv_bytes(std::max(1, 4 * nt), K);
-        ts += 4LL * nt;
+        bl += ees_lv_bytes(std::max(1, nt), K);
+        ts += nt;
         nchmax = std::max(nchmax, (int)n.tch[t].size());
       }
       CPSTEP_CUDA_TRY(cudaMalloc(&n.blv, bl));
@@ -858,7 +849,8 @@ static int ees_sep_run(cpstep_ctx* c) {
   if (int rc = ees_bspline_launch(c, c->atoms.frac, n.natm, n.nkf, n.ig, n.mn, n.dmn)) return rc;
   const long long nsep = (long long)n.natm * 6 * (2 * n.km + 1);
   ees::k_ees_sep<<<(unsigned)((nsep + 255) / 256), 256, 0, c->stream>>>(n.ig, n.mn, n.dmn, n.natm,
-                                                                         n.nkf, n.km, n.sep);
+                                                                         n.nkf, n.km, n.sep, c->atoms.rank,
+                                                                         n.sepf);
   CPSTEP_LAUNCH_CHECK();
   return CPSTEP_OK;
 }
@@ -883,22 +875,22 @@ static int ees_gspace_run(cpstep_ctx* c, const double* psi, const double* occ, d
   A.grid = (double)n.nkf;
   // bounds of |S| (the FP16 scales of the S rows' levels) and the largest |Z|
   // entry per type (the psi force's)
-  CPSTEP_CUDA_TRY(cudaMemsetAsync(n.d_hmax, 0, sizeof(float) * 2 * ntyp, c->stream));
+  CPSTEP_CUDA_TRY(cudaMemsetAsync(n.d_hmax, 0, sizeof(float) * (2 * ntyp + 1), c->stream));
   unsigned int* smax_u = reinterpret_cast<unsigned int*>(n.d_hmax);
   unsigned int* zmax_u = smax_u + ntyp;
   ees::k_ees_bound<<<cdiv(32 * natm, 256), 256, 0, c->stream>>>(
-      n.sep, natm, n.km, c->atoms.typ, c->atoms.rank, td, A, n.tsc, n.tinv, smax_u);
+      n.sep, natm, n.km, c->atoms.typ, c->atoms.rank, td, n.tsc, n.tinv, smax_u);
   CPSTEP_LAUNCH_CHECK();
   const int nsp_s = cdiv(2 * c->npts, 32) * 2;  // K steps of a pre-split row tile
   ees::k_ees_smat<<<dim3(cdiv(c->npts, 128), cdiv(natm, 8)), 256, 0, c->stream>>>(
-      n.sep, c->d_kx, c->d_ky, c->d_kz, c->npts, n.km, c->atoms.typ, n.d_order, natm, td, A,
+      n.sep, c->d_kx, c->d_ky, c->d_kz, c->npts, n.km, c->atoms.typ, n.d_order, natm, td,
       n.ld_s, n.sv, n.tsc, n.blv, nsp_s);
   CPSTEP_LAUNCH_CHECK();
   CPSTEP_CUDA_TRY(cudaMemsetAsync(n.enl_s, 0, sizeof(double) * S, c->stream));
-  CPSTEP_CUDA_TRY(cudaMemsetAsync(n.fnl, 0, sizeof(double) * S * natm * 3, c->stream));
   // the types with projectors, two at a time: A of both split from one read of psi
   std::vector<int> tl;
   EesForceType ft[2];
+  int rank0[2] = {0, 0};
   for (int t = 0; t < ntyp; ++t)
     if (!n.tch[t].empty() && c->atoms.tstart[t + 1] > c->atoms.tstart[t]) tl.push_back(t);
   for (size_t q = 0; q < tl.size(); ++q) {
@@ -917,28 +909,39 @@ static int ees_gspace_run(cpstep_ctx* c, const double* psi, const double* occ, d
         dm[k] = n.tdmax_c[tl[q + k]].data();
         nc[k] = (int)n.tch[tl[q + k]].size();
       }
-      if (int rc = ees_tc_presplit_a(c, psi, np2, dy, n.ld_d32, nc, dm, al, n.alv_bytes)) return rc;
+      if (int rc = ees_tc_presplit_a(c, psi, np2, dy, n.ld_d32, nc, dm, al, n.alv_bytes,
+                                     n.d_hmax + 2 * ntyp))
+        return rc;
     }
-    if (int rc = ees_tc_sums_pre(c, nch, n.tdmax_c[t].data(), n.blv + n.blv_off[t], 4 * nt,
+    if (int rc = ees_tc_sums_pre(c, nch, n.tdmax_c[t].data(), n.blv + n.blv_off[t], nt,
                                  n.tinv + n.tsoff[t], alv, n.csum))
       return rc;
     const int ldz = (nch * nt + 1) / 2 * 2;
     double* zt = n.zt + (q & 1) * n.zt_slot;
-    ees::k_ees_zglue<<<S, 128, 0, c->stream>>>(n.csum, S, nt, nch, n.d_tch + 4 * t, n.d_vn,
-                                                n.d_order, c->atoms.tstart[t], natm, occ, zt, ldz,
-                                                n.enl_s, n.fnl, zmax_u + t);
+    ees::k_ees_zglue<<<S, 128, 0, c->stream>>>(n.csum, S, nt, nch, n.d_tch + 4 * t, n.d_vn, occ,
+                                                zt, ldz, n.enl_s, zmax_u + t);
     CPSTEP_LAUNCH_CHECK();
     ft[q & 1] = EesForceType{n.sv + n.sv_off[t], n.ld_s, n.tdyp[t], nch, nt, zt, ldz,
                              n.d_hmax + t, n.d_hmax + ntyp + t, n.pf_z + (q & 1) * n.pf_zbytes,
                              n.pf_st + (q & 1) * n.pf_stbytes};
-    // the psi force of the pair (F read and written once for both types)
-    if (q % 2 == 1 || q + 1 == tl.size())
-      if (int rc = ees_tc_force_pre(c, (int)(q % 2) + 1, ft, n.ld_d32, -1.0, fpsi, n.pf_zbytes,
-                                    n.pf_stbytes))
+    rank0[q & 1] = c->atoms.tstart[t];
+    if (q % 2 == 0 && q + 1 < tl.size()) continue;
+    // the pair's psi force (F read and written once for both types) and atom forces
+    const int np2 = (int)(q % 2) + 1;
+    if (int rc = ees_tc_force_pre(c, np2, ft, n.ld_d32, -1.0, fpsi, n.pf_zbytes, n.pf_stbytes))
+      return rc;
+    if (fatm) {
+      int nblk = 0;
+      if (int rc = ees_tc_atom_force(c, np2, ft, rank0, psi, n.d_hmax + 2 * ntyp, q < 2, n.sepf, n.km, n.kw, n.ld_d32,
+                                     n.psi_t, n.af_z, n.af_part, &nblk))
         return rc;
+      const int na2 = ft[0].natm_t + (np2 > 1 ? ft[1].natm_t : 0);
+      ees::k_ees_atoms<<<cdiv(na2, 4), 128, 0, c->stream>>>(
+          n.af_part, nblk, ft[0].natm_t, na2, rank0[0], np2 > 1 ? rank0[1] : 0, n.d_order, A, fatm);
+      CPSTEP_LAUNCH_CHECK();
+    }
   }
-  ees::k_nl_finish<<<cdiv(std::max(1, 3 * natm), 128), 128, 0, c->stream>>>(
-      n.enl_s, n.fnl, S, natm, energies, fatm);
+  ees::k_nl_finish<<<1, 128, 0, c->stream>>>(n.enl_s, nullptr, S, natm, energies, nullptr);
   CPSTEP_LAUNCH_CHECK();
   return CPSTEP_OK;
 }

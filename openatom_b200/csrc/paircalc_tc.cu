@@ -1325,6 +1325,7 @@ struct PreA {
   float sig[2][4];
   uint8_t* dst[2];
   int* err;
+  unsigned int* pmax;  // largest |component| of psi (float bits, atomicMax)
 };
 __global__ void __launch_bounds__(256) k_presplit_ees_a(const PreA a) {
   const long long wid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -1340,7 +1341,7 @@ __global__ void __launch_bounds__(256) k_presplit_ees_a(const PreA a) {
   const int kh = (lane >> 3) & 1;
   const int s = rt * ROWS + sl;
   const int k0 = 16 * st + 8 * kh;  // first real; 4 points from k0 / 2
-  float xr[4], xi[4];
+  float xr[4], xi[4], mx = 0.f;
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
     const int pt = (k0 >> 1) + e;
@@ -1348,9 +1349,12 @@ __global__ void __launch_bounds__(256) k_presplit_ees_a(const PreA a) {
     const double2 x = ok ? *reinterpret_cast<const double2*>(a.psi + (size_t)s * a.K + 2 * pt)
                          : make_double2(0.0, 0.0);
     const float ws = ok ? (float)a.w[pt] : 0.f;
+    mx = fmaxf(mx, fmaxf(fabsf((float)x.x), fabsf((float)x.y)));
     xr[e] = (float)x.x * ws;
     xi[e] = (float)x.y * ws;
   }
+  const unsigned int mb = __reduce_max_sync(0xffffffffu, __float_as_uint(mx));
+  if (lane == 0 && mb > *(volatile unsigned int*)a.pmax) atomicMax(a.pmax, mb);
   bool big = false;
 #pragma unroll
   for (int t = 0; t < 2; ++t) {
@@ -1418,20 +1422,38 @@ struct PFArgs {
   double alpha;
   double* f;             // [S][2 npts] (+=)
   int* err;
+  // ATOM: rows 4 a + c of the atoms of one or two types (nat[0] + nat[1] of them,
+  // type-order ranks from rank0[t]); one operand pair in a[0], b[0], nks[0]
+  int nat[2], rank0[2];
+  const float* pmax;     // the psi levels' scale is pow2_scale(*pmax)
+  const float2* sep;     // [axis][Mn, dMn][k + km][rank]
+  int km, natm;
+  const int2* kw;        // per point: kx | ky << 16, kz (zero past npts)
+  double* fpart;         // [gridDim.x][nat[0] + nat[1]][3]
 };
 
+// ATOM: the atom-force sums of the EES pass with the same streaming and
+// accumulators.  D = A B^T with A = zs transposed (rows 4 a + c, K = states) and
+// B = psi transposed (rows = reals of the points), so a row is
+// G_ac(p) = sum_s zs(s, ac) psi_s(p); the epilogue adds the four channel lanes
+// of an atom, P_a = sum_c dyp_c G_ac, and lane c < 3 sums
+// w Re(conj(P_a) dS_a) of lattice axis c over the points in FP64 (FP32 within
+// 16 points): fpart.  One product of the size of Z, where sums with the three
+// gradients of S took three.
+template <bool ATOM>
 __global__ void __launch_bounds__(PP_NTHR, 1) k_pf_tc(const PFArgs p) {
   extern __shared__ uint8_t dsm[];
   __shared__ uint64_t full[PF_NST], empty[PF_NST], gfull[2], tfree[2];
   __shared__ uint32_t tslot;
   __shared__ int stop_s, issued_s, req_s;
+  __shared__ double fred[ATOM ? 4 : 1][ATOM ? ROWS : 1];  // ATOM: sums of the column groups
   volatile int* stop = &stop_s;
   const uint32_t s0 = tc::smem_u32(dsm);
   uint8_t* base = dsm + (((s0 + 1023u) & ~1023u) - s0);
   const uint32_t base_s = tc::smem_u32(base);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int m = blockIdx.y;
-  const int ntyp = p.ntyp;
+  const int ntyp = ATOM ? 1 : p.ntyp;
   const int nkc0 = (p.nks[0] + PF_KS - 1) / PF_KS;                   // K chunks per tile, type 0
   const int nkc1 = ntyp > 1 ? (p.nks[1] + PF_KS - 1) / PF_KS : 0;    // type 1
   // this CTA's point tiles: blockIdx.x, + gridDim.x, ...
@@ -1533,6 +1555,83 @@ __global__ void __launch_bounds__(PP_NTHR, 1) k_pf_tc(const PFArgs p) {
       issued_s = it;
     }
     __syncwarp();
+  } else if (ATOM) {
+    const int rl = 32 * (warp & 3) + lane, rg = m * ROWS + rl;
+    const int al = rg >> 2, c = rg & 3;
+    const bool atom = al < p.nat[0] + p.nat[1];
+    const int t = al >= p.nat[0];
+    // the tables are [k][rank]: a warp's 8 atoms at one k are one 64-byte piece
+    const int rank = atom ? (t ? p.rank0[1] + al - p.nat[0] : p.rank0[0] + al) : 0;
+    const long long nk = 2 * p.km + 1;
+    const float2* T = p.sep + (long long)p.km * p.natm + rank;
+    const float2* Tx = T + (c == 0 ? nk * p.natm : 0);
+    const float2* Ty = T + (c == 1 ? 3 : 2) * nk * p.natm;
+    const float2* Tz = T + (c == 2 ? 5 : 4) * nk * p.natm;
+    const bool live = atom && c < (t ? p.nch[1] : p.nch[0]);
+    const float2* dyp = (t ? p.dyp[1] : p.dyp[0]) + (size_t)c * p.ld_d;
+    const float ri = 1.f / (tc::pow2_scale(t ? *p.zmax[1] : *p.zmax[0]) * tc::pow2_scale(*p.pmax));
+    double fsum = 0.0;
+    int bad = 0, cxy = 0x7fff7fff;  // a line's kx, ky; none yet
+    float ax = 0.f, ay = 0.f;       // its x and y factors times weight and scale
+    for (int tl = 0; tl < ntl && !bad; ++tl) {
+      const int acc = tl & 1;
+      if (!__all_sync(0xffffffffu, tc::mbar_wait_fast(&gfull[acc], (tl >> 1) & 1, stop))) {
+        bad = 1;
+        break;
+      }
+      tc::fence_after_sync();
+      const int n = blockIdx.x + tl * gridDim.x;
+      const int pt0 = (n * ROWS + 32 * (warp >> 2)) >> 1;  // 16 points
+      float f = 0.f;
+#pragma unroll
+      for (int hf = 0; hf < 2; ++hf) {  // 8 points (16 columns) at a time
+        const int p8 = pt0 + 8 * hf;
+        // every load of the 8 points is in flight before the first is used
+        int2 k[8];
+        float2 d[8], z[8];
+        const int4* kq = reinterpret_cast<const int4*>(p.kw + p8);  // padded to whole tiles
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int4 q = __ldg(kq + e);
+          k[2 * e] = make_int2(q.x, q.y);
+          k[2 * e + 1] = make_int2(q.z, q.w);
+        }
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+          d[e] = (live && p8 + e < p.npts) ? __ldg(dyp + p8 + e) : make_float2(0.f, 0.f);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) z[e] = __ldg(Tz + (long long)k[e].y * p.natm);
+        uint32_t v[16];
+        tc::tmem_ld16(tbase + tlanes + (uint32_t)(2 * acc * ROWS + 32 * (warp >> 2) + 16 * hf), v);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          const float qx = __uint_as_float(v[2 * e]), qy = __uint_as_float(v[2 * e + 1]);
+          float px = fmaf(d[e].x, qx, -d[e].y * qy), py = fmaf(d[e].x, qy, d[e].y * qx);
+          px += __shfl_xor_sync(0xffffffffu, px, 1);
+          py += __shfl_xor_sync(0xffffffffu, py, 1);
+          px += __shfl_xor_sync(0xffffffffu, px, 2);
+          py += __shfl_xor_sync(0xffffffffu, py, 2);
+          if (k[e].x != cxy) {  // the same for every lane
+            cxy = k[e].x;
+            const float2 x = Tx[(long long)(short)cxy * p.natm], y = Ty[(long long)(cxy >> 16) * p.natm];
+            const float w = (short)cxy == 0 ? ri : 2.f * ri;
+            ax = w * fmaf(x.x, y.x, -x.y * y.y);
+            ay = w * fmaf(x.x, y.y, x.y * y.x);
+          }
+          const float dx = fmaf(ax, z[e].x, -ay * z[e].y), dy = fmaf(ax, z[e].y, ay * z[e].x);
+          f = fmaf(px, dx, fmaf(py, dy, f));
+        }
+      }
+      fsum += (double)f;
+      tc::fence_before_sync();
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&tfree[acc]);
+    }
+    fred[ATOM ? warp >> 2 : 0][ATOM ? rl : 0] = fsum;
+    if (tc::bar_or(WBAR, NW, bad)) *stop = 1;  // also orders fred among the workers
+    if (warp < 4 && atom && c < 3)
+      p.fpart[((size_t)blockIdx.x * (p.nat[0] + p.nat[1]) + al) * 3 + c] =
+          (fred[0][rl] + fred[ATOM ? 1 : 0][rl]) + (fred[ATOM ? 2 : 0][rl] + fred[ATOM ? 3 : 0][rl]);
   } else {
     // rows 4 s + c of this warp's lanes; columns (reals) 32 (warp / 4).. of the tile
     const int rl = 32 * (warp & 3) + lane;
@@ -1650,11 +1749,40 @@ __global__ void k_presplit_z(const double* __restrict__ zt, int ldz, int S, int 
                 f, sc);
 }
 
+// zs transposed for the atom forces: rows 4 a + c of the atoms of two types
+// (zero for c >= nch), K = states (zero past S).  One thread = 8 states.
+struct ZtArgs {
+  const double* zt[2];  // type t: [S][ldz[t]], inner index c nat[t] + a
+  int ldz[2], nat[2], nch[2];
+  const float* zmax[2];
+};
+__global__ void k_presplit_zt(const ZtArgs z, int S, int nks, int nrow, uint8_t* __restrict__ dst) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= (long long)nrow * nks * 2) return;
+  const int r = (int)(i % nrow), u = (int)(i / nrow);
+  const int al = r >> 2, c = r & 3, t = al >= z.nat[0];
+  const int a = t ? al - z.nat[0] : al, nat = t ? z.nat[1] : z.nat[0];
+  const bool live = a < nat && c < (t ? z.nch[1] : z.nch[0]);
+  const double* src = (t ? z.zt[1] : z.zt[0]) + (live ? c * nat + a : 0);
+  const int ldz = t ? z.ldz[1] : z.ldz[0];
+  const float sc = live ? tc::pow2_scale(t ? *z.zmax[1] : *z.zmax[0]) : 1.f;
+  float f[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    const int s = 8 * u + e;
+    f[e] = live && s < S ? (float)src[(size_t)s * ldz] : 0.f;
+  }
+  split_store_h(dst + ((size_t)(r / ROWS) * nks + (u >> 1)) * STEP_H + core_off(r % ROWS, 8 * (u & 1)),
+                f, sc);
+}
+
 // The real views of a type's Mn rows transposed for k_pf_tc: rows = reals k of
 // the points (zero past 2 npts), K = atoms (zero past natm_t), from the FP32
 // rows sv[a ld_s + k], scaled by pow2_scale(*smax).  One thread = 8 atoms of
-// one real.
-__global__ void k_presplit_st(const float* __restrict__ sv, long long ld_s, int kr, int natm_t,
+// one real.  With T = double and states for
+// atoms: psi transposed for the atom forces.
+template <typename T>
+__global__ void k_presplit_st(const T* __restrict__ sv, long long ld_s, int kr, int natm_t,
                               int nks, int nrow, const float* __restrict__ smax,
                               uint8_t* __restrict__ dst) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1666,7 +1794,7 @@ __global__ void k_presplit_st(const float* __restrict__ sv, long long ld_s, int 
 #pragma unroll
   for (int e = 0; e < 8; ++e) {
     const int a = 8 * u + e;
-    f[e] = (k < kr && a < natm_t) ? sv[(size_t)a * ld_s + k] : 0.f;
+    f[e] = (k < kr && a < natm_t) ? (float)sv[(size_t)a * ld_s + k] : 0.f;
   }
   split_store_h(dst + ((size_t)(k / ROWS) * nks + (u >> 1)) * STEP_H + core_off(k % ROWS, 8 * (u & 1)),
                 f, sc);
@@ -1779,10 +1907,11 @@ size_t ees_lv_bytes(int rows, int K) {
 static float ees_sig(const float* dmax, int c) { return tc::pow2_scale(4.f * dmax[c]); }
 
 // A of the EES sums of ntyp (1 or 2) atom types, split from one read of psi
-// into alv[t] (rows c S + s = w psi_s dyp_{t,c}, scale ees_sig(dmax[t], c)).
+// into alv[t] (rows c S + s = w psi_s dyp_{t,c}, scale ees_sig(dmax[t], c)); *pmax
+// is raised to the largest |component| of psi.
 int ees_tc_presplit_a(cpstep_ctx* c, const double* psi, int ntyp, const float2* const* dyp,
                       int ld_d, const int* nch, const float* const* dmax, uint8_t* const* alv,
-                      size_t alv_bytes) {
+                      size_t alv_bytes, float* pmax) {
   using namespace pctc;
   const int S = c->nstates, K = 2 * c->npts, nsp = pre_nsp(K);
   if (ntyp < 1 || ntyp > 2 || (ld_d & 1) || !al16(psi)) return CPSTEP_ERR_ARG;
@@ -1804,6 +1933,7 @@ int ees_tc_presplit_a(cpstep_ctx* c, const double* psi, int ntyp, const float2* 
     for (int q = 0; q < 4; ++q) pa.sig[t][q] = q < nch[t] ? ees_sig(dmax[t], q) : 1.f;
   }
   pa.err = c->d_dev_err;
+  pa.pmax = reinterpret_cast<unsigned int*>(pmax);
   const long long warps = (long long)cdiv(S, ROWS) * nsp * 8;
   k_presplit_ees_a<<<(unsigned)((warps + 7) / 8), 256, 0, c->stream>>>(pa);  // 8 warps per block
   CPSTEP_LAUNCH_CHECK();
@@ -1867,7 +1997,7 @@ int ees_tc_force_pre(cpstep_ctx* c, int ntyp, const EesForceType* ty, int ld_d, 
     k_presplit_z<<<(unsigned)((nz + 255) / 256), 256, 0, c->stream>>>(
         y.Z, y.ldz, S, y.nch, y.natm_t, nks, tm * ROWS, y.zmax, y.zlv);
     CPSTEP_LAUNCH_CHECK();
-    k_presplit_st<<<(unsigned)((ns + 255) / 256), 256, 0, c->stream>>>(
+    k_presplit_st<float><<<(unsigned)((ns + 255) / 256), 256, 0, c->stream>>>(
         y.sv, y.ld_s, kr, y.natm_t, nks, ntile * ROWS, y.smax, y.stlv);
     CPSTEP_LAUNCH_CHECK();
     pf.a[t] = y.zlv;
@@ -1886,19 +2016,85 @@ int ees_tc_force_pre(cpstep_ctx* c, int ntyp, const EesForceType* ty, int ld_d, 
   pf.alpha = alpha;
   pf.f = fpsi;
   pf.err = c->d_dev_err;
-  static unsigned long long attr_done = 0;  // per-device attribute, one bit per device
-  int dev = 0;
-  CPSTEP_CUDA_TRY(cudaGetDevice(&dev));
-  const unsigned long long bit = 1ull << (dev & 63);
-  if (!(__atomic_load_n(&attr_done, __ATOMIC_ACQUIRE) & bit)) {
-    CPSTEP_CUDA_TRY(cudaFuncSetAttribute(k_pf_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         PF_BYTES));
-    __atomic_or_fetch(&attr_done, bit, __ATOMIC_RELEASE);
-  }
+  CPSTEP_CUDA_TRY(cudaFuncSetAttribute(k_pf_tc<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       PF_BYTES));
   const int gx = std::max(1, std::min(ntile, c->num_sms / tm));
-  k_pf_tc<<<dim3(gx, tm), PP_NTHR, PF_BYTES, c->stream>>>(pf);
+  k_pf_tc<false><<<dim3(gx, tm), PP_NTHR, PF_BYTES, c->stream>>>(pf);
   CPSTEP_LAUNCH_CHECK();
   return CPSTEP_OK;
+}
+
+// Atom forces of one or two atom types (k_pf_tc<true>): psi split transposed into
+// psi_t (ees_psit_bytes), zs transposed into zlv (ees_ztlv_bytes); partial sums
+// per lattice axis in fpart [*nblk][atoms of the types][3].
+int ees_tc_atom_force(cpstep_ctx* c, int ntyp, const EesForceType* ty, const int* rank0,
+                      const double* psi, const float* pmax, bool split_psi,
+                      const float2* sep, int km, const int2* kw, int ld_d, uint8_t* psi_t,
+                      uint8_t* zlv, double* fpart, int* nblk) {
+  using namespace pctc;
+  const int S = c->nstates, kr = 2 * c->npts, nks = cdiv(S, 16), ntile = cdiv(kr, ROWS);
+  if (ntyp < 1 || ntyp > 2 || (ld_d & 1) || !al16(psi) || !al16(psi_t) || !al16(zlv))
+    return CPSTEP_ERR_ARG;
+  if (split_psi) {
+    const long long np = (long long)ntile * ROWS * nks * 2;
+    k_presplit_st<double><<<(unsigned)((np + 255) / 256), 256, 0, c->stream>>>(
+        psi, kr, kr, S, nks, ntile * ROWS, pmax, psi_t);
+    CPSTEP_LAUNCH_CHECK();
+  }
+  ZtArgs z{};
+  PFArgs pf{};
+  int na = 0;
+  for (int t = 0; t < ntyp; ++t) {
+    z.zt[t] = ty[t].Z;
+    z.ldz[t] = ty[t].ldz;
+    z.nat[t] = pf.nat[t] = ty[t].natm_t;
+    z.nch[t] = pf.nch[t] = ty[t].nch;
+    z.zmax[t] = pf.zmax[t] = ty[t].zmax;
+    pf.dyp[t] = ty[t].dyp;
+    pf.rank0[t] = rank0[t];
+    na += ty[t].natm_t;
+  }
+  if (ntyp == 1) {
+    z.zt[1] = z.zt[0];
+    z.zmax[1] = pf.zmax[1] = pf.zmax[0];
+    pf.dyp[1] = pf.dyp[0];
+  }
+  const int tm = cdiv(4 * na, ROWS);
+  const long long nz = (long long)tm * ROWS * nks * 2;
+  k_presplit_zt<<<(unsigned)((nz + 255) / 256), 256, 0, c->stream>>>(z, S, nks, tm * ROWS, zlv);
+  CPSTEP_LAUNCH_CHECK();
+  pf.ntyp = 1;
+  pf.a[0] = zlv;
+  pf.b[0] = psi_t;
+  pf.nks[0] = nks;
+  pf.ntile = ntile;
+  pf.S = S;
+  pf.npts = c->npts;
+  pf.ld_d = ld_d;
+  pf.natm = c->atoms.natm;
+  pf.pmax = pmax;
+  pf.sep = sep;
+  pf.km = km;
+  pf.kw = kw;
+  pf.fpart = fpart;
+  pf.err = c->d_dev_err;
+  CPSTEP_CUDA_TRY(cudaFuncSetAttribute(k_pf_tc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       PF_BYTES));
+  *nblk = ees_af_blocks(c, na);
+  k_pf_tc<true><<<dim3(*nblk, tm), PP_NTHR, PF_BYTES, c->stream>>>(pf);
+  CPSTEP_LAUNCH_CHECK();
+  return CPSTEP_OK;
+}
+
+// point-tile blocks of the atom-force kernel for na atoms, and its level bytes
+int ees_af_blocks(const cpstep_ctx* c, int na) {
+  return std::max(1, std::min(cdiv(2 * c->npts, pctc::ROWS), c->num_sms / cdiv(4 * na, pctc::ROWS)));
+}
+size_t ees_psit_bytes(int nstates, int npts) {
+  return (size_t)cdiv(2 * npts, pctc::ROWS) * cdiv(nstates, 16) * pctc::STEP_H;
+}
+size_t ees_ztlv_bytes(int nstates, int na) {
+  return (size_t)cdiv(4 * na, pctc::ROWS) * cdiv(nstates, 16) * pctc::STEP_H;
 }
 
 // Level bytes of the psi force's operands: Z (rows 4 S) and S^T (2 npts reals)

@@ -190,3 +190,41 @@ def test_fp64_gspace_matches_grid_form(states, atoms, keep):
     for a, b in zip(*out):
         assert np.max(np.abs(b)) > 0.0
         assert np.max(np.abs(a - b)) <= 1e-11 * np.max(np.abs(b))
+
+
+@pytest.mark.parametrize("states,atoms,keep", [
+    (1, {"H": 1}, None), (16, {"O": 31, "H": 1}, None), (17, {"O": 32, "H": 33}, None),
+    (33, {"O": 3, "H": 6}, (0, 1)), (33, {"O": 3, "H": 6}, (1, 0))])
+def test_mixed_atom_forces_tile_edges(states, atoms, keep):
+    """Mixed contexts: energy, psi force and atom forces of the G-space form
+    against an FP64 context at the edges of the tiles (32 atoms; 16 states) and
+    with a type without channels.  FP16 pairs hold 22 bits and the sums FP32's 24
+    in chunks, added to the forces' largest entry: the module's 1e-5."""
+    if not cuda_ok():
+        pytest.skip("no CUDA device")
+    import torch
+    from openatom_b200.context import StepContext
+    from openatom_b200.system import System
+    s = System(12.0, 25.0, states, atoms, nfft=40, seed=5)
+    if keep is not None:
+        s.channels = [c for c in s.channels if (c["type"], c["l"]) == keep]
+    g = torch.Generator(device="cuda").manual_seed(states)
+    psi = torch.view_as_complex(torch.randn((states, s.layout.npts, 2), generator=g,
+                                            dtype=torch.float64, device="cuda"))
+    f0 = 0.1 * psi.flip(0).contiguous()
+    occ = 1.0 + torch.arange(states, dtype=torch.float64, device="cuda") % 2
+    out = []
+    for precision in ("mixed", "fp64"):
+        ctx = StepContext(s.layout, states, precision=precision)
+        try:
+            ctx.set_atoms(s)
+            ctx.set_nonlocal(s)
+            ctx.tune_set({"ees_gspace": 1})
+            f, e, fa = ctx.ees_nonlocal(psi, occ, fpsi=f0.clone())
+            out.append((e[7:8].cpu().numpy(), f.cpu().numpy(), fa.cpu().numpy()))
+            assert ctx.device_errors() == 0
+        finally:
+            ctx.close()
+    for a, b in zip(*out):
+        assert np.max(np.abs(b)) > 0.0
+        assert np.max(np.abs(a - b)) <= 1e-5 * np.max(np.abs(b))
