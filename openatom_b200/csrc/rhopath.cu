@@ -444,22 +444,54 @@ __global__ void k_local_forces_lines(const double4* __restrict__ fterm,
           double2 u = make_double2(x.x * y.x - x.y * y.y, x.x * y.y + x.y * y.x);
           const double2* T = sT + (size_t)t * lmax;
           double px = 0.0, py = 0.0, qx = 0.0, qy = 0.0;
-          // REC: kz runs up by one along the line, so e^{i2pi kz sz} is
-          // advanced by e^{i2pi sz} (the reference's ei_inc recursion)
-          double2 e = REC ? A.ez[(size_t)(skz[0] + A.kzm) * A.natm + at] : make_double2(0.0, 0.0);
-          const double2 inc = REC ? A.ez[(size_t)(1 + A.kzm) * A.natm + at] : e;
+          if (REC) {
+            // kz = c + j about the line's middle m: with z = e^{i2pi sz} and S = sum
+            // T_j z^j, P = e_c S and Q = e_c (c S + sum j T_j z^j).  Upper half and
+            // lower half (in 1/z = z*) are polynomials with their derivatives by
+            // Horner: 8 FMAs per (atom, point) where phase, P and Q took 12, and
+            // half the line's rounding in each chain.
+            const int m = len >> 1;
+            const double2 e0 = A.ez[(size_t)(skz[m] + A.kzm) * A.natm + at];
+            const double2 z = A.ez[(size_t)(1 + A.kzm) * A.natm + at];
+            double2 u = make_double2(0.0, 0.0), du = u, l = u, dl = u;
+            // (v, d) <- (t + z v, v + z d), zy negated for the lower half
+            auto term = [&](double2& v, double2& d, double2 tt, double zx, double zy) {
+              const double ex = fma(d.x, zx, fma(-d.y, zy, v.x)), ey = fma(d.x, zy, fma(d.y, zx, v.y));
+              const double wx = fma(v.x, zx, fma(-v.y, zy, tt.x)), wy = fma(v.x, zy, fma(v.y, zx, tt.y));
+              d = make_double2(ex, ey);
+              v = make_double2(wx, wy);
+            };
+            if (len & 1) u = T[len - 1];  // the upper half's extra term
+            const double2 *tu = T + 2 * m - 1, *tl = T;
 #pragma unroll 4
-          for (int i = 0; i < len; ++i) {
-            const int c = skz[i];
-            if (!REC) e = A.ez[(size_t)(c + A.kzm) * A.natm + at];
-            double2 tt = T[i];
-            double rx = e.x * tt.x - e.y * tt.y;
-            double ry = e.x * tt.y + e.y * tt.x;
-            px += rx;
-            py += ry;
-            qx += c * rx;
-            qy += c * ry;
-            if (REC) e = make_double2(e.x * inc.x - e.y * inc.y, e.x * inc.y + e.y * inc.x);
+            for (int i = 0; i < m; ++i) {
+              term(u, du, tu[-i], z.x, z.y);
+              term(l, dl, tl[i], z.x, -z.y);
+            }
+            const double lx = l.x * z.x + l.y * z.y, ly = l.y * z.x - l.x * z.y;  // l z*
+            const double sx = u.x + lx, sy = u.y + ly;
+            // sum j T_j z^j = z du - z* (l + z* dl)
+            const double hx = l.x + dl.x * z.x + dl.y * z.y, hy = l.y + dl.y * z.x - dl.x * z.y;
+            const double c = skz[m];
+            const double tx = c * sx + (z.x * du.x - z.y * du.y) - (hx * z.x + hy * z.y);
+            const double ty = c * sy + (z.x * du.y + z.y * du.x) - (hy * z.x - hx * z.y);
+            px = e0.x * sx - e0.y * sy;
+            py = e0.x * sy + e0.y * sx;
+            qx = e0.x * tx - e0.y * ty;
+            qy = e0.x * ty + e0.y * tx;
+          } else {
+#pragma unroll 4
+            for (int i = 0; i < len; ++i) {
+              const int c = skz[i];
+              const double2 e = A.ez[(size_t)(c + A.kzm) * A.natm + at];
+              const double2 tt = T[i];
+              const double rx = e.x * tt.x - e.y * tt.y;
+              const double ry = e.x * tt.y + e.y * tt.x;
+              px += rx;
+              py += ry;
+              qx += c * rx;
+              qy += c * ry;
+            }
           }
           double ip = u.x * py + u.y * px;  // Im(u P)
           double iq = u.x * qy + u.y * qx;  // Im(u Q)
