@@ -38,13 +38,20 @@ __device__ __forceinline__ double2 cm(double2 a, double2 b) {
   return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
 
-// the four columns of atom rank r at point p
-__device__ __forceinline__ void columns(const Geo& G, int r, int p, double2 (&b)[4]) {
+// the atom of rank r (-1: none) and its type's channels
+__device__ __forceinline__ int atom_of(const Geo& G, int r, int4& ch) {
+  const int a = r < G.na ? G.act[r] : -1;
+  ch = a >= 0 ? *reinterpret_cast<const int4*>(G.tch + 4 * G.typ[a]) : make_int4(-1, -1, -1, -1);
+  return a;
+}
+
+// the four columns of atom a (< 0: none) with channels ch4 at point p
+__device__ __forceinline__ void columns(const Geo& G, int a, int4 ch4, int p, double2 (&b)[4]) {
 #pragma unroll
   for (int k = 0; k < 4; ++k) b[k] = make_double2(0.0, 0.0);
-  if (r >= G.na || p >= G.npts) return;
-  const int a = G.act[r], nk = 2 * G.km + 1;
-  const int* ch = G.tch + 4 * G.typ[a];
+  if (a < 0 || p >= G.npts) return;
+  const int nk = 2 * G.km + 1;
+  const int ch[4] = {ch4.x, ch4.y, ch4.z, ch4.w};
   const double2* T = G.sep + (size_t)a * 6 * nk + G.km;
   double2 S = cm(T[G.kx[p]], cm(T[2 * nk + G.ky[p]], T[4 * nk + G.kz[p]]));
   const double w = G.w[p];
@@ -77,6 +84,10 @@ __global__ void __launch_bounds__(MT * 4) k_sums(const double2* __restrict__ psi
   const int r0 = blockIdx.x * 32, s0 = blockIdx.y * MT;
   const int c0 = (int)((long long)nchunk * blockIdx.z / gridDim.z);
   const int c1 = (int)((long long)nchunk * (blockIdx.z + 1) / gridDim.z);
+  __shared__ int4 ch_s[32];
+  __shared__ int act_s[32];
+  if (tid < 32) act_s[tid] = atom_of(G, r0 + tid, ch_s[tid]);
+  __syncthreads();
   double acc[4][4][2];
   dm::zero(acc);
   auto load = [&](int st, int c) {
@@ -92,7 +103,7 @@ __global__ void __launch_bounds__(MT * 4) k_sums(const double2* __restrict__ psi
     for (int q = tid; q < 512; q += THREADS) {
       const int pt = q & 15, al = q >> 4;
       double2 b[4];
-      columns(G, r0 + al, c * 16 + pt, b);
+      columns(G, act_s[al], ch_s[al], c * 16 + pt, b);
 #pragma unroll
       for (int k = 0; k < 4; ++k)
         *reinterpret_cast<double2*>(Bs + (st * NT + 4 * al + k) * dm::LDK + 2 * pt) = b[k];
@@ -181,7 +192,9 @@ __global__ void __launch_bounds__(MT * 4) k_psi_force(const double* __restrict__
     for (int q = tid; q < 512; q += THREADS) {
       const int pt = q & 63, al = q >> 6;
       double2 b[4];
-      columns(G, c * 8 + al, p0 + pt, b);
+      int4 ch;
+      const int a = atom_of(G, c * 8 + al, ch);
+      columns(G, a, ch, p0 + pt, b);
 #pragma unroll
       for (int k = 0; k < 4; ++k)
         *reinterpret_cast<double2*>(Bs + (st * 32 + 4 * al + k) * dm::LDN + 2 * pt) = b[k];
@@ -261,31 +274,50 @@ __global__ void __launch_bounds__(512) k_atom_force(const double* __restrict__ z
     dm::chunk_kn(acc, As + (st * NT + wm * 32) * dm::LDK, Bs + st * 32 * dm::LDN + wn * 32, lane);
     if (it % nkc != nkc - 1) continue;
     const int p0 = ((int)blockIdx.y + (it / nkc) * (int)gridDim.y) * 64;
+    // two points of an atom at a time, the loads of both in flight before the
+    // first is used; past the ends they read valid entries that count for nothing
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int r = r0 + wm * 8 + i * 2 + (g >> 2);
-      const int a = r < G.na ? G.act[r] : -1;
-      const int c = a >= 0 ? G.tch[4 * G.typ[a] + ch] : -1;
-      const double2* T = G.sep + (size_t)max(a, 0) * 6 * nk + G.km;
+    for (int h = 0; h < 2; ++h) {
+      int pt[2], kx[2], ky[2], kz[2];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int p = p0 + wn * 16 + j * 4 + t;
-        double2 x = make_double2(0.0, 0.0);
-        if (c >= 0 && p < G.npts) {
-          const double2 d = G.dyp[(size_t)c * G.npts + p];
-          x = cm(d, make_double2(acc[i][j][0], acc[i][j][1]));
+      for (int j = 0; j < 2; ++j) {
+        pt[j] = min(p0 + wn * 16 + (2 * h + j) * 4 + t, G.npts - 1);
+        kx[j] = __ldg(G.kx + pt[j]);
+        ky[j] = __ldg(G.ky + pt[j]);
+        kz[j] = __ldg(G.kz + pt[j]);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int r = r0 + wm * 8 + i * 2 + (g >> 2);
+        const int a = r < G.na ? __ldg(G.act + r) : -1;
+        const int c = a >= 0 ? __ldg(G.tch + 4 * G.typ[a] + ch) : -1;
+        const double2* T = G.sep + (size_t)max(a, 0) * 6 * nk + G.km;
+        const double2* Tx = T + (ch == 0 ? nk : 0);
+        const double2* Ty = T + (ch == 1 ? 3 : 2) * nk;
+        const double2* Tz = T + (ch == 2 ? 5 : 4) * nk;
+        const double2* dyp = G.dyp + (size_t)max(c, 0) * G.npts;
+        double2 d[2], x[2], y[2], z[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          d[j] = __ldg(dyp + pt[j]);
+          x[j] = __ldg(Tx + kx[j]);
+          y[j] = __ldg(Ty + ky[j]);
+          z[j] = __ldg(Tz + kz[j]);
         }
-        acc[i][j][0] = acc[i][j][1] = 0.0;
 #pragma unroll
-        for (int o = 4; o <= 8; o <<= 1) {
-          x.x += __shfl_xor_sync(0xffffffffu, x.x, o);
-          x.y += __shfl_xor_sync(0xffffffffu, x.y, o);
-        }
-        if (ch < 3 && a >= 0 && p < G.npts) {
-          const double2 D = cm(T[(ch == 0 ? nk : 0) + G.kx[p]],
-                               cm(T[(ch == 1 ? 3 : 2) * nk + G.ky[p]],
-                                  T[(ch == 2 ? 5 : 4) * nk + G.kz[p]]));
-          fa[i] += G.w[p] * (x.x * D.x + x.y * D.y);
+        for (int j = 0; j < 2; ++j) {
+          double2 q = cm(d[j], make_double2(acc[i][2 * h + j][0], acc[i][2 * h + j][1]));
+          if (c < 0) q = make_double2(0.0, 0.0);
+          acc[i][2 * h + j][0] = acc[i][2 * h + j][1] = 0.0;
+#pragma unroll
+          for (int o = 4; o <= 8; o <<= 1) {
+            q.x += __shfl_xor_sync(0xffffffffu, q.x, o);
+            q.y += __shfl_xor_sync(0xffffffffu, q.y, o);
+          }
+          if (ch < 3 && a >= 0 && p0 + wn * 16 + (2 * h + j) * 4 + t < G.npts) {
+            const double2 D = cm(x[j], cm(y[j], z[j]));
+            fa[i] += __ldg(G.w + pt[j]) * (q.x * D.x + q.y * D.y);
+          }
         }
       }
     }
