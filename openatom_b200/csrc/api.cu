@@ -289,6 +289,9 @@ int cpstep_ctx_destroy(cpstep_ctx* c) {
   cudaFree(c->d_force_atoms);
   graph_drop(c);
   if (c->cap_stream) cudaStreamDestroy(c->cap_stream);
+  if (c->side) cudaStreamDestroy(c->side);
+  if (c->side_fork) cudaEventDestroy(c->side_fork);
+  if (c->side_join) cudaEventDestroy(c->side_join);
   for (auto& e : c->prof_ev) cudaEventDestroy(e);
   nl_free(c);
   sf_free(c);

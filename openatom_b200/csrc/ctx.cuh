@@ -205,7 +205,7 @@ struct NlData {
   std::vector<size_t> tab_off;
   std::vector<int> tab_cap;
   // G-space evaluation of the same sums (mixed contexts on the tensor cores,
-  // ees_gspace_run): per atom separable transforms, S matrices (FP32) of each
+  // nl_front, nl_back): per atom separable transforms, S matrices (FP32) of each
   // type [atom of type][ld_s], each type's channels with contiguous dyp
   int km = 0;                       // largest |k| of the state sphere on an axis
   double2* sep = nullptr;           // [natm][3][2][2 km + 1]
@@ -414,6 +414,8 @@ struct cpstep_ctx {
   int graph_warm = 0;              // a direct step with gkey ran
   StepKey gkey{};
   cudaStream_t cap_stream = nullptr;
+  cudaStream_t side = nullptr;        // the non-local front beside the density side (step_run)
+  cudaEvent_t side_fork = nullptr, side_join = nullptr;
   cudaGraphExec_t gexec = nullptr;
   unsigned long long gkernels = 0;  // kernels in the graph
   unsigned gen = 0;                 // counts graph_drop calls (batch graphs recapture)
@@ -467,8 +469,8 @@ int nl_grid_reserve(cpstep_ctx* c);
 // ees64.cu: the same pass of an FP64 context in G space
 int ees64_set(cpstep_ctx* c, const std::vector<int>& order);
 bool ees64_faster(const cpstep_ctx* c);
-int ees64_run(cpstep_ctx* c, const double* psi, double* fpsi, const double* occ, double* energies,
-              double* fatm);
+int ees64_front(cpstep_ctx* c, const double* psi, const double* occ, bool forces);
+int ees64_back(cpstep_ctx* c, double* fpsi, double* energies, double* fatm);
 int nl_grid_size(int kmax, double scale, int n_interp);
 int eext_grid_size(int kmax, double scale, int n_interp);
 // eesAtmBsplineRgrp's indices, Mn and dMn of every atom on an nkf grid
@@ -527,6 +529,17 @@ struct EesForceType {
 };
 int ees_tc_force_pre(cpstep_ctx* c, int ntyp, const EesForceType* ty, int ld_d, double alpha,
                      double* fpsi, size_t zlv_bytes, size_t stlv_bytes);
+// The non-local pass in G space cut in two.  The front needs psi alone: sums, Z and
+// the atom forces' partial sums.  The back adds to the psi force, the atom forces
+// and the energies.  *split is false where the pass is not cut (NL-grid form, more
+// than two types with projectors): nl_run does all of it then.
+struct NlFront {
+  EesForceType ft[2];
+  int ntyp = 0, rank0[2] = {0, 0}, nblk = 0;
+};
+int nl_front(cpstep_ctx* c, const double* psi, const double* occ, bool forces, NlFront* h,
+             bool* split);
+int nl_back(cpstep_ctx* c, double* fpsi, double* energies, double* fatm, const NlFront& h);
 int ees_tc_atom_force(cpstep_ctx* c, int ntyp, const EesForceType* ty, const int* rank0,
                       const double* psi, const float* pmax, bool split_psi,
                       const float2* sep, int km, const int2* kw, int ld_d, uint8_t* psi_t,

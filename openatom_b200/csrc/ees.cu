@@ -858,8 +858,16 @@ static int ees_sep_run(cpstep_ctx* c) {
 // The EES pass in G space (see k_ees_sep): per type, the forward sums as one
 // tensor-core product of psi with conj(dyp) S, the glue, and the psi force as
 // one back-multiply with the same matrix.
-static int ees_gspace_run(cpstep_ctx* c, const double* psi, const double* occ, double* fpsi,
-                          double* energies, double* fatm) {
+// the types with projectors
+static std::vector<int> nl_types(const cpstep_ctx* c) {
+  std::vector<int> tl;
+  for (int t = 0; t < c->atoms.ntyp; ++t)
+    if (!c->nl.tch[t].empty() && c->atoms.tstart[t + 1] > c->atoms.tstart[t]) tl.push_back(t);
+  return tl;
+}
+
+// The mixed pass in G space: separable transforms and S rows of every atom,
+static int ees_gspace_tables(cpstep_ctx* c) {
   NlData& n = c->nl;
   const int S = c->nstates, natm = n.natm, ntyp = c->atoms.ntyp;
   if (int rc = ees_sep_run(c)) return rc;
@@ -870,9 +878,6 @@ static int ees_gspace_run(cpstep_ctx* c, const double* psi, const double* occ, d
     td.tsoff[t] = n.tsoff[t];
     td.bloff[t] = (long long)n.blv_off[t];
   }
-  NlAtoms A{};
-  for (int k = 0; k < 9; ++k) A.hmati[k] = c->hmati[k];
-  A.grid = (double)n.nkf;
   // bounds of |S| (the FP16 scales of the S rows' levels) and the largest |Z|
   // entry per type (the psi force's)
   CPSTEP_CUDA_TRY(cudaMemsetAsync(n.d_hmax, 0, sizeof(float) * (2 * ntyp + 1), c->stream));
@@ -887,63 +892,101 @@ static int ees_gspace_run(cpstep_ctx* c, const double* psi, const double* occ, d
       n.ld_s, n.sv, n.tsc, n.blv, nsp_s);
   CPSTEP_LAUNCH_CHECK();
   CPSTEP_CUDA_TRY(cudaMemsetAsync(n.enl_s, 0, sizeof(double) * S, c->stream));
-  // the types with projectors, two at a time: A of both split from one read of psi
-  std::vector<int> tl;
-  EesForceType ft[2];
-  int rank0[2] = {0, 0};
-  for (int t = 0; t < ntyp; ++t)
-    if (!n.tch[t].empty() && c->atoms.tstart[t + 1] > c->atoms.tstart[t]) tl.push_back(t);
-  for (size_t q = 0; q < tl.size(); ++q) {
-    const int t = tl[q];
-    const int nch = (int)n.tch[t].size();
+  return CPSTEP_OK;
+}
+
+// then for one or two types t[0 .. np) sums, Z and atom-force partials (A of both
+// types split from one read of psi; first: psi's transposed levels are not there yet),
+static int ees_gspace_front(cpstep_ctx* c, const double* psi, const double* occ, bool forces,
+                            const int* tt, int np, bool first, NlFront* h) {
+  NlData& n = c->nl;
+  const int S = c->nstates, ntyp = c->atoms.ntyp;
+  unsigned int* zmax_u = reinterpret_cast<unsigned int*>(n.d_hmax) + ntyp;
+  const float2* dy[2];
+  const float* dm[2];
+  int nc[2];
+  uint8_t* al[2] = {n.alv, n.alv + n.alv_bytes};
+  for (int k = 0; k < np; ++k) {
+    dy[k] = n.tdyp[tt[k]];
+    dm[k] = n.tdmax_c[tt[k]].data();
+    nc[k] = (int)n.tch[tt[k]].size();
+  }
+  if (int rc = ees_tc_presplit_a(c, psi, np, dy, n.ld_d32, nc, dm, al, n.alv_bytes,
+                                 n.d_hmax + 2 * ntyp))
+    return rc;
+  h->ntyp = np;
+  for (int k = 0; k < np; ++k) {
+    const int t = tt[k], nch = nc[k];
     const int nt = c->atoms.tstart[t + 1] - c->atoms.tstart[t];
-    uint8_t* alv = n.alv + (q & 1) * n.alv_bytes;
-    if (q % 2 == 0) {
-      const int np2 = q + 1 < tl.size() ? 2 : 1;
-      const float2* dy[2];
-      const float* dm[2];
-      int nc[2];
-      uint8_t* al[2] = {n.alv, n.alv + n.alv_bytes};
-      for (int k = 0; k < np2; ++k) {
-        dy[k] = n.tdyp[tl[q + k]];
-        dm[k] = n.tdmax_c[tl[q + k]].data();
-        nc[k] = (int)n.tch[tl[q + k]].size();
-      }
-      if (int rc = ees_tc_presplit_a(c, psi, np2, dy, n.ld_d32, nc, dm, al, n.alv_bytes,
-                                     n.d_hmax + 2 * ntyp))
-        return rc;
-    }
     if (int rc = ees_tc_sums_pre(c, nch, n.tdmax_c[t].data(), n.blv + n.blv_off[t], nt,
-                                 n.tinv + n.tsoff[t], alv, n.csum))
+                                 n.tinv + n.tsoff[t], al[k], n.csum))
       return rc;
     const int ldz = (nch * nt + 1) / 2 * 2;
-    double* zt = n.zt + (q & 1) * n.zt_slot;
+    double* zt = n.zt + k * n.zt_slot;
     ees::k_ees_zglue<<<S, 128, 0, c->stream>>>(n.csum, S, nt, nch, n.d_tch + 4 * t, n.d_vn, occ,
                                                 zt, ldz, n.enl_s, zmax_u + t);
     CPSTEP_LAUNCH_CHECK();
-    ft[q & 1] = EesForceType{n.sv + n.sv_off[t], n.ld_s, n.tdyp[t], nch, nt, zt, ldz,
-                             n.d_hmax + t, n.d_hmax + ntyp + t, n.pf_z + (q & 1) * n.pf_zbytes,
-                             n.pf_st + (q & 1) * n.pf_stbytes};
-    rank0[q & 1] = c->atoms.tstart[t];
-    if (q % 2 == 0 && q + 1 < tl.size()) continue;
-    // the pair's psi force (F read and written once for both types) and atom forces
-    const int np2 = (int)(q % 2) + 1;
-    if (int rc = ees_tc_force_pre(c, np2, ft, n.ld_d32, -1.0, fpsi, n.pf_zbytes, n.pf_stbytes))
-      return rc;
-    if (fatm) {
-      int nblk = 0;
-      if (int rc = ees_tc_atom_force(c, np2, ft, rank0, psi, n.d_hmax + 2 * ntyp, q < 2, n.sepf, n.km, n.kw, n.ld_d32,
-                                     n.psi_t, n.af_z, n.af_part, &nblk))
-        return rc;
-      const int na2 = ft[0].natm_t + (np2 > 1 ? ft[1].natm_t : 0);
-      ees::k_ees_atoms<<<cdiv(na2, 4), 128, 0, c->stream>>>(
-          n.af_part, nblk, ft[0].natm_t, na2, rank0[0], np2 > 1 ? rank0[1] : 0, n.d_order, A, fatm);
-      CPSTEP_LAUNCH_CHECK();
-    }
+    h->ft[k] = EesForceType{n.sv + n.sv_off[t], n.ld_s, n.tdyp[t], nch, nt, zt, ldz,
+                            n.d_hmax + t, n.d_hmax + ntyp + t, n.pf_z + k * n.pf_zbytes,
+                            n.pf_st + k * n.pf_stbytes};
+    h->rank0[k] = c->atoms.tstart[t];
   }
-  ees::k_nl_finish<<<1, 128, 0, c->stream>>>(n.enl_s, nullptr, S, natm, energies, nullptr);
+  if (!forces) return CPSTEP_OK;
+  return ees_tc_atom_force(c, np, h->ft, h->rank0, psi, n.d_hmax + 2 * ntyp, first, n.sepf, n.km,
+                           n.kw, n.ld_d32, n.psi_t, n.af_z, n.af_part, &h->nblk);
+}
+
+// and their psi force (F read and written once for both types) and atom forces
+static int ees_gspace_back(cpstep_ctx* c, double* fpsi, double* fatm, const NlFront& h) {
+  NlData& n = c->nl;
+  if (int rc = ees_tc_force_pre(c, h.ntyp, h.ft, n.ld_d32, -1.0, fpsi, n.pf_zbytes, n.pf_stbytes))
+    return rc;
+  if (!fatm) return CPSTEP_OK;
+  NlAtoms A{};
+  for (int k = 0; k < 9; ++k) A.hmati[k] = c->hmati[k];
+  A.grid = (double)n.nkf;
+  const int na2 = h.ft[0].natm_t + (h.ntyp > 1 ? h.ft[1].natm_t : 0);
+  ees::k_ees_atoms<<<cdiv(na2, 4), 128, 0, c->stream>>>(n.af_part, h.nblk, h.ft[0].natm_t, na2,
+                                                         h.rank0[0], h.ntyp > 1 ? h.rank0[1] : 0,
+                                                         n.d_order, A, fatm);
   CPSTEP_LAUNCH_CHECK();
   return CPSTEP_OK;
+}
+
+static int ees_gspace_energy(cpstep_ctx* c, double* energies) {
+  ees::k_nl_finish<<<1, 128, 0, c->stream>>>(c->nl.enl_s, nullptr, c->nstates, c->nl.natm, energies,
+                                             nullptr);
+  CPSTEP_LAUNCH_CHECK();
+  return CPSTEP_OK;
+}
+
+static bool nl_gmixed(const cpstep_ctx* c) {
+  return c->nl.gspace_ok && c->precision == CPSTEP_PREC_MIXED && c->tc_ok && c->tune.ees_gspace;
+}
+
+int nl_front(cpstep_ctx* c, const double* psi, const double* occ, bool forces, NlFront* h,
+             bool* split) {
+  *split = false;
+  if (!c->nl.on || c->nl.natm != c->atoms.natm) return CPSTEP_OK;  // nl_run reports it
+  if (nl_gmixed(c)) {
+    const std::vector<int> tl = nl_types(c);
+    if (tl.size() > 2) return CPSTEP_OK;
+    *split = true;
+    if (int rc = ees_gspace_tables(c)) return rc;
+    return tl.empty() ? CPSTEP_OK
+                      : ees_gspace_front(c, psi, occ, forces, tl.data(), (int)tl.size(), true, h);
+  }
+  if (!nl_g64(c)) return CPSTEP_OK;
+  *split = true;
+  if (int rc = ees_sep_run(c)) return rc;
+  return ees64_front(c, psi, occ, forces);
+}
+
+int nl_back(cpstep_ctx* c, double* fpsi, double* energies, double* fatm, const NlFront& h) {
+  if (!nl_gmixed(c)) return ees64_back(c, fpsi, energies, fatm);
+  if (h.ntyp)
+    if (int rc = ees_gspace_back(c, fpsi, fatm, h)) return rc;
+  return ees_gspace_energy(c, energies);
 }
 
 int nl_run(cpstep_ctx* c, const double* psi, const double* occ, double* fpsi, double* energies,
@@ -957,11 +1000,20 @@ int nl_run(cpstep_ctx* c, const double* psi, const double* occ, double* fpsi, do
     cpstep_set_error("ees_nonlocal: atoms changed since cpstep_set_nonlocal");
     return CPSTEP_ERR_STATE;
   }
-  if (n.gspace_ok && c->precision == CPSTEP_PREC_MIXED && c->tc_ok && c->tune.ees_gspace)
-    return ees_gspace_run(c, psi, occ, fpsi, energies, fatm);
-  if (nl_g64(c)) {
-    if (int rc = ees_sep_run(c)) return rc;
-    return ees64_run(c, psi, fpsi, occ, energies, fatm);
+  NlFront h;
+  bool split = false;
+  if (int rc = nl_front(c, psi, occ, fatm != nullptr, &h, &split)) return rc;
+  if (split) return nl_back(c, fpsi, energies, fatm, h);
+  if (nl_gmixed(c)) {  // more than two types with projectors: two at a time
+    const std::vector<int> tl = nl_types(c);
+    if (int rc = ees_gspace_tables(c)) return rc;
+    for (size_t q = 0; q < tl.size(); q += 2) {
+      if (int rc = ees_gspace_front(c, psi, occ, fatm != nullptr, tl.data() + q,
+                                    (int)std::min<size_t>(2, tl.size() - q), q == 0, &h))
+        return rc;
+      if (int rc = ees_gspace_back(c, fpsi, fatm, h)) return rc;
+    }
+    return ees_gspace_energy(c, energies);
   }
   if (int rc = nl_grid_reserve(c)) return rc;
   const int S = c->nstates, natm = n.natm;

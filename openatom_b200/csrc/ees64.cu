@@ -459,15 +459,13 @@ bool ees64_faster(const cpstep_ctx* c) {
   return tg < tf;
 }
 
-int ees64_run(cpstep_ctx* c, const double* psi, double* fpsi, const double* occ, double* energies,
-              double* fatm) {
+int ees64_front(cpstep_ctx* c, const double* psi, const double* occ, bool forces) {
   NlData& n = c->nl;
   const int S = c->nstates;
   e64::Geo G{n.sep,   c->d_kx,   c->d_ky,       c->d_kz, c->d_wpt, n.dyp,
              n.d_tch, n.e64_act, c->atoms.typ,  c->npts, n.km,     n.e64_na};
   const int ntile = cdiv(n.e64_na, 32), ncolp = ntile * e64::NT, Sp = cdiv(S, 32) * 32;
   const double2* ps = reinterpret_cast<const double2*>(psi);
-  double2* f = reinterpret_cast<double2*>(fpsi);
   double* zst = n.e64_zs + (size_t)ncolp * Sp;
   int rc;
   switch (e64::tile_rows(S)) {
@@ -479,18 +477,29 @@ int ees64_run(cpstep_ctx* c, const double* psi, double* fpsi, const double* occ,
   e64::k_scale<<<dim3(ncolp / 8, Sp / 32), dim3(32, 8), 0, c->stream>>>(
       n.e64_part, n.e64_split, ncolp, Sp, S, G, n.d_vn, occ, n.e64_zs, zst, n.e64_e);
   CPSTEP_LAUNCH_CHECK();
+  if (forces) {
+    const size_t b = sizeof(double) * 2 * (e64::NT * dm::LDK + 32 * dm::LDN);
+    if ((rc = e64::smem(e64::k_atom_force, b))) return rc;
+    e64::k_atom_force<<<dim3(ntile, n.e64_nblk), 512, b, c->stream>>>(zst, Sp, ps, S, G, n.e64_f);
+    CPSTEP_LAUNCH_CHECK();
+  }
+  return CPSTEP_OK;
+}
+
+int ees64_back(cpstep_ctx* c, double* fpsi, double* energies, double* fatm) {
+  NlData& n = c->nl;
+  const int S = c->nstates;
+  e64::Geo G{n.sep,   c->d_kx,   c->d_ky,       c->d_kz, c->d_wpt, n.dyp,
+             n.d_tch, n.e64_act, c->atoms.typ,  c->npts, n.km,     n.e64_na};
+  const int ncolp = cdiv(n.e64_na, 32) * e64::NT, Sp = cdiv(S, 32) * 32;
+  double2* f = reinterpret_cast<double2*>(fpsi);
+  int rc;
   switch (e64::tile_rows(S)) {
     case 32: rc = e64::psi_force<32>(c, G, ncolp, f); break;
     case 64: rc = e64::psi_force<64>(c, G, ncolp, f); break;
     default: rc = e64::psi_force<128>(c, G, ncolp, f); break;
   }
   if (rc) return rc;
-  if (fatm) {
-    const size_t b = sizeof(double) * 2 * (e64::NT * dm::LDK + 32 * dm::LDN);
-    if ((rc = e64::smem(e64::k_atom_force, b))) return rc;
-    e64::k_atom_force<<<dim3(ntile, n.e64_nblk), 512, b, c->stream>>>(zst, Sp, ps, S, G, n.e64_f);
-    CPSTEP_LAUNCH_CHECK();
-  }
   e64::Cell C;
   for (int k = 0; k < 9; ++k) C.h[k] = c->hmati[k];
   C.grid = (double)n.nkf;

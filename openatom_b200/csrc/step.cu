@@ -327,6 +327,43 @@ static int ensure_buf(double** p, size_t bytes) {
   return CPSTEP_OK;
 }
 
+// The part of the non-local pass that needs psi alone, on a stream of its own beside
+// density, V_KS and V.psi.  Small systems' kernels are latencies one after the other
+// (24 atoms 353 -> 300 us, 45 states FP64 at 60^3 457 -> 422), large ones' last waves
+// fill up (192 atoms 3486 -> 3432, 768 atoms 85500 -> 81320), so there is no size rule.
+// The front writes scratch of its own (NlData) and the PairCalculator's split-K
+// partials, which nothing between fork and join uses.  The step's stream waits for it at join(), which every way out of the step passes,
+// so that nothing is left running when the step's stream has finished.
+struct NlBeside {
+  cpstep_ctx* c;
+  NlFront h;
+  bool split = false, open = false;
+  explicit NlBeside(cpstep_ctx* ctx) : c(ctx) {}
+  ~NlBeside() { join(); }
+  int start(const double* psi, const double* occ, bool forces) {
+    if (!c->side) {
+      CPSTEP_CUDA_TRY(cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking));
+      CPSTEP_CUDA_TRY(cudaEventCreateWithFlags(&c->side_fork, cudaEventDisableTiming));
+      CPSTEP_CUDA_TRY(cudaEventCreateWithFlags(&c->side_join, cudaEventDisableTiming));
+    }
+    CPSTEP_CUDA_TRY(cudaEventRecord(c->side_fork, c->stream));
+    CPSTEP_CUDA_TRY(cudaStreamWaitEvent(c->side, c->side_fork, 0));
+    open = true;
+    const cudaStream_t own = c->stream;
+    c->stream = c->side;
+    const int rc = nl_front(c, psi, occ, forces, &h, &split);
+    c->stream = own;
+    return rc;
+  }
+  int join() {
+    if (!open) return CPSTEP_OK;
+    open = false;
+    CPSTEP_CUDA_TRY(cudaEventRecord(c->side_join, c->side));
+    CPSTEP_CUDA_TRY(cudaStreamWaitEvent(c->stream, c->side_join, 0));
+    return CPSTEP_OK;
+  }
+};
+
 // One CP electronic step on psi (orthonormal on entry and exit).
 int step_run(cpstep_ctx* c, double* psi, double* vpsi, const double* occ, double dt,
              int iteration, double* energies, double* atom_force, int ortho_check) {
@@ -351,6 +388,9 @@ int step_run(cpstep_ctx* c, double* psi, double* vpsi, const double* occ, double
       cudaEventRecord(c->prof_ev[(size_t)c->prof_pending * (CPSTEP_NPHASE + 1) + k], c->stream);
   };
   mark(0);
+  NlBeside nl(c);
+  // (phase timing wants the phases one after the other)
+  if (c->nl.on && !c->profile && (rc = nl.start(psi, occ, atom_force != nullptr))) return rc;
   // 1. density and V_KS (XC, Hartree, local pseudopotential, Ewald)
   if ((rc = statefft_density(c, psi, occ, c->d_rho))) return rc;
   mark(1);
@@ -365,7 +405,10 @@ int step_run(cpstep_ctx* c, double* psi, double* vpsi, const double* occ, double
   mark(3);
   // 2b. non-local energy, psi force and atom forces (EES or structure factors)
   if (c->nl.on) {
-    if ((rc = nl_run(c, psi, occ, c->d_force, energies, atom_force))) return rc;
+    if ((rc = nl.join())) return rc;
+    if ((rc = nl.split ? nl_back(c, c->d_force, energies, atom_force, nl.h)
+                       : nl_run(c, psi, occ, c->d_force, energies, atom_force)))
+      return rc;
   } else if (c->sf.on) {
     if ((rc = sf_run(c, psi, occ, c->d_force, energies, atom_force))) return rc;
   } else {
