@@ -541,7 +541,8 @@ CPSTEP_API int cpstep_ctx_set_graph(cpstep_ctx* ctx, int enable);
  * Launch choices of a context (no reference counterpart; FFTW_MEASURE plans,
  * fftCache.C:252-255, are the nearest relative).  CPSTEP_NTUNE values:
  *   [0] state plane passes: register-shuffle line FFTs (1), shared-memory
- *       Stockham (0) or the two-stage line FFTs (2) where they exist;  [1] state plane passes: blocks about
+ *       Stockham (0) or the two-stage line FFTs (2; in FP64 1 as well) where
+ *       they exist;  [1] state plane passes: blocks about
  *       this many times the SM count;  [2] EES plane kernels: the same;
  *   [3] PairCalc overlap split-K: CTAs about this many times the SM count;
  *   [4] mixed contexts: tensor-core products (1) or FP64 (0);

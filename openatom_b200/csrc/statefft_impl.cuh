@@ -2033,11 +2033,13 @@ struct StateFft {
     return CPSTEP_OK;
   }
 
-  // whether the two-stage P x Q plane passes (k_two) run this size
+  // whether the two-stage P x Q plane passes (k_two) run this size; in FP64 as form 1
+  // too, whose shuffles lost on every grid (128 states of 128^3, density / V.psi:
+  // 1425/2606 against 720/1440 us)
   static constexpr bool two_built = TwoCfg<N>::ok && !(sizeof(T) == 8 && N == 200);
   static bool two_fits(const cpstep_ctx* c, const FftJob& j) {
     if constexpr (two_built)
-      return c->tune.shfl == 2 && j.g.nlines < 0xffff &&
+      return c->tune.shfl >= (sizeof(T) == 8 ? 1 : 2) && j.g.nlines < 0xffff &&
              std::max(TwoShape<T, N>::bytes(j.g.nplane_x, j.g.nlines),
                       TwoShape<T, N, true>::bytes(j.g.nplane_x, j.g.nlines)) <= 227 * 1024;
     return false;
