@@ -342,7 +342,8 @@ struct Cell {
   double grid;
 };
 
-// energies[NL] (block 0) and the Cartesian atom forces (one thread per atom)
+// energies[NL] (block 0) and the Cartesian atom forces (one warp per atom: a thread
+// each took 20 us over 74 partials, latency after latency)
 __global__ void k_finish(const double* __restrict__ epart, int ne, double* __restrict__ energies,
                          const double* __restrict__ fpart, int nblk, Geo G, Cell C,
                          double* __restrict__ fatm) {
@@ -354,16 +355,18 @@ __global__ void k_finish(const double* __restrict__ epart, int ne, double* __res
     if (threadIdx.x == 0 && energies) energies[CPSTEP_E_NL] = e;
     return;
   }
-  const int r = (blockIdx.x - 1) * blockDim.x + threadIdx.x;
+  const int r = (int)((blockIdx.x - 1) * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (r >= G.na) return;
   double f[3] = {0.0, 0.0, 0.0};
-  for (int b = 0; b < nblk; ++b)
+  for (int b = lane; b < nblk; b += 32)
 #pragma unroll
     for (int d = 0; d < 3; ++d) f[d] += fpart[((size_t)b * G.na + r) * 3 + d];
-  double* o = fatm + 3 * (size_t)G.act[r];
 #pragma unroll
   for (int d = 0; d < 3; ++d)
-    o[d] -= C.grid * (f[0] * C.h[3 * d] + f[1] * C.h[3 * d + 1] + f[2] * C.h[3 * d + 2]);
+    for (int o = 16; o > 0; o >>= 1) f[d] += __shfl_xor_sync(0xffffffffu, f[d], o);
+  if (lane >= 3) return;
+  fatm[3 * (size_t)G.act[r] + lane] -=
+      C.grid * (f[0] * C.h[3 * lane] + f[1] * C.h[3 * lane + 1] + f[2] * C.h[3 * lane + 2]);
 }
 
 template <typename K>
@@ -503,7 +506,7 @@ int ees64_back(cpstep_ctx* c, double* fpsi, double* energies, double* fatm) {
   e64::Cell C;
   for (int k = 0; k < 9; ++k) C.h[k] = c->hmati[k];
   C.grid = (double)n.nkf;
-  e64::k_finish<<<1 + (fatm ? cdiv(n.e64_na, 128) : 0), 128, 0, c->stream>>>(
+  e64::k_finish<<<1 + (fatm ? cdiv(n.e64_na, 4) : 0), 128, 0, c->stream>>>(
       n.e64_e, ncolp * (Sp / 32), energies, n.e64_f, n.e64_nblk, G, C, fatm);
   CPSTEP_LAUNCH_CHECK();
   return CPSTEP_OK;
