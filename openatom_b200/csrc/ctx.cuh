@@ -528,7 +528,7 @@ struct EesForceType {
   uint8_t* stlv;
 };
 int ees_tc_force_pre(cpstep_ctx* c, int ntyp, const EesForceType* ty, int ld_d, double alpha,
-                     double* fpsi, size_t zlv_bytes, size_t stlv_bytes);
+                     double* fpsi);
 // The non-local pass in G space cut in two.  The front needs psi alone: sums, Z and
 // the atom forces' partial sums.  The back adds to the psi force, the atom forces
 // and the energies.  *split is false where the pass is not cut (NL-grid form, more
@@ -540,10 +540,12 @@ struct NlFront {
 int nl_front(cpstep_ctx* c, const double* psi, const double* occ, bool forces, NlFront* h,
              bool* split);
 int nl_back(cpstep_ctx* c, double* fpsi, double* energies, double* fatm, const NlFront& h);
+int ees_tc_presplit_force(cpstep_ctx* c, int ntyp, const EesForceType* ty, size_t zlv_bytes,
+                          size_t stlv_bytes, const double* psi, const float* pmax, uint8_t* psi_t,
+                          uint8_t* af_z);
 int ees_tc_atom_force(cpstep_ctx* c, int ntyp, const EesForceType* ty, const int* rank0,
-                      const double* psi, const float* pmax, bool split_psi,
-                      const float2* sep, int km, const int2* kw, int ld_d, uint8_t* psi_t,
-                      uint8_t* zlv, double* fpart, int* nblk);
+                      const float* pmax, const float2* sep, int km, const int2* kw, int ld_d,
+                      const uint8_t* psi_t, const uint8_t* zlv, double* fpart, int* nblk);
 int ees_af_blocks(const cpstep_ctx* c, int na);
 size_t ees_psit_bytes(int nstates, int npts);
 size_t ees_ztlv_bytes(int nstates, int na);

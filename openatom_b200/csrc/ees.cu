@@ -931,15 +931,19 @@ static int ees_gspace_front(cpstep_ctx* c, const double* psi, const double* occ,
                             n.pf_st + k * n.pf_stbytes};
     h->rank0[k] = c->atoms.tstart[t];
   }
+  const float* pmax = n.d_hmax + 2 * ntyp;
+  if (int rc = ees_tc_presplit_force(c, np, h->ft, n.pf_zbytes, n.pf_stbytes, first ? psi : nullptr,
+                                     pmax, n.psi_t, forces ? n.af_z : nullptr))
+    return rc;
   if (!forces) return CPSTEP_OK;
-  return ees_tc_atom_force(c, np, h->ft, h->rank0, psi, n.d_hmax + 2 * ntyp, first, n.sepf, n.km,
-                           n.kw, n.ld_d32, n.psi_t, n.af_z, n.af_part, &h->nblk);
+  return ees_tc_atom_force(c, np, h->ft, h->rank0, pmax, n.sepf, n.km, n.kw, n.ld_d32, n.psi_t,
+                           n.af_z, n.af_part, &h->nblk);
 }
 
 // and their psi force (F read and written once for both types) and atom forces
 static int ees_gspace_back(cpstep_ctx* c, double* fpsi, double* fatm, const NlFront& h) {
   NlData& n = c->nl;
-  if (int rc = ees_tc_force_pre(c, h.ntyp, h.ft, n.ld_d32, -1.0, fpsi, n.pf_zbytes, n.pf_stbytes))
+  if (int rc = ees_tc_force_pre(c, h.ntyp, h.ft, n.ld_d32, -1.0, fpsi))
     return rc;
   if (!fatm) return CPSTEP_OK;
   NlAtoms A{};

@@ -1392,7 +1392,7 @@ __global__ void __launch_bounds__(256) k_presplit_ees_a(const PreA a) {
 //   Q_tcs(p) = sum_{a in t} Z_t(c natm_t + a, s) S_a(p)
 // as D_t = A_t B_t^T with A_t = Z_t (rows 4 s + c, K = the type's atoms) and
 // B_t = the real views of the type's S (Mn) rows transposed (rows = reals of
-// the points, K = atoms), both FP16 levels (k_presplit_z, k_presplit_st).  One
+// the points, K = atoms), both FP16 levels (k_presplit_force).  One
 // output tile = 32 states x 4 channel rows x 128 reals (64 points); the CTAs
 // of one row tile walk the point tiles (persistent), the K chunks of a tile
 // (the first type's, then the second's, each into its own accumulator)
@@ -1414,7 +1414,7 @@ struct PFArgs {
   int nks[2];            // K steps of type t: cdiv(natm_t, 16)
   int nch[2];
   const float* zmax[2];  // the FP16 scales of Z_t (pow2_scale(*zmax[t])) and of S^T_t
-  const float* smax[2];  // (pow2_scale(*smax[t])), as k_presplit_z / k_presplit_st
+  const float* smax[2];  // (pow2_scale(*smax[t])), as k_presplit_force
   const float2* dyp[2];  // type t, channel c at dyp[t] + c ld_d (FP32)
   int ntile;             // row tiles of B (point tiles)
   int S, npts, ld_d;
@@ -1727,76 +1727,85 @@ __global__ void __launch_bounds__(PP_NTHR, 1) k_pf_tc(const PFArgs p) {
   if (failed && tid == 0) atomicOr(p.err, 1);
 }
 
-// Z levels for k_pf_tc: rows 4 s + c (zero for c >= nch or s >= S), K = the
-// type's atoms a (zero past natm_t): Z(c natm_t + a, s) = zt[s ldz + c natm_t
-// + a], scaled by pow2_scale(*zmax).  One thread = 8 atoms of one row.
-__global__ void k_presplit_z(const double* __restrict__ zt, int ldz, int S, int nch, int natm_t,
-                             int nks, int nrow, const float* __restrict__ zmax,
-                             uint8_t* __restrict__ dst) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (long long)nrow * nks * 2) return;
-  const int r = (int)(i % nrow);
-  const int u = (int)(i / nrow);  // 8-atom unit: K step u / 2, half u & 1
-  const int s = r >> 2, c = r & 3;
-  const float sc = tc::pow2_scale(*zmax);
-  float f[8];
-#pragma unroll
-  for (int e = 0; e < 8; ++e) {
-    const int a = 8 * u + e;
-    f[e] = (s < S && c < nch && a < natm_t) ? (float)zt[(size_t)s * ldz + c * natm_t + a] : 0.f;
-  }
-  split_store_h(dst + ((size_t)(r / ROWS) * nks + (u >> 1)) * STEP_H + core_off(r % ROWS, 8 * (u & 1)),
-                f, sc);
-}
-
-// zs transposed for the atom forces: rows 4 a + c of the atoms of two types
-// (zero for c >= nch), K = states (zero past S).  One thread = 8 states.
+// The FP16 level images of k_pf_tc's operands, all of them in one launch (as six
+// launches they weighed more than their work in small systems):
+//   Z    Z levels of a type: rows 4 s + c (zero for c >= nch or s >= S), K = the
+//        type's atoms; source zt[s ld + c natm_t + a]
+//   ST   transposed real views: rows = reals k of the points, K = atoms (the Mn rows
+//        of a type, FP32) or states (psi, FP64); source rows src[a ld + k]
+//   ZT   zs transposed: rows 4 a + c of the atoms of two types (zero for c >= nch),
+//        K = states
+// scaled by pow2_scale(*mx).  A thread takes 8 of K of a row.
 struct ZtArgs {
   const double* zt[2];  // type t: [S][ldz[t]], inner index c nat[t] + a
   int ldz[2], nat[2], nch[2];
   const float* zmax[2];
 };
-__global__ void k_presplit_zt(const ZtArgs z, int S, int nks, int nrow, uint8_t* __restrict__ dst) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (long long)nrow * nks * 2) return;
-  const int r = (int)(i % nrow), u = (int)(i / nrow);
-  const int al = r >> 2, c = r & 3, t = al >= z.nat[0];
-  const int a = t ? al - z.nat[0] : al, nat = t ? z.nat[1] : z.nat[0];
-  const bool live = a < nat && c < (t ? z.nch[1] : z.nch[0]);
-  const double* src = (t ? z.zt[1] : z.zt[0]) + (live ? c * nat + a : 0);
-  const int ldz = t ? z.ldz[1] : z.ldz[0];
-  const float sc = live ? tc::pow2_scale(t ? *z.zmax[1] : *z.zmax[0]) : 1.f;
-  float f[8];
-#pragma unroll
-  for (int e = 0; e < 8; ++e) {
-    const int s = 8 * u + e;
-    f[e] = live && s < S ? (float)src[(size_t)s * ldz] : 0.f;
+enum { SPLIT_Z, SPLIT_ST, SPLIT_ST64, SPLIT_ZT };
+struct SplitJob {
+  int kind;
+  unsigned first;   // first block
+  int nrow, nks;    // rows (whole tiles), K steps
+  int live, kc;     // rows and K in use (Z: channels and atoms)
+  long long ld;
+  const void* src;
+  const float* mx;
+  uint8_t* dst;
+};
+struct SplitJobs {
+  SplitJob j[6];
+  int n, S;
+  unsigned blocks;
+  ZtArgs z;
+  void add(int kind, int nrow, int nks, int live, int kc, long long ld, const void* src,
+           const float* mx, uint8_t* dst) {
+    j[n++] = SplitJob{kind, blocks, nrow, nks, live, kc, ld, src, mx, dst};
+    blocks += (unsigned)(((long long)nrow * nks * 2 + 255) / 256);
   }
-  split_store_h(dst + ((size_t)(r / ROWS) * nks + (u >> 1)) * STEP_H + core_off(r % ROWS, 8 * (u & 1)),
-                f, sc);
-}
-
-// The real views of a type's Mn rows transposed for k_pf_tc: rows = reals k of
-// the points (zero past 2 npts), K = atoms (zero past natm_t), from the FP32
-// rows sv[a ld_s + k], scaled by pow2_scale(*smax).  One thread = 8 atoms of
-// one real.  With T = double and states for
-// atoms: psi transposed for the atom forces.
-template <typename T>
-__global__ void k_presplit_st(const T* __restrict__ sv, long long ld_s, int kr, int natm_t,
-                              int nks, int nrow, const float* __restrict__ smax,
-                              uint8_t* __restrict__ dst) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (long long)nrow * nks * 2) return;
-  const int k = (int)(i % nrow);
-  const int u = (int)(i / nrow);
-  const float sc = tc::pow2_scale(*smax);
-  float f[8];
+};
+__global__ void __launch_bounds__(256) k_presplit_force(const __grid_constant__ SplitJobs J) {
+  int q = 0;
+  while (q + 1 < J.n && blockIdx.x >= J.j[q + 1].first) ++q;
+  const SplitJob& j = J.j[q];
+  const long long i = (long long)(blockIdx.x - j.first) * 256 + threadIdx.x;
+  if (i >= (long long)j.nrow * j.nks * 2) return;
+  const int r = (int)(i % j.nrow), u = (int)(i / j.nrow);  // 8 of K: K step u / 2, half u & 1
+  const int k0 = 8 * u;
+  float f[8], sc = 1.f;
+  if (j.kind == SPLIT_ZT) {
+    const ZtArgs& z = J.z;
+    const int c = r & 3, al = r >> 2, t = al >= z.nat[0];
+    const int a = t ? al - z.nat[0] : al, nat = t ? z.nat[1] : z.nat[0];
+    const bool live = a < nat && c < (t ? z.nch[1] : z.nch[0]);
+    const double* src = (t ? z.zt[1] : z.zt[0]) + (live ? c * nat + a : 0);
+    const int ldz = t ? z.ldz[1] : z.ldz[0];
+    if (live) sc = tc::pow2_scale(t ? *z.zmax[1] : *z.zmax[0]);
 #pragma unroll
-  for (int e = 0; e < 8; ++e) {
-    const int a = 8 * u + e;
-    f[e] = (k < kr && a < natm_t) ? (float)sv[(size_t)a * ld_s + k] : 0.f;
+    for (int e = 0; e < 8; ++e)
+      f[e] = live && k0 + e < j.kc ? (float)src[(size_t)(k0 + e) * ldz] : 0.f;
+  } else if (j.kind == SPLIT_Z) {
+    const int s = r >> 2, c = r & 3;
+    const bool live = s < J.S && c < j.live;
+    const double* src = static_cast<const double*>(j.src) + (live ? (size_t)s * j.ld + c * j.kc : 0);
+    sc = tc::pow2_scale(*j.mx);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) f[e] = live && k0 + e < j.kc ? (float)src[k0 + e] : 0.f;
+  } else {
+    const bool live = r < j.live;
+    sc = tc::pow2_scale(*j.mx);
+    if (j.kind == SPLIT_ST) {
+      const float* src = static_cast<const float*>(j.src) + r;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) f[e] = live && k0 + e < j.kc ? src[(size_t)(k0 + e) * j.ld] : 0.f;
+    } else {
+      const double* src = static_cast<const double*>(j.src) + r;
+#pragma unroll
+      for (int e = 0; e < 8; ++e)
+        f[e] = live && k0 + e < j.kc ? (float)src[(size_t)(k0 + e) * j.ld] : 0.f;
+    }
   }
-  split_store_h(dst + ((size_t)(k / ROWS) * nks + (u >> 1)) * STEP_H + core_off(k % ROWS, 8 * (u & 1)),
+  split_store_h(j.dst + ((size_t)(r / ROWS) * j.nks + (u >> 1)) * STEP_H +
+                    core_off(r % ROWS, 8 * (u & 1)),
                 f, sc);
 }
 
@@ -1974,12 +1983,54 @@ int ees_tc_sums_pre(cpstep_ctx* c, int nch, const float* dmax, const uint8_t* bl
   return pc_splitk_reduce_launch(c, nsplit, S, nch * jp, 1.0, 0.0, C, S, 0);
 }
 
+// The level images of k_pf_tc's operands for one or two types (k_presplit_force): Z and
+// S^T of each type for the psi force and, where af_z is given, zs^T (ees_ztlv_bytes) and
+// with psi psi^T (psi_t, ees_psit_bytes) for the atom forces.
+int ees_tc_presplit_force(cpstep_ctx* c, int ntyp, const EesForceType* ty, size_t zlv_bytes,
+                          size_t stlv_bytes, const double* psi, const float* pmax, uint8_t* psi_t,
+                          uint8_t* af_z) {
+  using namespace pctc;
+  const int S = c->nstates, kr = 2 * c->npts, snks = cdiv(S, 16);
+  const int tm = cdiv(4 * S, ROWS), ntile = cdiv(kr, ROWS);
+  if (ntyp < 1 || ntyp > 2 || !al16(psi_t) || !al16(af_z)) return CPSTEP_ERR_ARG;
+  SplitJobs J{};
+  J.S = S;
+  int na = 0;
+  for (int t = 0; t < ntyp; ++t) {
+    const EesForceType& y = ty[t];
+    const int nks = cdiv(y.natm_t, 16);
+    if (y.nch < 1 || y.nch > 4 || y.natm_t < 1 || (y.ld_s & 3) || !al16(y.zlv) ||
+        !al16(y.stlv) || zlv_bytes < (size_t)tm * nks * STEP_H ||
+        stlv_bytes < (size_t)ntile * nks * STEP_H || y.ldz < y.nch * y.natm_t)
+      return CPSTEP_ERR_ARG;
+    J.add(SPLIT_Z, tm * ROWS, nks, y.nch, y.natm_t, y.ldz, y.Z, y.zmax, y.zlv);
+    J.add(SPLIT_ST, ntile * ROWS, nks, kr, y.natm_t, y.ld_s, y.sv, y.smax, y.stlv);
+    J.z.zt[t] = y.Z;
+    J.z.ldz[t] = y.ldz;
+    J.z.nat[t] = y.natm_t;
+    J.z.nch[t] = y.nch;
+    J.z.zmax[t] = y.zmax;
+    na += y.natm_t;
+  }
+  if (ntyp == 1) {
+    J.z.zt[1] = J.z.zt[0];
+    J.z.zmax[1] = J.z.zmax[0];
+  }
+  if (af_z) {
+    J.add(SPLIT_ZT, cdiv(4 * na, ROWS) * ROWS, snks, 0, S, 0, nullptr, nullptr, af_z);
+    if (psi) J.add(SPLIT_ST64, ntile * ROWS, snks, kr, S, kr, psi, pmax, psi_t);
+  }
+  k_presplit_force<<<J.blocks, 256, 0, c->stream>>>(J);
+  CPSTEP_LAUNCH_CHECK();
+  return CPSTEP_OK;
+}
+
 // EES psi force of one or two atom types from pre-split operands (k_pf_tc):
 // per type Z column-major [S][ldz] (inner index c natm_t + a) and the FP32
 // Mn rows sv[a ld_s + k], split into zlv and stlv; F += alpha w sum_t
 // (conj(dyp_t) S_t Z_t), F read and written once.
 int ees_tc_force_pre(cpstep_ctx* c, int ntyp, const EesForceType* ty, int ld_d, double alpha,
-                     double* fpsi, size_t zlv_bytes, size_t stlv_bytes) {
+                     double* fpsi) {
   using namespace pctc;
   const int S = c->nstates, npts = c->npts, kr = 2 * npts;
   const int tm = cdiv(4 * S, ROWS), ntile = cdiv(kr, ROWS);
@@ -1989,17 +2040,6 @@ int ees_tc_force_pre(cpstep_ctx* c, int ntyp, const EesForceType* ty, int ld_d, 
   for (int t = 0; t < ntyp; ++t) {
     const EesForceType& y = ty[t];
     const int nks = cdiv(y.natm_t, 16);
-    if (y.nch < 1 || y.nch > 4 || y.natm_t < 1 || (y.ld_s & 3) || !al16(y.zlv) ||
-        !al16(y.stlv) || zlv_bytes < (size_t)tm * nks * STEP_H ||
-        stlv_bytes < (size_t)ntile * nks * STEP_H || y.ldz < y.nch * y.natm_t)
-      return CPSTEP_ERR_ARG;
-    const long long nz = (long long)tm * ROWS * nks * 2, ns = (long long)ntile * ROWS * nks * 2;
-    k_presplit_z<<<(unsigned)((nz + 255) / 256), 256, 0, c->stream>>>(
-        y.Z, y.ldz, S, y.nch, y.natm_t, nks, tm * ROWS, y.zmax, y.zlv);
-    CPSTEP_LAUNCH_CHECK();
-    k_presplit_st<float><<<(unsigned)((ns + 255) / 256), 256, 0, c->stream>>>(
-        y.sv, y.ld_s, kr, y.natm_t, nks, ntile * ROWS, y.smax, y.stlv);
-    CPSTEP_LAUNCH_CHECK();
     pf.a[t] = y.zlv;
     pf.b[t] = y.stlv;
     pf.nks[t] = nks;
@@ -2024,45 +2064,30 @@ int ees_tc_force_pre(cpstep_ctx* c, int ntyp, const EesForceType* ty, int ld_d, 
   return CPSTEP_OK;
 }
 
-// Atom forces of one or two atom types (k_pf_tc<true>): psi split transposed into
-// psi_t (ees_psit_bytes), zs transposed into zlv (ees_ztlv_bytes); partial sums
-// per lattice axis in fpart [*nblk][atoms of the types][3].
+// Atom forces of one or two atom types (k_pf_tc<true>) from the level images psi_t and
+// zlv; partial sums per lattice axis in fpart [*nblk][atoms of the types][3].
 int ees_tc_atom_force(cpstep_ctx* c, int ntyp, const EesForceType* ty, const int* rank0,
-                      const double* psi, const float* pmax, bool split_psi,
-                      const float2* sep, int km, const int2* kw, int ld_d, uint8_t* psi_t,
-                      uint8_t* zlv, double* fpart, int* nblk) {
+                      const float* pmax, const float2* sep, int km, const int2* kw, int ld_d,
+                      const uint8_t* psi_t, const uint8_t* zlv, double* fpart, int* nblk) {
   using namespace pctc;
   const int S = c->nstates, kr = 2 * c->npts, nks = cdiv(S, 16), ntile = cdiv(kr, ROWS);
-  if (ntyp < 1 || ntyp > 2 || (ld_d & 1) || !al16(psi) || !al16(psi_t) || !al16(zlv))
+  if (ntyp < 1 || ntyp > 2 || (ld_d & 1) || !al16(psi_t) || !al16(zlv))
     return CPSTEP_ERR_ARG;
-  if (split_psi) {
-    const long long np = (long long)ntile * ROWS * nks * 2;
-    k_presplit_st<double><<<(unsigned)((np + 255) / 256), 256, 0, c->stream>>>(
-        psi, kr, kr, S, nks, ntile * ROWS, pmax, psi_t);
-    CPSTEP_LAUNCH_CHECK();
-  }
-  ZtArgs z{};
   PFArgs pf{};
   int na = 0;
   for (int t = 0; t < ntyp; ++t) {
-    z.zt[t] = ty[t].Z;
-    z.ldz[t] = ty[t].ldz;
-    z.nat[t] = pf.nat[t] = ty[t].natm_t;
-    z.nch[t] = pf.nch[t] = ty[t].nch;
-    z.zmax[t] = pf.zmax[t] = ty[t].zmax;
+    pf.nat[t] = ty[t].natm_t;
+    pf.nch[t] = ty[t].nch;
+    pf.zmax[t] = ty[t].zmax;
     pf.dyp[t] = ty[t].dyp;
     pf.rank0[t] = rank0[t];
     na += ty[t].natm_t;
   }
   if (ntyp == 1) {
-    z.zt[1] = z.zt[0];
-    z.zmax[1] = pf.zmax[1] = pf.zmax[0];
+    pf.zmax[1] = pf.zmax[0];
     pf.dyp[1] = pf.dyp[0];
   }
   const int tm = cdiv(4 * na, ROWS);
-  const long long nz = (long long)tm * ROWS * nks * 2;
-  k_presplit_zt<<<(unsigned)((nz + 255) / 256), 256, 0, c->stream>>>(z, S, nks, tm * ROWS, zlv);
-  CPSTEP_LAUNCH_CHECK();
   pf.ntyp = 1;
   pf.a[0] = zlv;
   pf.b[0] = psi_t;
