@@ -153,6 +153,7 @@ __global__ void k_scale(const double* __restrict__ part, int nsplit, int ncolp, 
   if (c >= 0 && s < S) {
     const size_t step = (size_t)ncolp * Sp;
     const double* q = part + (size_t)col * Sp + s;
+#pragma unroll 8
     for (int k = 0; k < nsplit; ++k) z += q[k * step];
     const double f = vn[c] * occ[s];
     e = z * z * f;
@@ -398,14 +399,17 @@ int psi_force(cpstep_ctx* c, const Geo& G, int ncolp, double2* f) {
 // rows of states per tile: the smallest of 32, 64, 128 that holds them all
 int tile_rows(int S) { return S <= 32 ? 32 : (S <= 64 ? 64 : 128); }
 
-// K splits of k_sums: enough blocks for the SMs, the split with the fewest
-// block rounds per unit of work
+// K splits of k_sums: the fewest chunks one after the other (block rounds times the
+// chunks of a split) plus the splits' own cost in k_scale's sum, about a twentieth
+// of a chunk each (a chunk of 128 states takes 5.4 us, a partial's load 0.1 to 0.2);
+// four chunks at least.  54 atoms, 101 states of 14,835 points: 22 splits 237 us,
+// 72 80 us.
 int splits(int sms, int tiles, int nchunk) {
   int best = 1;
   double cost = 1e30;
-  for (int k = 1; k <= std::min(64, std::max(1, nchunk / 4)); ++k) {
+  for (int k = 1; k <= std::max(1, std::min(sms, nchunk / 4)); ++k) {
     if ((long long)tiles * k > 4LL * sms && k > 1) break;
-    const double cst = (double)((tiles * k + sms - 1) / sms) / k + 0.002 * k;
+    const double cst = (double)((tiles * k + sms - 1) / sms) * ((nchunk + k - 1) / k) + 0.05 * k;
     if (cst < cost) {
       cost = cst;
       best = k;
