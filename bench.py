@@ -773,7 +773,7 @@ def main():
         "scaling": "weak",
         "vs_baseline": None,
         "dtype": "f32 FFT/density/V.psi with f64 rho/energy accumulation; PairCalc split-BF16 "
-                 "tensor-core products (FP32 accumulate, FP64 sums); Ortho f32 + f64 correction",
+                 "tensor-core products (FP32 accumulate, FP64 sums); Ortho f64 + correction",
         "data": "synthetic",
         "config": {"workload": wname, "parallelism": "replicas" if ws > 1 else "1 GPU",
                    "inputs_vs_L2": "inputs larger than L2: psi %.1f MB FP64 per replica"
