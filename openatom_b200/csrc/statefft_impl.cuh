@@ -629,9 +629,9 @@ __device__ __forceinline__ void shfl_extract_row(const cplx<T> (&v)[ShflCfg<N>::
   }
 }
 
-// K2 (shuffle form): planes -> psi(r).  MODE 0 accumulates occ psi^2 into the
-// group's FP64 registers (row pairs grp, grp + NG, ...), MODE 1 writes psi(r).
-template <typename T, int N, int MODE>
+// K2 (shuffle form): planes -> occ psi^2 accumulated in the group's FP64 registers
+// (row pairs grp, grp + NG, ...).
+template <typename T, int N>
 __global__ void __launch_bounds__(PTHREADS, 1)
 k_xy_fwd_s(const cplx<T>* __restrict__ pen, StateGeom g, const cplx<T>* __restrict__ twx_g,
            const double* __restrict__ occ, int nstates, int spg, double* __restrict__ out) {
@@ -658,7 +658,7 @@ k_xy_fwd_s(const cplx<T>* __restrict__ pen, StateGeom g, const cplx<T>* __restri
     scatter_plane<T, N>(pen + ((size_t)s * N + z) * g.nlpad, plane, g);
     shfl_columns<T, N, false, true>(plane, LDY, g.nplane_x, F, tw, grp, NG);  // FFTW_FORWARD y
     __syncthreads();
-    const double w = (MODE == 0) ? occ[s] : 1.0;
+    const double w = occ[s];
     // every lane of a warp runs the shuffles: groups past the last pair
     // transform row 0 and drop the result
 #pragma unroll
@@ -670,49 +670,36 @@ k_xy_fwd_s(const cplx<T>* __restrict__ pen, StateGeom g, const cplx<T>* __restri
       shfl_build_row<T, N>(plane, LDY, g.nplane_x, ya, F, v);
       F.template dif<true>(v, tw);  // C2R, +i sign
       if (act) {
-        if (MODE == 0) {
 #pragma unroll
-          for (int k = 0; k < M; ++k) {
-            acc[q][0][k] += w * (double)v[k].x * (double)v[k].x;
-            acc[q][1][k] += w * (double)v[k].y * (double)v[k].y;
-          }
-        } else {
-          double* o = out + (((size_t)s * N + z) * N + ya) * N;
-#pragma unroll
-          for (int k = 0; k < M; ++k) {
-            const int x = F.pos(k);
-            o[x] = (double)v[k].x;
-            o[N + x] = (double)v[k].y;
-          }
+        for (int k = 0; k < M; ++k) {
+          acc[q][0][k] += w * (double)v[k].x * (double)v[k].x;
+          acc[q][1][k] += w * (double)v[k].y * (double)v[k].y;
         }
       }
     }
     __syncthreads();
   }
-  if (MODE == 0) {
-    double* o = out + ((size_t)blockIdx.y * N + z) * N * N;
+  double* o = out + ((size_t)blockIdx.y * N + z) * N * N;
 #pragma unroll
-    for (int q = 0; q < QMAX; ++q) {
-      const int pp = grp + NG * q;
-      if (pp < N / 2) {
-        const int ya = 2 * pp;
+  for (int q = 0; q < QMAX; ++q) {
+    const int pp = grp + NG * q;
+    if (pp < N / 2) {
+      const int ya = 2 * pp;
 #pragma unroll
-        for (int k = 0; k < M; ++k) {
-          const int x = F.pos(k);
-          o[(size_t)ya * N + x] = acc[q][0][k];
-          o[(size_t)(ya + 1) * N + x] = acc[q][1][k];
-        }
+      for (int k = 0; k < M; ++k) {
+        const int x = F.pos(k);
+        o[(size_t)ya * N + x] = acc[q][0][k];
+        o[(size_t)(ya + 1) * N + x] = acc[q][1][k];
       }
     }
   }
 }
 
-// K3 (shuffle form): MODE 0 pencils -> psi(r) -> psi V occ -> pencils_out;
-// MODE 1 real f(r) (FP64, [s][z][y][x]) -> pencils_out.
-template <typename T, int N, int MODE>
+// K3 (shuffle form): pencils -> psi(r) -> psi V occ -> pencils_out.
+template <typename T, int N>
 __global__ void __launch_bounds__(PTHREADS, 1)
-k_xy_bwd_s(const cplx<T>* __restrict__ pen, const double* __restrict__ freal,
-           const T* __restrict__ vks, cplx<T>* __restrict__ pen_out, StateGeom g,
+k_xy_bwd_s(const cplx<T>* __restrict__ pen, const T* __restrict__ vks,
+           cplx<T>* __restrict__ pen_out, StateGeom g,
            const cplx<T>* __restrict__ twx_g, const double* __restrict__ occ, int nstates,
            int spg) {
   using S = SShape<T, N>;
@@ -724,39 +711,28 @@ k_xy_bwd_s(const cplx<T>* __restrict__ pen, const double* __restrict__ freal,
   const int z = blockIdx.x;
   const int s0 = blockIdx.y * spg, s1 = min(nstates, s0 + spg);
   for (int i = threadIdx.x; i < N; i += PTHREADS) tw[i] = twx_g[i];
-  const T* vplane = (MODE == 0) ? vks + (size_t)z * N * N : nullptr;
+  const T* vplane = vks + (size_t)z * N * N;
   __syncthreads();
   ShflFft<T, N> F;
   F.init(tw);
   for (int s = s0; s < s1; ++s) {
-    if (MODE == 0) {
-      scatter_plane<T, N>(pen + ((size_t)s * N + z) * g.nlpad, plane, g);
-      shfl_columns<T, N, false, true>(plane, LDY, g.nplane_x, F, tw, grp, NG);
-      __syncthreads();
-    }
-    const T w = (MODE == 0) ? (T)occ[s] : (T)1;
+    scatter_plane<T, N>(pen + ((size_t)s * N + z) * g.nlpad, plane, g);
+    shfl_columns<T, N, false, true>(plane, LDY, g.nplane_x, F, tw, grp, NG);
+    __syncthreads();
+    const T w = (T)occ[s];
     // same trip count for every group of a warp (the shuffles need all lanes)
     for (int p0 = 0; p0 < N / 2; p0 += NG) {
       const int pp = p0 + grp;
       const bool act = pp < N / 2;
       const int ya = act ? 2 * pp : 0;
       cplx<T> v[M];
-      if (MODE == 0) {
-        shfl_build_row<T, N>(plane, LDY, g.nplane_x, ya, F, v);
-        F.template dif<true>(v, tw);  // C2R, +i sign
+      shfl_build_row<T, N>(plane, LDY, g.nplane_x, ya, F, v);
+      F.template dif<true>(v, tw);  // C2R, +i sign
 #pragma unroll
-        for (int k = 0; k < M; ++k) {
-          const int x = F.pos(k);
-          v[k].x *= __ldg(vplane + ya * N + x) * w;
-          v[k].y *= __ldg(vplane + (ya + 1) * N + x) * w;
-        }
-      } else {
-        const double* fs = freal + ((size_t)s * N + z) * N * N;
-#pragma unroll
-        for (int k = 0; k < M; ++k) {
-          const int x = F.pos(k);
-          v[k] = mk<T>((T)fs[ya * N + x], (T)fs[(ya + 1) * N + x]);
-        }
+      for (int k = 0; k < M; ++k) {
+        const int x = F.pos(k);
+        v[k].x *= __ldg(vplane + ya * N + x) * w;
+        v[k].y *= __ldg(vplane + (ya + 1) * N + x) * w;
       }
       F.template dit<false>(v, tw);  // R2C, -i sign
       shfl_extract_row<T, N>(v, plane, LDY, g.nplane_x, ya, F, act);
@@ -2105,8 +2081,8 @@ struct StateFft {
         int ng = std::min(c->ngroups_rho, plane_groups(c, c->nstates, 1));
         int spg = cdiv(c->nstates, ng);
         ng = cdiv(c->nstates, spg);
-        if (int rc = set_smem(k_xy_fwd_s<T, N, 0>, smem)) return rc;
-        k_xy_fwd_s<T, N, 0><<<dim3(N, ng), PTHREADS, smem, c->stream>>>(
+        if (int rc = set_smem(k_xy_fwd_s<T, N>, smem)) return rc;
+        k_xy_fwd_s<T, N><<<dim3(N, ng), PTHREADS, smem, c->stream>>>(
             reinterpret_cast<const cplx<T>*>(j.pen_a), j.g, tws<T>(c).x, occ, c->nstates, spg,
             c->d_rho_part);
         CPSTEP_LAUNCH_CHECK();
@@ -2286,9 +2262,9 @@ struct StateFft {
     if constexpr (ShflCfg<N>::ok) {
       if (c->tune.shfl && !shfl_done) {
         const size_t smem = SShape<T, N>::bytes(j.g.nplane_x);
-        if (int rc = set_smem(k_xy_bwd_s<T, N, 0>, smem)) return rc;
-        k_xy_bwd_s<T, N, 0><<<dim3(N, ng), PTHREADS, smem, c->stream>>>(
-            reinterpret_cast<const cplx<T>*>(j.pen_a), nullptr, vt,
+        if (int rc = set_smem(k_xy_bwd_s<T, N>, smem)) return rc;
+        k_xy_bwd_s<T, N><<<dim3(N, ng), PTHREADS, smem, c->stream>>>(
+            reinterpret_cast<const cplx<T>*>(j.pen_a), vt,
             reinterpret_cast<cplx<T>*>(j.pen_b), j.g, tws<T>(c).x, occ, c->nstates, spg);
         shfl_done = true;
       }
