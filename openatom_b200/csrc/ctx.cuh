@@ -138,6 +138,7 @@ struct AtomData {
   double* fpart = nullptr;
   double* pos = nullptr;  // Cartesian positions [natm][3] (bohr)
   std::vector<double> h_q;  // charges, host copy
+  std::vector<int> h_typ;   // types, host copy
 };
 
 // Isokinetic NHC thermostat of the CP coefficients (cpstep_set_cp_thermostat):
@@ -197,7 +198,8 @@ struct NlData {
   double* zs = nullptr;             // [nstates][natm]
   double* enl_s = nullptr;          // [nstates]
   double* fnl = nullptr;            // [nstates][natm][3]
-  int natm = 0;
+  int natm = 0, ntyp = 0;
+  std::vector<int> typ;             // the atoms' types that the tables below were made for
   // stencil tables (NlAtoms), one block per type: type t starts at entry
   // tab_off[t] (nkf * tab_cap[t] entries), tab_cap[t] = 64 * atoms of type t
   int *tcell = nullptr, *gcell = nullptr, *goff = nullptr, *gent = nullptr, *gcount = nullptr;
@@ -466,6 +468,7 @@ int sf_run(cpstep_ctx* c, const double* psi, const double* occ, double* fpsi, do
 int nl_run(cpstep_ctx* c, const double* psi, const double* occ, double* fpsi, double* energies,
            double* fatm);
 int nl_grid_reserve(cpstep_ctx* c);
+int nl_follow_atoms(cpstep_ctx* c);
 // ees64.cu: the same pass of an FP64 context in G space
 int ees64_set(cpstep_ctx* c, const std::vector<int>& order);
 bool ees64_faster(const cpstep_ctx* c);

@@ -492,36 +492,30 @@ int ees_bspline_launch(cpstep_ctx* c, const double* frac, int natm, int nkf, int
   return CPSTEP_OK;
 }
 
+// What follows the types of all atoms: per-type lists, row offsets, scratch sizes.
+static void nl_types_free(NlData& n) {
+  auto drop = [](auto*& p) {
+    cudaFree(p);
+    p = nullptr;
+  };
+  drop(n.plist); drop(n.pcount); drop(n.tcell); drop(n.tval); drop(n.gcell); drop(n.goff);
+  drop(n.gent); drop(n.gcount);
+  n.grid_ready = 0;
+  drop(n.sep); drop(n.sepf); drop(n.kw); drop(n.psi_t); drop(n.af_z); drop(n.af_part);
+  drop(n.sv); drop(n.csum); drop(n.zt); drop(n.d_hmax); drop(n.blv); drop(n.tsc); drop(n.tinv);
+  drop(n.alv); drop(n.pf_z); drop(n.pf_st); drop(n.d_tch); drop(n.d_vn); drop(n.d_order);
+  for (auto d : n.tdyp) cudaFree(d);
+  n.tdyp.clear();
+  drop(n.e64_act); drop(n.e64_part); drop(n.e64_zs); drop(n.e64_e); drop(n.e64_f);
+  n.gspace_ok = n.gspace64 = 0;
+}
+
 void nl_free(cpstep_ctx* c) {
   NlData& n = c->nl;
+  nl_types_free(n);
   cudaFree(n.dyp); cudaFree(n.line_zneg); cudaFree(n.line_zpos); cudaFree(n.line_xy);
   cudaFree(n.pen_a); cudaFree(n.pen_b); cudaFree(n.tw); cudaFree(n.ig); cudaFree(n.mn);
   cudaFree(n.dmn); cudaFree(n.zpart); cudaFree(n.zs); cudaFree(n.enl_s); cudaFree(n.fnl);
-  cudaFree(n.tcell); cudaFree(n.tval); cudaFree(n.gcell); cudaFree(n.goff); cudaFree(n.gent);
-  cudaFree(n.gcount);
-  cudaFree(n.sep); cudaFree(n.sv); cudaFree(n.d_order); cudaFree(n.d_tch); cudaFree(n.d_vn);
-  cudaFree(n.csum); cudaFree(n.zt);
-  for (auto d : n.tdyp) cudaFree(d);
-  n.tdyp.clear();
-  cudaFree(n.d_hmax);
-  n.d_hmax = nullptr;
-  cudaFree(n.blv);
-  cudaFree(n.tsc);
-  cudaFree(n.tinv);
-  cudaFree(n.alv);
-  cudaFree(n.pf_z);
-  cudaFree(n.pf_st);
-  n.pf_z = n.pf_st = nullptr;
-  n.pf_zbytes = n.pf_stbytes = 0;
-  n.blv = n.alv = nullptr;
-  n.tsc = n.tinv = nullptr;
-  n.alv_bytes = 0;
-  n.sep = nullptr; n.sv = nullptr; n.d_order = nullptr; n.d_tch = nullptr; n.d_vn = nullptr;
-  n.csum = nullptr; n.zt = nullptr; n.gspace_ok = 0;
-  cudaFree(n.plist); cudaFree(n.pcount);
-  cudaFree(n.sepf); cudaFree(n.kw); cudaFree(n.psi_t); cudaFree(n.af_z); cudaFree(n.af_part);
-  cudaFree(n.e64_act); cudaFree(n.e64_part); cudaFree(n.e64_zs); cudaFree(n.e64_e);
-  cudaFree(n.e64_f);
   n = NlData();
 }
 
@@ -557,6 +551,7 @@ int nl_grid_reserve(cpstep_ctx* c) {
       (rc = get(&n.pcount, sizeof(int) * (size_t)at.ntyp * nkf)) ||
       (rc = get(&n.zpart, sizeof(double) * c->nstates * na * kNlInterp * 4)) ||
       (rc = get(&n.zs, sizeof(double) * c->nstates * na)) ||
+      (rc = get(&n.fnl, sizeof(double) * c->nstates * na * 3)) ||
       (rc = get(&n.tcell, sizeof(int) * tot1)) || (rc = get(&n.tval, sizeof(NlVal) * tot1)) ||
       (rc = get(&n.gcell, sizeof(int) * tot1)) || (rc = get(&n.gent, sizeof(int) * tot1)) ||
       (rc = get(&n.goff, sizeof(int) * (tot + (size_t)at.ntyp * nkf))) ||
@@ -569,6 +564,141 @@ int nl_grid_reserve(cpstep_ctx* c) {
 // whether an FP64 context's pass runs in G space (ees64.cu)
 static bool nl_g64(const cpstep_ctx* c) {
   return c->nl.gspace64 && c->tune.ees_gspace && ees64_faster(c);
+}
+
+// The lists, offsets and scratch that follow the atoms' types, for the atoms now set
+static int nl_types_set(cpstep_ctx* c) {
+  NlData& n = c->nl;
+  const AtomData& at = c->atoms;
+  const bool fp64 = c->precision == CPSTEP_PREC_FP64;
+  const size_t na = (size_t)at.natm;
+  const int km = n.km;
+  int rc = CPSTEP_OK;
+  nl_types_free(n);
+  n.typ = at.h_typ;
+  n.ntyp = at.ntyp;
+  // G-space form (mixed contexts): channels per type, S matrices, scratch
+  n.tch.assign(at.ntyp, {});
+  for (int k = 0; k < n.nchan; ++k) n.tch[n.ch_type[k]].push_back(k);
+  n.gspace_ok = c->precision == CPSTEP_PREC_MIXED;
+  for (int t = 0; t < at.ntyp; ++t) n.gspace_ok = n.gspace_ok && n.tch[t].size() <= 4;
+  if (n.gspace_ok) {
+    n.ld_s = (long long)((2 * (size_t)c->npts + 3) / 4 * 4);
+    n.sv_off.assign(at.ntyp, 0);
+    long long tot = 0;
+    size_t csz = 1, zsz = 1;
+    for (int t = 0; t < at.ntyp; ++t) {
+      const int nt = at.tstart[t + 1] - at.tstart[t];
+      n.sv_off[t] = tot;
+      tot += (long long)nt * n.ld_s;
+      csz = std::max(csz, (size_t)n.tch[t].size() * nt * c->nstates);
+      zsz = std::max(zsz, (size_t)c->nstates * (((size_t)n.tch[t].size() * nt + 1) / 2 * 2));
+    }
+    CPSTEP_CUDA_TRY(cudaMalloc(&n.sv, sizeof(float) * (size_t)std::max(tot, 4LL)));
+    CPSTEP_CUDA_TRY(cudaMemset(n.sv, 0, sizeof(float) * (size_t)std::max(tot, 4LL)));
+    CPSTEP_CUDA_TRY(cudaMalloc(&n.sep, sizeof(double2) * na * 6 * (2 * (size_t)km + 1)));
+    CPSTEP_CUDA_TRY(cudaMalloc(&n.sepf, sizeof(float2) * na * 6 * (2 * (size_t)km + 1)));
+    {
+      std::vector<int2> kw((c->npts + 63) / 64 * 64, make_int2(0, 0));
+      for (int p = 0; p < c->npts; ++p)
+        kw[p] = make_int2((int)((unsigned)(c->h_kx[p] & 0xffff) | (unsigned)c->h_ky[p] << 16),
+                          c->h_kz[p]);
+      CPSTEP_CUDA_TRY(cudaMalloc(&n.kw, sizeof(int2) * kw.size()));
+      CPSTEP_CUDA_TRY(cudaMemcpy(n.kw, kw.data(), sizeof(int2) * kw.size(), cudaMemcpyHostToDevice));
+      int two = 1;  // atoms of two types at most, and their partials' rows
+      size_t rows = 1;
+      for (int t = 0; t < at.ntyp; ++t)
+        for (int u = 0; u <= t; ++u) {
+          const int a2 = at.tstart[t + 1] - at.tstart[t] + (u < t ? at.tstart[u + 1] - at.tstart[u] : 0);
+          if (a2 < 1) continue;
+          two = std::max(two, a2);
+          rows = std::max(rows, (size_t)ees_af_blocks(c, a2) * a2);
+        }
+      CPSTEP_CUDA_TRY(cudaMalloc(&n.psi_t, ees_psit_bytes(c->nstates, c->npts)));
+      CPSTEP_CUDA_TRY(cudaMalloc(&n.af_z, ees_ztlv_bytes(c->nstates, two)));
+      CPSTEP_CUDA_TRY(cudaMalloc(&n.af_part, sizeof(double) * 3 * rows));
+    }
+    CPSTEP_CUDA_TRY(cudaMalloc(&n.csum, sizeof(double) * csz));
+    n.zt_slot = zsz;  // two types at a time
+    CPSTEP_CUDA_TRY(cudaMalloc(&n.zt, sizeof(double) * 2 * zsz));
+    n.tdyp.assign(at.ntyp, nullptr);
+    n.tdmax.assign(at.ntyp, 0.f);
+    n.tdmax_c.assign(at.ntyp, std::vector<float>(4, 0.f));
+    n.ld_d32 = (c->npts + 1) / 2 * 2;
+    CPSTEP_CUDA_TRY(cudaMalloc(&n.d_hmax, sizeof(float) * (2 * std::max(1, at.ntyp) + 1)));
+    std::vector<int> htch((size_t)at.ntyp * 4, -1);
+    for (int t = 0; t < at.ntyp; ++t) {
+      const size_t nc = n.tch[t].size();
+      if (!nc) continue;
+      // FP32 copies, rows padded to an even number of points (16-byte rows)
+      const size_t ld = n.ld_d32;
+      CPSTEP_CUDA_TRY(cudaMalloc(&n.tdyp[t], sizeof(float2) * nc * ld));
+      std::vector<double2> hd(c->npts);
+      std::vector<float2> hf(nc * ld, make_float2(0.f, 0.f));
+      for (size_t k = 0; k < nc; ++k) {
+        htch[(size_t)t * 4 + k] = n.tch[t][k];
+        CPSTEP_CUDA_TRY(cudaMemcpy(hd.data(), n.dyp + (size_t)n.tch[t][k] * c->npts,
+                                   sizeof(double2) * c->npts, cudaMemcpyDeviceToHost));
+        for (int q = 0; q < c->npts; ++q) {
+          hf[k * ld + q] = make_float2((float)hd[q].x, (float)hd[q].y);
+          n.tdmax[t] = std::max(n.tdmax[t], (float)std::hypot(hd[q].x, hd[q].y));
+          n.tdmax_c[t][k] = std::max(n.tdmax_c[t][k], (float)std::hypot(hd[q].x, hd[q].y));
+        }
+      }
+      CPSTEP_CUDA_TRY(cudaMemcpy(n.tdyp[t], hf.data(), sizeof(float2) * nc * ld,
+                                 cudaMemcpyHostToDevice));
+    }
+    // FP16 levels of the S rows (zero past each type's rows and past K, never
+    // written there), their scales, and the A operand of the sums
+    {
+      const int K = 2 * c->npts;
+      n.blv_off.assign(at.ntyp, 0);
+      n.tsoff.assign(at.ntyp, 0);
+      size_t bl = 0;
+      long long ts = 0;
+      int nchmax = 1;
+      for (int t = 0; t < at.ntyp; ++t) {
+        const int nt = at.tstart[t + 1] - at.tstart[t];
+        n.blv_off[t] = bl;
+        n.tsoff[t] = ts;
+        bl += ees_lv_bytes(std::max(1, nt), K);
+        ts += nt;
+        nchmax = std::max(nchmax, (int)n.tch[t].size());
+      }
+      CPSTEP_CUDA_TRY(cudaMalloc(&n.blv, bl));
+      CPSTEP_CUDA_TRY(cudaMemset(n.blv, 0, bl));
+      CPSTEP_CUDA_TRY(cudaMalloc(&n.tsc, sizeof(float) * (size_t)std::max(1LL, ts)));
+      CPSTEP_CUDA_TRY(cudaMalloc(&n.tinv, sizeof(float) * (size_t)std::max(1LL, ts)));
+      n.alv_bytes = ees_lv_bytes(nchmax * c->nstates, K);  // per type; two types at a time
+      CPSTEP_CUDA_TRY(cudaMalloc(&n.alv, 2 * n.alv_bytes));
+      int ntmax = 1;
+      for (int t = 0; t < at.ntyp; ++t) ntmax = std::max(ntmax, at.tstart[t + 1] - at.tstart[t]);
+      n.pf_zbytes = ees_pf_zbytes(c->nstates, ntmax);
+      n.pf_stbytes = ees_pf_stbytes(c->npts, ntmax);
+      CPSTEP_CUDA_TRY(cudaMalloc(&n.pf_z, 2 * n.pf_zbytes));  // two types at a time
+      CPSTEP_CUDA_TRY(cudaMalloc(&n.pf_st, 2 * n.pf_stbytes));
+    }
+    CPSTEP_CUDA_TRY(cudaMalloc(&n.d_tch, sizeof(int) * htch.size()));
+    CPSTEP_CUDA_TRY(cudaMemcpy(n.d_tch, htch.data(), sizeof(int) * htch.size(),
+                               cudaMemcpyHostToDevice));
+    CPSTEP_CUDA_TRY(cudaMalloc(&n.d_vn, sizeof(double) * n.nchan));
+    CPSTEP_CUDA_TRY(cudaMemcpy(n.d_vn, n.ch_vn.data(), sizeof(double) * n.nchan,
+                               cudaMemcpyHostToDevice));
+    std::vector<int> hrank(na), horder(na);
+    CPSTEP_CUDA_TRY(cudaMemcpy(hrank.data(), at.rank, sizeof(int) * na, cudaMemcpyDeviceToHost));
+    for (int a = 0; a < (int)na; ++a) horder[hrank[a]] = a;
+    CPSTEP_CUDA_TRY(cudaMalloc(&n.d_order, sizeof(int) * na));
+    CPSTEP_CUDA_TRY(cudaMemcpy(n.d_order, horder.data(), sizeof(int) * na,
+                               cudaMemcpyHostToDevice));
+  }
+  if (fp64) {
+    std::vector<int> hrank(na), horder(na);
+    CPSTEP_CUDA_TRY(cudaMemcpy(hrank.data(), at.rank, sizeof(int) * na, cudaMemcpyDeviceToHost));
+    for (int a = 0; a < (int)na; ++a) horder[hrank[a]] = a;
+    if ((rc = ees64_set(c, horder))) return rc;
+  }
+  n.on = 1;
+  return nl_g64(c) ? CPSTEP_OK : nl_grid_reserve(c);
 }
 
 int nl_set(cpstep_ctx* c, int nkf, int n_interp, int nchan, const int* ch_type, const int* ch_l,
@@ -710,137 +840,33 @@ int nl_set(cpstep_ctx* c, int nkf, int n_interp, int nchan, const int* ch_type, 
   CPSTEP_CUDA_TRY(cudaMalloc(&n.dyp, sizeof(double2) * dyp.size()));
   CPSTEP_CUDA_TRY(cudaMemcpy(n.dyp, dyp.data(), sizeof(double2) * dyp.size(),
                              cudaMemcpyHostToDevice));
-  const bool fp64 = c->precision == CPSTEP_PREC_FP64;
   const size_t na = (size_t)at.natm;
   CPSTEP_CUDA_TRY(cudaMalloc(&n.ig, sizeof(int) * na * 3 * kNlInterp));
   CPSTEP_CUDA_TRY(cudaMalloc(&n.mn, sizeof(double) * na * 3 * kNlInterp));
   CPSTEP_CUDA_TRY(cudaMalloc(&n.dmn, sizeof(double) * na * 3 * kNlInterp));
   CPSTEP_CUDA_TRY(cudaMalloc(&n.enl_s, sizeof(double) * c->nstates));
-  CPSTEP_CUDA_TRY(cudaMalloc(&n.fnl, sizeof(double) * c->nstates * na * 3));
-  // G-space form (mixed contexts): channels per type, S matrices, scratch
   n.km = km;
-  n.tch.assign(at.ntyp, {});
-  for (int k = 0; k < nchan; ++k) n.tch[ch_type[k]].push_back(k);
-  n.gspace_ok = c->precision == CPSTEP_PREC_MIXED;
-  for (int t = 0; t < at.ntyp; ++t) n.gspace_ok = n.gspace_ok && n.tch[t].size() <= 4;
-  if (n.gspace_ok) {
-    n.ld_s = (long long)((2 * (size_t)c->npts + 3) / 4 * 4);
-    n.sv_off.assign(at.ntyp, 0);
-    long long tot = 0;
-    size_t csz = 1, zsz = 1;
-    for (int t = 0; t < at.ntyp; ++t) {
-      const int nt = at.tstart[t + 1] - at.tstart[t];
-      n.sv_off[t] = tot;
-      tot += (long long)nt * n.ld_s;
-      csz = std::max(csz, (size_t)n.tch[t].size() * nt * c->nstates);
-      zsz = std::max(zsz, (size_t)c->nstates * (((size_t)n.tch[t].size() * nt + 1) / 2 * 2));
-    }
-    CPSTEP_CUDA_TRY(cudaMalloc(&n.sv, sizeof(float) * (size_t)std::max(tot, 4LL)));
-    CPSTEP_CUDA_TRY(cudaMemset(n.sv, 0, sizeof(float) * (size_t)std::max(tot, 4LL)));
-    CPSTEP_CUDA_TRY(cudaMalloc(&n.sep, sizeof(double2) * na * 6 * (2 * (size_t)km + 1)));
-    CPSTEP_CUDA_TRY(cudaMalloc(&n.sepf, sizeof(float2) * na * 6 * (2 * (size_t)km + 1)));
-    {
-      std::vector<int2> kw((c->npts + 63) / 64 * 64, make_int2(0, 0));
-      for (int p = 0; p < c->npts; ++p)
-        kw[p] = make_int2((int)((unsigned)(c->h_kx[p] & 0xffff) | (unsigned)c->h_ky[p] << 16),
-                          c->h_kz[p]);
-      CPSTEP_CUDA_TRY(cudaMalloc(&n.kw, sizeof(int2) * kw.size()));
-      CPSTEP_CUDA_TRY(cudaMemcpy(n.kw, kw.data(), sizeof(int2) * kw.size(), cudaMemcpyHostToDevice));
-      int two = 1;  // atoms of two types at most, and their partials' rows
-      size_t rows = 1;
-      for (int t = 0; t < at.ntyp; ++t)
-        for (int u = 0; u <= t; ++u) {
-          const int a2 = at.tstart[t + 1] - at.tstart[t] + (u < t ? at.tstart[u + 1] - at.tstart[u] : 0);
-          if (a2 < 1) continue;
-          two = std::max(two, a2);
-          rows = std::max(rows, (size_t)ees_af_blocks(c, a2) * a2);
-        }
-      CPSTEP_CUDA_TRY(cudaMalloc(&n.psi_t, ees_psit_bytes(c->nstates, c->npts)));
-      CPSTEP_CUDA_TRY(cudaMalloc(&n.af_z, ees_ztlv_bytes(c->nstates, two)));
-      CPSTEP_CUDA_TRY(cudaMalloc(&n.af_part, sizeof(double) * 3 * rows));
-    }
-    CPSTEP_CUDA_TRY(cudaMalloc(&n.csum, sizeof(double) * csz));
-    n.zt_slot = zsz;  // two types at a time
-    CPSTEP_CUDA_TRY(cudaMalloc(&n.zt, sizeof(double) * 2 * zsz));
-    n.tdyp.assign(at.ntyp, nullptr);
-    n.tdmax.assign(at.ntyp, 0.f);
-    n.tdmax_c.assign(at.ntyp, std::vector<float>(4, 0.f));
-    n.ld_d32 = (c->npts + 1) / 2 * 2;
-    CPSTEP_CUDA_TRY(cudaMalloc(&n.d_hmax, sizeof(float) * (2 * std::max(1, at.ntyp) + 1)));
-    std::vector<int> htch((size_t)at.ntyp * 4, -1);
-    for (int t = 0; t < at.ntyp; ++t) {
-      const size_t nc = n.tch[t].size();
-      if (!nc) continue;
-      // FP32 copies, rows padded to an even number of points (16-byte rows)
-      const size_t ld = n.ld_d32;
-      CPSTEP_CUDA_TRY(cudaMalloc(&n.tdyp[t], sizeof(float2) * nc * ld));
-      std::vector<double2> hd(c->npts);
-      std::vector<float2> hf(nc * ld, make_float2(0.f, 0.f));
-      for (size_t k = 0; k < nc; ++k) {
-        htch[(size_t)t * 4 + k] = n.tch[t][k];
-        CPSTEP_CUDA_TRY(cudaMemcpy(hd.data(), n.dyp + (size_t)n.tch[t][k] * c->npts,
-                                   sizeof(double2) * c->npts, cudaMemcpyDeviceToHost));
-        for (int q = 0; q < c->npts; ++q) {
-          hf[k * ld + q] = make_float2((float)hd[q].x, (float)hd[q].y);
-          n.tdmax[t] = std::max(n.tdmax[t], (float)std::hypot(hd[q].x, hd[q].y));
-          n.tdmax_c[t][k] = std::max(n.tdmax_c[t][k], (float)std::hypot(hd[q].x, hd[q].y));
-        }
-      }
-      CPSTEP_CUDA_TRY(cudaMemcpy(n.tdyp[t], hf.data(), sizeof(float2) * nc * ld,
-                                 cudaMemcpyHostToDevice));
-    }
-    // FP16 levels of the S rows (zero past each type's rows and past K, never
-    // written there), their scales, and the A operand of the sums
-    {
-      const int K = 2 * c->npts;
-      n.blv_off.assign(at.ntyp, 0);
-      n.tsoff.assign(at.ntyp, 0);
-      size_t bl = 0;
-      long long ts = 0;
-      int nchmax = 1;
-      for (int t = 0; t < at.ntyp; ++t) {
-        const int nt = at.tstart[t + 1] - at.tstart[t];
-        n.blv_off[t] = bl;
-        n.tsoff[t] = ts;
-        bl += ees_lv_bytes(std::max(1, nt), K);
-        ts += nt;
-        nchmax = std::max(nchmax, (int)n.tch[t].size());
-      }
-      CPSTEP_CUDA_TRY(cudaMalloc(&n.blv, bl));
-      CPSTEP_CUDA_TRY(cudaMemset(n.blv, 0, bl));
-      CPSTEP_CUDA_TRY(cudaMalloc(&n.tsc, sizeof(float) * (size_t)std::max(1LL, ts)));
-      CPSTEP_CUDA_TRY(cudaMalloc(&n.tinv, sizeof(float) * (size_t)std::max(1LL, ts)));
-      n.alv_bytes = ees_lv_bytes(nchmax * c->nstates, K);  // per type; two types at a time
-      CPSTEP_CUDA_TRY(cudaMalloc(&n.alv, 2 * n.alv_bytes));
-      int ntmax = 1;
-      for (int t = 0; t < at.ntyp; ++t) ntmax = std::max(ntmax, at.tstart[t + 1] - at.tstart[t]);
-      n.pf_zbytes = ees_pf_zbytes(c->nstates, ntmax);
-      n.pf_stbytes = ees_pf_stbytes(c->npts, ntmax);
-      CPSTEP_CUDA_TRY(cudaMalloc(&n.pf_z, 2 * n.pf_zbytes));  // two types at a time
-      CPSTEP_CUDA_TRY(cudaMalloc(&n.pf_st, 2 * n.pf_stbytes));
-    }
-    CPSTEP_CUDA_TRY(cudaMalloc(&n.d_tch, sizeof(int) * htch.size()));
-    CPSTEP_CUDA_TRY(cudaMemcpy(n.d_tch, htch.data(), sizeof(int) * htch.size(),
-                               cudaMemcpyHostToDevice));
-    CPSTEP_CUDA_TRY(cudaMalloc(&n.d_vn, sizeof(double) * nchan));
-    CPSTEP_CUDA_TRY(cudaMemcpy(n.d_vn, n.ch_vn.data(), sizeof(double) * nchan,
-                               cudaMemcpyHostToDevice));
-    std::vector<int> hrank(na), horder(na);
-    CPSTEP_CUDA_TRY(cudaMemcpy(hrank.data(), at.rank, sizeof(int) * na, cudaMemcpyDeviceToHost));
-    for (int a = 0; a < (int)na; ++a) horder[hrank[a]] = a;
-    CPSTEP_CUDA_TRY(cudaMalloc(&n.d_order, sizeof(int) * na));
-    CPSTEP_CUDA_TRY(cudaMemcpy(n.d_order, horder.data(), sizeof(int) * na,
-                               cudaMemcpyHostToDevice));
-  }
-  if (fp64) {
-    std::vector<int> hrank(na), horder(na);
-    CPSTEP_CUDA_TRY(cudaMemcpy(hrank.data(), at.rank, sizeof(int) * na, cudaMemcpyDeviceToHost));
-    for (int a = 0; a < (int)na; ++a) horder[hrank[a]] = a;
-    if ((rc = ees64_set(c, horder))) return rc;
-  }
-  n.on = 1;
-  if (!nl_g64(c) && (rc = nl_grid_reserve(c))) n.on = 0;
+  if ((rc = nl_types_set(c))) n.on = 0;
   return rc;
+}
+
+// Atoms were set again: the same number with other types (an atom that has become
+// an O has channels now, and every rank may have moved) makes the tables anew.
+// Other numbers, or a channel of a type that is gone, leave them stale, which the
+// next pass reports.
+int nl_follow_atoms(cpstep_ctx* c) {
+  NlData& n = c->nl;
+  const AtomData& at = c->atoms;
+  if (!n.on || at.natm != n.natm || (at.ntyp == n.ntyp && at.h_typ == n.typ)) return CPSTEP_OK;
+  for (int t : n.ch_type)
+    if (t >= at.ntyp) return CPSTEP_OK;
+  const int rc = nl_types_set(c);
+  if (rc) n.typ.clear();
+  return rc;
+}
+
+static bool nl_stale(const cpstep_ctx* c) {
+  return c->nl.natm != c->atoms.natm || c->nl.ntyp != c->atoms.ntyp || c->nl.typ != c->atoms.h_typ;
 }
 
 // B-spline factors of the atoms and their separable transforms (n.sep)
@@ -971,7 +997,7 @@ static bool nl_gmixed(const cpstep_ctx* c) {
 int nl_front(cpstep_ctx* c, const double* psi, const double* occ, bool forces, NlFront* h,
              bool* split) {
   *split = false;
-  if (!c->nl.on || c->nl.natm != c->atoms.natm) return CPSTEP_OK;  // nl_run reports it
+  if (!c->nl.on || nl_stale(c)) return CPSTEP_OK;  // nl_run reports it
   if (nl_gmixed(c)) {
     const std::vector<int> tl = nl_types(c);
     if (tl.size() > 2) return CPSTEP_OK;
@@ -1000,7 +1026,7 @@ int nl_run(cpstep_ctx* c, const double* psi, const double* occ, double* fpsi, do
     cpstep_set_error("ees_nonlocal: call cpstep_set_nonlocal first");
     return CPSTEP_ERR_STATE;
   }
-  if (n.natm != c->atoms.natm) {
+  if (nl_stale(c)) {
     cpstep_set_error("ees_nonlocal: atoms changed since cpstep_set_nonlocal");
     return CPSTEP_ERR_STATE;
   }

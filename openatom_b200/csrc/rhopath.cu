@@ -1028,6 +1028,7 @@ int atoms_set(cpstep_ctx* c, int natm, int ntyp, const int* typ, const double* p
     return rc;
   a.h_q.resize(natm);
   for (int i = 0; i < natm; ++i) a.h_q[i] = q[t[i]];
+  a.h_typ = t;
   a.natm = natm;
   a.ntyp = ntyp;
   a.nspl = nspl;
@@ -1048,7 +1049,8 @@ int atoms_set(cpstep_ctx* c, int natm, int ntyp, const int* typ, const double* p
   CPSTEP_LAUNCH_CHECK();
   if (!c->d_hmati) CPSTEP_CUDA_TRY(cudaMalloc(&c->d_hmati, sizeof(double) * 9));
   CPSTEP_CUDA_TRY(cudaMemcpy(c->d_hmati, c->hmati, sizeof(double) * 9, cudaMemcpyHostToDevice));
-  if (c->eloc.on) return eesloc_alloc(c);  // the EES form's tables follow the atoms
+  if ((rc = nl_follow_atoms(c))) return rc;  // the non-local pass's tables follow their types,
+  if (c->eloc.on) return eesloc_alloc(c);    // the EES form's the atoms
   return CPSTEP_OK;
 }
 

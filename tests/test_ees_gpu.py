@@ -228,3 +228,93 @@ def test_mixed_atom_forces_tile_edges(states, atoms, keep):
     for a, b in zip(*out):
         assert np.max(np.abs(b)) > 0.0
         assert np.max(np.abs(a - b)) <= 1e-5 * np.max(np.abs(b))
+
+
+def _retyped(s, typ):
+    """`s` with the same positions and other atom types."""
+    import copy
+    t = copy.copy(s)
+    t.typ = np.ascontiguousarray(typ, dtype=np.asarray(s.typ).dtype)
+    return t
+
+
+@pytest.mark.parametrize("precision,form,keep", [
+    ("fp64", 1, None), ("fp64", 1, (0, 0)), ("fp64", 0, None), ("mixed", 1, None),
+    ("mixed", 1, (0, 0)), ("mixed", 0, None)])
+def test_atoms_of_other_types_after_set_nonlocal(precision, form, keep):
+    """set_atoms with the same number of atoms and other types after
+    set_nonlocal (the types permuted, and other counts of each): the pass is the
+    one of a context that saw these atoms only, bit for bit.  `keep`: one channel
+    on type 0 only, so that atoms gain and lose their projectors."""
+    if not cuda_ok():
+        pytest.skip("no CUDA device")
+    import torch
+    from openatom_b200.context import StepContext
+    from openatom_b200.system import System
+    s = System(12.0, 25.0, 33, {"O": 9, "H": 27}, nfft=40, seed=5)
+    if keep is not None:
+        s.channels = [c for c in s.channels if (c["type"], c["l"]) == keep]
+    typ = np.asarray(s.typ)
+    sets = [_retyped(s, typ[::-1]), _retyped(s, 1 - typ), s]
+    psi, occ = s.psi(), torch.ones(s.nstates, dtype=torch.float64, device="cuda")
+
+    def results(ctx):
+        f, e, fa = ctx.ees_nonlocal(psi, occ)
+        return float(e[7]), f.cpu().numpy(), fa.cpu().numpy()
+
+    def context(t):
+        ctx = StepContext(s.layout, s.nstates, precision=precision)
+        ctx.set_atoms(t)
+        ctx.set_nonlocal(t)
+        ctx.tune_set({"ees_gspace": form})
+        return ctx
+
+    ctx = context(s)
+    try:
+        results(ctx)
+        for t in sets:
+            ctx.set_atoms(t)
+            got = results(ctx)
+            ref = context(t)
+            try:
+                want = results(ref)
+            finally:
+                ref.close()
+            assert want[0] != 0.0 and np.max(np.abs(want[2])) > 0.0
+            for a, b in zip(got, want):
+                assert np.array_equal(a, b)
+    finally:
+        ctx.close()
+
+
+def test_other_atom_count_after_set_nonlocal_is_refused():
+    """Another number of atoms, or fewer types than the channels name, leaves the
+    non-local data stale: an error, and the first atoms again make it good."""
+    if not cuda_ok():
+        pytest.skip("no CUDA device")
+    import copy
+    import torch
+    from openatom_b200 import _lib
+    from openatom_b200.context import StepContext
+    from openatom_b200.system import System
+    s = System(12.0, 25.0, 8, {"O": 3, "H": 6}, nfft=40, seed=5)
+    fewer = copy.copy(s)
+    fewer.pos, fewer.typ = s.pos[:-1], s.typ[:-1]
+    one = copy.copy(s)  # all atoms of one type: type 1 and its channels are gone
+    one.typ = np.zeros_like(s.typ)
+    one.tab = dict(s.tab, q=s.tab["q"][:1], vps=s.tab["vps"][:1], gzvps=s.tab["gzvps"][:1])
+    psi, occ = s.psi(), torch.ones(s.nstates, dtype=torch.float64, device="cuda")
+    ctx = StepContext(s.layout, s.nstates, precision="fp64")
+    try:
+        ctx.set_atoms(s)
+        ctx.set_nonlocal(s)
+        e0 = float(ctx.ees_nonlocal(psi, occ)[1][7])
+        for t in (fewer, one):
+            ctx.set_atoms(t)
+            with pytest.raises(_lib.CpstepError) as err:
+                ctx.ees_nonlocal(psi, occ)
+            assert err.value.code == 5 and "atoms changed" in str(err.value)
+            ctx.set_atoms(s)
+            assert float(ctx.ees_nonlocal(psi, occ)[1][7]) == e0
+    finally:
+        ctx.close()
