@@ -206,7 +206,8 @@ __global__ void __launch_bounds__(NT) k_ortho(Work w) {
   double* X = w.newton ? w.X : w.T;
   for (size_t e = gtid; e < (size_t)nn; e += gstride) {
     const int i = e / n, j = e % n;
-    X[e] = w.newton ? 0.5 * (A[e] + A[(size_t)j * n + i]) * post : A[e] * post;
+    if (it == 0) X[e] = i == j ? post : 0.0;  // tol >= 1: no iteration, A = I
+    else X[e] = w.newton ? 0.5 * (A[e] + A[(size_t)j * n + i]) * post : A[e] * post;
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     w.status[0] = it;
@@ -318,6 +319,10 @@ __global__ void __launch_bounds__(SNT) k_ortho_small(Work w) {
     tol_now = r;
     double* t1 = A; A = A2; A2 = t1;
     double* t2 = B; B = B2; B2 = t2;
+  }
+  if (it == 0) {  // tol >= 1: no iteration, A = I
+    if (tid < n) A[tid * SLD + tid] = 1.0;
+    __syncthreads();
   }
   if (tid == 0) {
     w.status[0] = it;

@@ -187,6 +187,29 @@ def test_ortho_tile_edges(pc, n, mixed):
     assert np.max(np.abs(T.T @ (S / 2) @ T - np.eye(n))) < 1e-12
 
 
+@pytest.mark.parametrize("n", [1, 33, 64, 65, 130])
+@pytest.mark.parametrize("mixed,scale", [(False, False), (False, True), (True, False), (True, True)])
+def test_ortho_without_an_iteration(pc, n, mixed, scale):
+    """tol >= 1 runs no iteration: T is the starting iterate I times (sigma/2)^(-1/2),
+    in the mixed mode with the correction X (I - R/2 + 3 R^2/8), R = X (S/2) X - I,
+    whatever an earlier call left in the workspace.  At most 130 terms of order 1
+    in three products: 1e-12."""
+    import torch
+    rng = np.random.default_rng(n)
+    R = rng.standard_normal((n, n)) / (20.0 * np.sqrt(n))
+    S = 2.0 * np.eye(n) + R + R.T
+    d = torch.from_numpy(S).cuda()
+    pc["ctx"].ortho_tmat(d, mixed=mixed, scale=True, tol=2e-6, max_iter=40)
+    T, it, rms = pc["ctx"].ortho_tmat(d, mixed=mixed, scale=scale, tol=1.0, max_iter=10)
+    sigma = max(2.0, 1.0001 * np.abs(S).sum(1).max()) if scale else 2.0
+    want = np.eye(n) * np.sqrt(2.0 / sigma)
+    if mixed:
+        E = want @ (S / 2) @ want - np.eye(n)
+        want = want @ (np.eye(n) - 0.5 * E + 0.375 * E @ E)
+    assert it == 0 and rms == 1.0
+    assert np.max(np.abs(T.cpu().numpy() - want)) < 1e-12
+
+
 @pytest.mark.parametrize("m,n,k", [(1, 1, 1), (32, 33, 15), (31, 32, 128), (64, 1, 129), (97, 65, 16),
                                    (128, 128, 300)])
 def test_dgemm_tile_edges(pc, m, n, k):
