@@ -169,6 +169,7 @@ struct AtomNvt {
 // Structure-factor (non-EES) non-local state, l = 0 (cpstep_set_nonlocal_sf).
 struct SfData {
   int on = 0, n = 0, ldz = 0;       // n non-local atoms (type order)
+  std::vector<int> typ;             // the atoms' types at cpstep_set_nonlocal_sf
   int* atom = nullptr;              // [n] atom index
   int* ptab = nullptr;              // [n] projector table of the atom's type
   double* proj = nullptr;           // [tables][npts] y00 v_0(|G|)

@@ -196,6 +196,7 @@ int sf_set(cpstep_ctx* c, int nchan, const int* ch_type, const int* ch_l, const 
   CPSTEP_CUDA_TRY(cudaMemset(f.zs, 0, sizeof(double) * (size_t)f.ldz * S));
   CPSTEP_CUDA_TRY(cudaMalloc(&f.enl_s, sizeof(double) * S));
   CPSTEP_CUDA_TRY(cudaMalloc(&f.fnl, sizeof(double) * (size_t)S * at.natm * 3));
+  f.typ = typ;
   f.on = 1;
   nl_free(c);  // the EES path and this one exclude each other
   return CPSTEP_OK;
@@ -207,6 +208,10 @@ int sf_run(cpstep_ctx* c, const double* psi, const double* occ, double* fpsi, do
   SfData& f = c->sf;
   if (!f.on) {
     cpstep_set_error("sf_nonlocal: call cpstep_set_nonlocal_sf first");
+    return CPSTEP_ERR_STATE;
+  }
+  if (f.typ != c->atoms.h_typ) {  // the list of non-local atoms and the force scratch follow them
+    cpstep_set_error("sf_nonlocal: atoms changed since cpstep_set_nonlocal_sf");
     return CPSTEP_ERR_STATE;
   }
   const int S = c->nstates, np = c->npts, K = 2 * np, n = f.n, natm = c->atoms.natm;

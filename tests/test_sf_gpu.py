@@ -112,3 +112,34 @@ def test_step_with_sf_nonlocal_matches_oracle(sfstep, precision):
             assert np.max(np.abs(f.cpu().numpy() - fr)) <= 1e-5
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("change", ["types", "count"])
+def test_sf_other_atoms_are_refused(sfsys, change):
+    """Atoms of other types, or another number of them, after set_nonlocal_sf: the
+    list of non-local atoms is not theirs, an error; the first atoms again make
+    it good."""
+    import copy
+    import torch
+    from openatom_b200 import _lib
+    from openatom_b200.context import StepContext
+    s = sfsys
+    t = copy.copy(s)
+    if change == "types":
+        t.typ = np.ascontiguousarray(np.asarray(s.typ)[::-1])
+    else:
+        t.pos, t.typ = np.concatenate([s.pos, s.pos[:1] + 0.5]), np.append(s.typ, s.typ[0])
+    psi, occ = s.psi(), torch.ones(s.nstates, dtype=torch.float64, device="cuda")
+    ctx = StepContext(s.layout, s.nstates, precision="fp64")
+    try:
+        ctx.set_atoms(s)
+        ctx.set_nonlocal_sf(s)
+        e0 = float(ctx.sf_nonlocal(psi, occ)[1][7])
+        ctx.set_atoms(t)
+        with pytest.raises(_lib.CpstepError) as err:
+            ctx.sf_nonlocal(psi, occ)
+        assert err.value.code == 5 and "atoms changed" in str(err.value)
+        ctx.set_atoms(s)
+        assert float(ctx.sf_nonlocal(psi, occ)[1][7]) == e0
+    finally:
+        ctx.close()
