@@ -1406,6 +1406,7 @@ constexpr int PF_STAGE = 2 * PF_OPB;      // 64 KB
 constexpr int PF_NST = 3;
 constexpr int PF_BYTES = 1024 + PF_NST * PF_STAGE;
 constexpr uint32_t PF_TMEM_COLS = 4 * ROWS;  // [tile parity][type] accumulators
+constexpr int PF_FOLD = 256 / PF_KC;         // chunks of states an atom-force accumulator takes
 
 struct PFArgs {
   int ntyp;              // 1 or 2
@@ -1439,7 +1440,11 @@ struct PFArgs {
 // of an atom, P_a = sum_c dyp_c G_ac, and lane c < 3 sums
 // w Re(conj(P_a) dS_a) of lattice axis c over the points in FP64 (FP32 within
 // 16 points): fpart.  One product of the size of Z, where sums with the three
-// gradients of S took three.
+// gradients of S took three.  The tensor units' FP32 sums lose more the longer
+// they run (2-norm error of the forces with the whole sum in one accumulator: 1.9e-6
+// at 128 states, 3.0e-6 at 256, 3.7e-6 at 512, 4.9e-6 at 1024), so an accumulator
+// takes 256 states: two of them, the pair that the two types have in the psi force,
+// make a tile, and the epilogue, linear in G, runs once per 512 states.
 template <bool ATOM>
 __global__ void __launch_bounds__(PP_NTHR, 1) k_pf_tc(const PFArgs p) {
   extern __shared__ uint8_t dsm[];
@@ -1454,11 +1459,21 @@ __global__ void __launch_bounds__(PP_NTHR, 1) k_pf_tc(const PFArgs p) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int m = blockIdx.y;
   const int ntyp = ATOM ? 1 : p.ntyp;
+  const int nacc = ATOM ? 2 : ntyp;                                  // accumulators of a tile
   const int nkc0 = (p.nks[0] + PF_KS - 1) / PF_KS;                   // K chunks per tile, type 0
   const int nkc1 = ntyp > 1 ? (p.nks[1] + PF_KS - 1) / PF_KS : 0;    // type 1
-  // this CTA's point tiles: blockIdx.x, + gridDim.x, ...
-  const int ntl = p.ntile > (int)blockIdx.x ? (p.ntile - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
-  const int nitem = ntl * (nkc0 + nkc1);
+  // this CTA's point tiles: blockIdx.x, + gridDim.x, ...; ATOM: each nseg times, 2 PF_FOLD
+  // chunks of states at a time
+  const int npt = p.ntile > (int)blockIdx.x ? (p.ntile - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+  const int nseg = ATOM ? (nkc0 + 2 * PF_FOLD - 1) / (2 * PF_FOLD) : 1;
+  const int ntl = npt * nseg;
+  const int nitem = npt * (nkc0 + nkc1);
+  auto tile_of = [&](int tl) { return (int)blockIdx.x + (ATOM ? tl / nseg : tl) * (int)gridDim.x; };
+  // first chunk and chunks of accumulator t of tile tl
+  auto chunk0 = [&](int tl, int t) { return ATOM ? (2 * (tl % nseg) + t) * PF_FOLD : 0; };
+  auto chunks = [&](int tl, int t) {
+    return ATOM ? max(0, min(PF_FOLD, nkc0 - chunk0(tl, t))) : (t == 0 ? nkc0 : nkc1);
+  };
 
   if (warp == 0) tc::tmem_alloc(&tslot, PF_TMEM_COLS);
   if (tid == 0) {
@@ -1486,12 +1501,11 @@ __global__ void __launch_bounds__(PP_NTHR, 1) k_pf_tc(const PFArgs p) {
       int req = 0;
       bool bad = false;
       for (int tl = 0; tl < ntl && !bad; ++tl) {
-        const int n = blockIdx.x + tl * gridDim.x;
-        for (int t = 0; t < ntyp && !bad; ++t) {
-          const int nkc = t == 0 ? nkc0 : nkc1, nks = t == 0 ? p.nks[0] : p.nks[1];
-          const uint8_t* ga = t == 0 ? p.a[0] : p.a[1];
-          const uint8_t* gb = t == 0 ? p.b[0] : p.b[1];
-          for (int kc = 0; kc < nkc; ++kc, ++req) {
+        const int n = tile_of(tl);
+        for (int t = 0; t < nacc && !bad; ++t) {
+          const int c0 = chunk0(tl, t), c1 = c0 + chunks(tl, t), q = ATOM ? 0 : t, nks = p.nks[q];
+          const uint8_t *ga = p.a[q], *gb = p.b[q];
+          for (int kc = c0; kc < c1; ++kc, ++req) {
             const int st = req % PF_NST;
             if (req >= PF_NST &&
                 !tc::mbar_wait_fast(&empty[st], ((req - PF_NST) / PF_NST) & 1, stop)) {
@@ -1517,11 +1531,12 @@ __global__ void __launch_bounds__(PP_NTHR, 1) k_pf_tc(const PFArgs p) {
       bool bad = false;
       for (int tl = 0; tl < ntl && !bad; ++tl) {
         const int acc = tl & 1;
-        for (int t = 0; t < ntyp && !bad; ++t) {
-          const int nkc = t == 0 ? nkc0 : nkc1, nks = t == 0 ? p.nks[0] : p.nks[1];
-          for (int kc = 0; kc < nkc; ++kc, ++it) {
+        for (int t = 0; t < nacc && !bad; ++t) {
+          const int c0 = chunk0(tl, t), c1 = c0 + chunks(tl, t), nks = p.nks[ATOM ? 0 : t];
+          const bool last = t == nacc - 1 || (ATOM && c1 == nkc0);
+          for (int kc = c0; kc < c1; ++kc, ++it) {
             const int st = it % PF_NST;
-            if (t == 0 && kc == 0 && tl >= 2) {  // accumulator pair acc read back (tile tl - 2)
+            if (t == 0 && kc == c0 && tl >= 2) {  // accumulator pair acc read back (tile tl - 2)
               if (!tc::mbar_wait_fast(&tfree[acc], ((tl - 2) >> 1) & 1, stop)) {
                 bad = true;
                 break;
@@ -1542,12 +1557,12 @@ __global__ void __launch_bounds__(PP_NTHR, 1) k_pf_tc(const PFArgs p) {
                 const int la = q == 0 ? 1 : 0, lb = q == 1 ? 1 : 0;  // (m, h), (h, m), (h, h)
                 const uint64_t da = tc::smem_desc_kmajor(a0 + s * STEP_H + la * TILE_B, 128, 256);
                 const uint64_t db = tc::smem_desc_kmajor(b0 + s * STEP_H + lb * TILE_B, 128, 256);
-                const bool zero = kc == 0 && s == 0 && q == 0;
+                const bool zero = kc == c0 && s == 0 && q == 0;
                 tc::mma_bf16(d, da, db, IDESC_H, zero ? 0u : 1u);
               }
             }
             tc::commit(&empty[st]);
-            if (t == ntyp - 1 && kc == nkc - 1) tc::commit(&gfull[acc]);
+            if (last && kc == c1 - 1) tc::commit(&gfull[acc]);
           }
         }
       }
@@ -1580,8 +1595,8 @@ __global__ void __launch_bounds__(PP_NTHR, 1) k_pf_tc(const PFArgs p) {
         break;
       }
       tc::fence_after_sync();
-      const int n = blockIdx.x + tl * gridDim.x;
-      const int pt0 = (n * ROWS + 32 * (warp >> 2)) >> 1;  // 16 points
+      const bool two = chunks(tl, 1) > 0;
+      const int pt0 = (tile_of(tl) * ROWS + 32 * (warp >> 2)) >> 1;  // 16 points
       float f = 0.f;
 #pragma unroll
       for (int hf = 0; hf < 2; ++hf) {  // 8 points (16 columns) at a time
@@ -1601,8 +1616,18 @@ __global__ void __launch_bounds__(PP_NTHR, 1) k_pf_tc(const PFArgs p) {
           d[e] = (live && p8 + e < p.npts) ? __ldg(dyp + p8 + e) : make_float2(0.f, 0.f);
 #pragma unroll
         for (int e = 0; e < 8; ++e) z[e] = __ldg(Tz + (long long)k[e].y * p.natm);
+        const uint32_t col = tbase + tlanes + (uint32_t)(2 * acc * ROWS + 32 * (warp >> 2) + 16 * hf);
         uint32_t v[16];
-        tc::tmem_ld16(tbase + tlanes + (uint32_t)(2 * acc * ROWS + 32 * (warp >> 2) + 16 * hf), v);
+        tc::tmem_ld16(col, v);
+        if (two)
+#pragma unroll
+          for (int h = 0; h < 16; h += 8) {
+            uint32_t u[8];
+            tc::tmem_ld8u(col + ROWS + h, u);
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+              v[h + e] = __float_as_uint(__uint_as_float(v[h + e]) + __uint_as_float(u[e]));
+          }
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
           const float qx = __uint_as_float(v[2 * e]), qy = __uint_as_float(v[2 * e + 1]);

@@ -318,3 +318,36 @@ def test_other_atom_count_after_set_nonlocal_is_refused():
             assert float(ctx.ees_nonlocal(psi, occ)[1][7]) == e0
     finally:
         ctx.close()
+
+
+def test_mixed_atom_forces_do_not_lose_with_states():
+    """Mixed atom forces at 256 states, where one accumulator takes the whole sum over
+    the states, and at 257, 512, 513 and 1030, where two, a full pair and further
+    pairs do: an accumulator never takes more than 256, so the relative error
+    against FP64 stays that of 256 states.  144 force components scatter an error's
+    norm by 1 / sqrt(288) = 6 %, a ratio of two by 8 %: at most 1.3."""
+    if not cuda_ok():
+        pytest.skip("no CUDA device")
+    import torch
+    from openatom_b200.context import StepContext
+    from openatom_b200.system import System
+    s = System(12.0, 25.0, 8, {"O": 16, "H": 32}, nfft=40, seed=5)
+    g = torch.Generator(device="cuda").manual_seed(4)
+    psi = torch.view_as_complex(torch.randn((1030, s.layout.npts, 2), generator=g,
+                                            dtype=torch.float64, device="cuda"))
+    psi /= 8.0  # the mixed operands' FP16 levels hold |psi| < 4 (else a device error)
+    err = {}
+    for states in (256, 257, 512, 513, 1030):
+        occ = torch.ones(states, dtype=torch.float64, device="cuda")
+        f = []
+        for precision in ("mixed", "fp64"):
+            ctx = StepContext(s.layout, states, precision=precision)
+            try:
+                ctx.set_atoms(s)
+                ctx.set_nonlocal(s)
+                f.append(ctx.ees_nonlocal(psi[:states], occ)[2].cpu().numpy())
+                assert ctx.device_errors() == 0
+            finally:
+                ctx.close()
+        err[states] = np.linalg.norm(f[0] - f[1]) / np.linalg.norm(f[1])
+    assert max(err.values()) <= 1.3 * err[256], err
