@@ -1445,7 +1445,9 @@ struct PFArgs {
 // at 128 states, 3.0e-6 at 256, 3.7e-6 at 512, 4.9e-6 at 1024), so an accumulator
 // takes 256 states: two of them, the pair that the two types have in the psi force,
 // make a tile, and the epilogue, linear in G, runs once per 512 states.
-template <bool ATOM>
+// MANY: more than 256 (192 atoms at 128 states: 25 us of the pass faster without the
+// tile arithmetic and the second accumulator).
+template <bool ATOM, bool MANY = false>
 __global__ void __launch_bounds__(PP_NTHR, 1) k_pf_tc(const PFArgs p) {
   extern __shared__ uint8_t dsm[];
   __shared__ uint64_t full[PF_NST], empty[PF_NST], gfull[2], tfree[2];
@@ -1459,20 +1461,20 @@ __global__ void __launch_bounds__(PP_NTHR, 1) k_pf_tc(const PFArgs p) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int m = blockIdx.y;
   const int ntyp = ATOM ? 1 : p.ntyp;
-  const int nacc = ATOM ? 2 : ntyp;                                  // accumulators of a tile
+  const int nacc = MANY ? 2 : ntyp;                                  // accumulators of a tile
   const int nkc0 = (p.nks[0] + PF_KS - 1) / PF_KS;                   // K chunks per tile, type 0
   const int nkc1 = ntyp > 1 ? (p.nks[1] + PF_KS - 1) / PF_KS : 0;    // type 1
-  // this CTA's point tiles: blockIdx.x, + gridDim.x, ...; ATOM: each nseg times, 2 PF_FOLD
+  // this CTA's point tiles: blockIdx.x, + gridDim.x, ...; MANY: each nseg times, 2 PF_FOLD
   // chunks of states at a time
   const int npt = p.ntile > (int)blockIdx.x ? (p.ntile - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
-  const int nseg = ATOM ? (nkc0 + 2 * PF_FOLD - 1) / (2 * PF_FOLD) : 1;
+  const int nseg = MANY ? (nkc0 + 2 * PF_FOLD - 1) / (2 * PF_FOLD) : 1;
   const int ntl = npt * nseg;
   const int nitem = npt * (nkc0 + nkc1);
-  auto tile_of = [&](int tl) { return (int)blockIdx.x + (ATOM ? tl / nseg : tl) * (int)gridDim.x; };
+  auto tile_of = [&](int tl) { return (int)blockIdx.x + (MANY ? tl / nseg : tl) * (int)gridDim.x; };
   // first chunk and chunks of accumulator t of tile tl
-  auto chunk0 = [&](int tl, int t) { return ATOM ? (2 * (tl % nseg) + t) * PF_FOLD : 0; };
+  auto chunk0 = [&](int tl, int t) { return MANY ? (2 * (tl % nseg) + t) * PF_FOLD : 0; };
   auto chunks = [&](int tl, int t) {
-    return ATOM ? max(0, min(PF_FOLD, nkc0 - chunk0(tl, t))) : (t == 0 ? nkc0 : nkc1);
+    return MANY ? max(0, min(PF_FOLD, nkc0 - chunk0(tl, t))) : (t == 0 ? nkc0 : nkc1);
   };
 
   if (warp == 0) tc::tmem_alloc(&tslot, PF_TMEM_COLS);
@@ -1533,7 +1535,7 @@ __global__ void __launch_bounds__(PP_NTHR, 1) k_pf_tc(const PFArgs p) {
         const int acc = tl & 1;
         for (int t = 0; t < nacc && !bad; ++t) {
           const int c0 = chunk0(tl, t), c1 = c0 + chunks(tl, t), nks = p.nks[ATOM ? 0 : t];
-          const bool last = t == nacc - 1 || (ATOM && c1 == nkc0);
+          const bool last = t == nacc - 1 || (MANY && c1 == nkc0);
           for (int kc = c0; kc < c1; ++kc, ++it) {
             const int st = it % PF_NST;
             if (t == 0 && kc == c0 && tl >= 2) {  // accumulator pair acc read back (tile tl - 2)
@@ -1595,7 +1597,7 @@ __global__ void __launch_bounds__(PP_NTHR, 1) k_pf_tc(const PFArgs p) {
         break;
       }
       tc::fence_after_sync();
-      const bool two = chunks(tl, 1) > 0;
+      const bool two = MANY && chunks(tl, 1) > 0;
       const int pt0 = (tile_of(tl) * ROWS + 32 * (warp >> 2)) >> 1;  // 16 points
       float f = 0.f;
 #pragma unroll
@@ -2128,10 +2130,10 @@ int ees_tc_atom_force(cpstep_ctx* c, int ntyp, const EesForceType* ty, const int
   pf.kw = kw;
   pf.fpart = fpart;
   pf.err = c->d_dev_err;
-  CPSTEP_CUDA_TRY(cudaFuncSetAttribute(k_pf_tc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       PF_BYTES));
+  auto kern = nks > PF_FOLD * PF_KS ? k_pf_tc<true, true> : k_pf_tc<true, false>;
+  CPSTEP_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PF_BYTES));
   *nblk = ees_af_blocks(c, na);
-  k_pf_tc<true><<<dim3(*nblk, tm), PP_NTHR, PF_BYTES, c->stream>>>(pf);
+  kern<<<dim3(*nblk, tm), PP_NTHR, PF_BYTES, c->stream>>>(pf);
   CPSTEP_LAUNCH_CHECK();
   return CPSTEP_OK;
 }
