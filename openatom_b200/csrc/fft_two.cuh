@@ -96,7 +96,10 @@ __device__ __forceinline__ void rdft(cplx<T> (&v)[R]) {
 // ---- shapes -----------------------------------------------------------------
 // P, Q; G row pairs per warp and round; W warps per block; YS row splits of the
 // density pass (its FP64 accumulators of a 200 x 200 plane exceed a register
-// file: three blocks take a third of the rows each and repeat the columns)
+// file: three blocks take a third of the rows each and repeat the columns).
+// Of the factorings of a size the FP32 error decides before the time: 40 = 10 x 4 had a
+// V.psi error of 3.05e-8 where the one-stage passes have 2.90e-8, 8 x 5 3.19e-8, 4 x 10
+// 3.54e-8, 5 x 8 2.72e-8 (64 states, density + V.psi: 101 us as 10 x 4, 97 as 5 x 8).
 template <int N> struct TwoCfg { static constexpr bool ok = false; };
 #define CPSTEP_TWO(N_, P_, Q_, G_, W_, YS_)                                     \
   template <> struct TwoCfg<N_> {                                              \
@@ -105,7 +108,7 @@ template <int N> struct TwoCfg { static constexpr bool ok = false; };
   }
 CPSTEP_TWO(28, 7, 4, 8, 2, 1);
 CPSTEP_TWO(32, 8, 4, 8, 2, 1);
-CPSTEP_TWO(40, 10, 4, 8, 3, 1);
+CPSTEP_TWO(40, 5, 8, 4, 5, 1);
 CPSTEP_TWO(42, 7, 6, 4, 6, 1);
 CPSTEP_TWO(48, 8, 6, 4, 6, 1);
 CPSTEP_TWO(60, 10, 6, 5, 6, 1);

@@ -267,3 +267,41 @@ def test_line_and_real_passes_match_oracle(grid, box, states, precision):
         assert relerr(out, OF.state_r_to_g(f.cpu().numpy(), olay)) < TOL[precision]
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("grid,box,ecut,vpsi,density", [
+    (28, 8.0, 18.0, 1.937e-08, 8.421e-08), (32, 8.0, 24.0, 2.624e-08, 1.545e-07),
+    (40, 8.7, 45.0, 1.938e-08, 1.020e-07), (42, 9.0, 45.0, 2.518e-08, 1.186e-07),
+    (48, 10.4, 45.0, 2.996e-08, 1.582e-07), (60, 13.0, 45.0, 1.868e-08, 8.599e-08),
+    (64, 13.9, 45.0, 2.937e-08, 1.833e-07), (80, 17.4, 45.0, 2.197e-08, 1.001e-07),
+    (96, 20.0, 45.0, 3.896e-08, 2.087e-07), (120, 22.0, 45.0, 1.943e-08, 9.152e-08),
+    (128, 23.5, 45.0, 2.925e-08, 1.883e-07)])
+def test_fp32_error_by_grid(grid, box, ecut, vpsi, density):
+    """Relative error of FP32 V.psi and density against an FP64 context on every
+    grid, no larger than the shuffle and Stockham line FFTs had on the same inputs
+    (the numbers given).  Some 1e5 rounding errors make up a norm, four draws: it
+    scatters by a few tenths of a percent, 1 % is allowed."""
+    if not cuda_ok():
+        pytest.skip("no CUDA device")
+    import torch
+    from openatom_b200.context import StepContext
+    from openatom_b200.layout import StateLayout
+    from openatom_b200.system import make_psi
+    lay = StateLayout(box, ecut, nfft=grid)
+    ctx = {p: StepContext(lay, 16, precision=p) for p in ("mixed", "fp64")}
+    try:
+        occ = torch.ones(16, dtype=torch.float64, device="cuda")
+        x = torch.arange(grid, dtype=torch.float64, device="cuda") * (2 * np.pi / grid)
+        c = torch.cos(x)
+        vks = -0.5 + 0.4 * (c[:, None, None] + torch.cos(2 * x)[None, :, None] * c[None, None, :])
+        e2 = np.zeros(2)
+        for seed in range(4):
+            psi = make_psi(lay, 16, seed=seed, device="cuda")
+            got, ref = ((torch.view_as_real(k.vks_psi(psi, vks, occ)[0]), k.density(psi, occ))
+                        for k in (ctx["mixed"], ctx["fp64"]))
+            e2 += [float((a - b).norm() / b.norm()) ** 2 for a, b in zip(got, ref)]
+        err = np.sqrt(e2 / 4)
+        assert (err > 0.0).all() and (err <= 1.01 * np.array([vpsi, density])).all(), err
+    finally:
+        for k in ctx.values():
+            k.close()
