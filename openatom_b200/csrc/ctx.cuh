@@ -102,6 +102,7 @@ struct StateFftOps {
   int (*nl_force)(cpstep_ctx*, const NlJob&, const double*, const double2*, int, double*);
   size_t (*nl_smem)(int nplane_x);
   int lb;  // z-lines per block of the z-passes
+  int shfl_lines;  // the lines of this size have a register-shuffle form (fft_shfl.cuh)
 };
 template <typename T, int N>
 StateFftOps statefft_ops();

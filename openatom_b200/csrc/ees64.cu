@@ -457,12 +457,29 @@ int ees64_set(cpstep_ctx* c, const std::vector<int>& order) {
   return CPSTEP_OK;
 }
 
-// Whether the G-space pass is the faster one: its work grows with atoms x
-// points, the NL-grid path's with channels x grid points (both times states).
+// Whether the G-space pass is the faster one.  Its three products cost 48 flops per
+// (atom, point, state), states and atoms padded to whole tiles, at the rates the
+// tiles reach (an estimate of the whole pass, launches included); the NL-grid form
+// a transform pair per channel and state, slower where the line length has no
+// shuffle form or a plane leaves room for one block per SM, and the stencils of
+// each atom.  ms, G-space / grid form:
+//   195 atoms, 65,736 points, NL 80^3: 1.63/0.50 with 1 state, 1.63/0.87 with 8,
+//   1.64/1.57 with 16, 1.92/2.58 with 33, 3.4/8.9 with 128; 600 atoms there, 64
+//   states: 5.6/6.0, 900 atoms 8.1/6.8
+//   405 atoms, 136,092 points, NL 96^3: 7.6/11.3 with 64
+//   771 atoms, 258,510 points, NL 120^3: 20/12.5 with 16, 29/24 with 33, 29/48 with
+//   64, 96/189 with 256
+//   27 atoms, 2,575 points, NL 28^3: 0.09/0.48 with 1
 bool ees64_faster(const cpstep_ctx* c) {
   const NlData& n = c->nl;
-  const double tg = 48.0 * n.e64_na * (double)c->npts / 28e12;
-  const double tf = 1.7e-11 * n.nchan * (double)n.nkf * n.nkf * n.nkf;
+  const int S = c->nstates, mt = e64::tile_rows(S);
+  const double rate = mt == 32 ? 1.5e13 : (mt == 64 ? 2.2e13 : 2.65e13);
+  const double rows = (double)cdiv(S, mt) * mt, atoms = 32.0 * cdiv(n.e64_na, 32);
+  const double tg = 80e-6 + 48.0 * atoms * c->npts * rows / rate;
+  const bool one = 2 * (n.ops.nl_smem(c->nplane_x) + 1024) > 228 * 1024;  // plane blocks per SM
+  const double line = (n.ops.shfl_lines ? 1.1e-11 : 1.9e-11) * (one ? 1.6 : 1.0);
+  const double tf =
+      55e-6 * n.nchan + S * (line * n.nchan * (double)n.nkf * n.nkf * n.nkf + 7e-8 * n.e64_na);
   return tg < tf;
 }
 

@@ -2379,6 +2379,7 @@ struct StateFft {
     o.g2r_add = &g2r_add;
     o.r2g = &r2g;
     o.lb = ZShape<N>::LB;
+    o.shfl_lines = ShflCfg<N>::ok;
     return o;
   }
 };

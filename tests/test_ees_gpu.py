@@ -351,3 +351,39 @@ def test_mixed_atom_forces_do_not_lose_with_states():
                 ctx.close()
         err[states] = np.linalg.norm(f[0] - f[1]) / np.linalg.norm(f[1])
     assert max(err.values()) <= 1.3 * err[256], err
+
+
+def _launches(ctx, psi, occ):
+    """Kernels of one non-local pass."""
+    from openatom_b200 import _lib
+    n0 = _lib.lib().cpstep_launch_count()
+    ctx.ees_nonlocal(psi, occ)
+    return _lib.lib().cpstep_launch_count() - n0
+
+
+@pytest.mark.parametrize("states,gspace", [(1, False), (8, False), (64, True), (128, True)])
+def test_fp64_form_follows_the_states(states, gspace):
+    """195 atoms: the G-space products pay for whole tiles of states, so few states
+    take the NL-grid form (8 states: 0.9 ms against 1.6) and many the G-space one
+    (128: 3.4 ms against 8.9).  The form is told by the kernels of a pass."""
+    if not cuda_ok():
+        pytest.skip("no CUDA device")
+    import torch
+    from openatom_b200.context import StepContext
+    from openatom_b200.system import System
+    s = System(23.5, 70.0, states, {"O": 65, "H": 130}, nfft=128, seed=5)
+    g = torch.Generator(device="cuda").manual_seed(states)
+    psi = torch.view_as_complex(torch.randn((states, s.layout.npts, 2), generator=g,
+                                            dtype=torch.float64, device="cuda"))
+    occ = torch.ones(states, dtype=torch.float64, device="cuda")
+    ctx = StepContext(s.layout, states, precision="fp64")
+    try:
+        ctx.set_atoms(s)
+        ctx.set_nonlocal(s)
+        n = _launches(ctx, psi, occ)
+        ctx.tune_set({"ees_gspace": 0})
+        ngrid = _launches(ctx, psi, occ)
+        assert ngrid > 3 * len(s.channels)  # projection, sums and force of each channel
+        assert (n < ngrid) == gspace and (gspace or n == ngrid)
+    finally:
+        ctx.close()
