@@ -2021,9 +2021,12 @@ struct StateFft {
     return false;
   }
 
-  // blocks of the density pass: the resident ones, at least four items each
-  // (a block writes a partial plane per plane it touches), within the partial
-  // buffer and the partials per plane that the reduction lists
+  // blocks of the density pass: the resident ones, with at least four items each
+  // (a block writes a partial plane per plane it touches), fewer below 16 states,
+  // whose blocks are a chain of planes on a part of the SMs (1 state: 48^3 24.8 -> 18.7
+  // us with one item instead of four, 80^3 41 -> 27, 128^3 47 -> 29; 9 states: 48^3 24.8
+  // -> 22.8 with two; 24 states 27.9 with four, 30.0 with one or two), within the
+  // partial buffer and the partials per plane that the reduction lists
   static int two_density(cpstep_ctx* c, const FftJob& j, const double* occ, double* rho) {
     if constexpr (two_built) {
       constexpr int YS = TwoCfg<N>::YS;
@@ -2034,7 +2037,8 @@ struct StateFft {
         return rc;
       const long long items = (long long)N * c->nstates;
       int nb = std::max(1, c->two_blocks[0] / YS);
-      nb = (int)std::min<long long>(std::min(nb, 48 * N), std::max(1LL, items / 4));
+      const long long least = std::max(1, std::min(4, c->nstates / 4));
+      nb = (int)std::min<long long>(std::min(nb, 48 * N), std::max(1LL, items / least));
       auto segs = [&](int b) {
         return (int)(((items + b - 1) / b + c->nstates - 1) / c->nstates) + 1;
       };
