@@ -542,13 +542,14 @@ CPSTEP_API int cpstep_ctx_set_graph(cpstep_ctx* ctx, int enable);
  * fftCache.C:252-255, are the nearest relative).  CPSTEP_NTUNE values:
  *   [0] state plane passes: register-shuffle line FFTs (1), shared-memory
  *       Stockham (0) or the two-stage line FFTs (2; in FP64 1 as well) where
- *       they exist;  [1] state plane passes: blocks about
+ *       they exist;  [1] state plane passes of forms 0 and 1: blocks about
  *       this many times the SM count;  [2] EES plane kernels: the same;
  *   [3] PairCalc overlap split-K: CTAs about this many times the SM count;
  *   [4] mixed contexts: tensor-core products (1) or FP64 (0);
- *   [5] mixed contexts on the tensor cores: the EES non-local pass in G space
- *       (1: its grid sums by Parseval as tensor-core products with separable
- *       B-spline transforms) or through the NL-grid FFTs (0).
+ *   [5] the EES non-local pass through the NL-grid FFTs (0), or (1) in G space
+ *       where that is built (at most four channels per type; FP64 contexts, and
+ *       mixed ones on the tensor cores) and, in FP64, estimated to be the faster:
+ *       its grid sums by Parseval as products with separable B-spline transforms.
  * cpstep_autotune times the candidates of each choice on the caller's psi
  * (device, nstates x npts) and occ with CUDA events and keeps the fastest;
  * ms (may be NULL, CPSTEP_NTUNE doubles) receives the best time (ms) per

@@ -101,6 +101,7 @@ struct StateFftOps {
   int (*nl_proj)(cpstep_ctx*, const NlJob&, const double*, const double2*, int, double*);
   int (*nl_force)(cpstep_ctx*, const NlJob&, const double*, const double2*, int, double*);
   size_t (*nl_smem)(int nplane_x);
+  bool (*two_runs)(const cpstep_ctx*);  // the state plane passes run in their two-stage form
   int lb;  // z-lines per block of the z-passes
   int shfl_lines;  // the lines of this size have a register-shuffle form (fft_shfl.cuh)
 };
@@ -471,6 +472,7 @@ int nl_run(cpstep_ctx* c, const double* psi, const double* occ, double* fpsi, do
            double* fatm);
 int nl_grid_reserve(cpstep_ctx* c);
 int nl_follow_atoms(cpstep_ctx* c);
+bool nl_in_gspace(const cpstep_ctx* c);  // the pass runs in G space with the knobs as they are
 // ees64.cu: the same pass of an FP64 context in G space
 int ees64_set(cpstep_ctx* c, const std::vector<int>& order);
 bool ees64_faster(const cpstep_ctx* c);

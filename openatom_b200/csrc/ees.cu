@@ -994,6 +994,8 @@ static bool nl_gmixed(const cpstep_ctx* c) {
   return c->nl.gspace_ok && c->precision == CPSTEP_PREC_MIXED && c->tc_ok && c->tune.ees_gspace;
 }
 
+bool nl_in_gspace(const cpstep_ctx* c) { return nl_gmixed(c) || nl_g64(c); }
+
 int nl_front(cpstep_ctx* c, const double* psi, const double* occ, bool forces, NlFront* h,
              bool* split) {
   *split = false;

@@ -2382,6 +2382,7 @@ struct StateFft {
     o.g2r = &g2r;
     o.g2r_add = &g2r_add;
     o.r2g = &r2g;
+    o.two_runs = [](const cpstep_ctx* c) { return two_fits(c, c->state_job()); };
     o.lb = ZShape<N>::LB;
     o.shfl_lines = ShflCfg<N>::ok;
     return o;

@@ -9,6 +9,7 @@
 // differ from the default launch choices in rounding only (another FFT form or
 // another grouping of the same sums); cpstep_tune_get / cpstep_tune_set let a
 // caller record a choice and reuse it, so runs stay reproducible.
+#include <algorithm>
 #include <vector>
 
 #include "ctx.cuh"
@@ -110,6 +111,7 @@ int cpstep_autotune(cpstep_ctx* c, const double* d_psi, const double* d_occ, dou
   const size_t nr = (size_t)c->nx * c->ny * c->nz;
   const size_t ncoef = (size_t)S * c->npts;
   double *rho = nullptr, *force = nullptr, *eke = nullptr, *smat = nullptr, *en = nullptr;
+  double* fat = nullptr;
   int rc = CPSTEP_OK;
   auto al = [&](double** p, size_t n) {
     if (!rc && cudaMalloc(p, n * sizeof(double)) != cudaSuccess) rc = CPSTEP_ERR_CUDA;
@@ -132,23 +134,41 @@ int cpstep_autotune(cpstep_ctx* c, const double* d_psi, const double* d_occ, dou
     if (c->precision == CPSTEP_PREC_MIXED) forms.push_back(2);
     rc = pick(c, &c->tune.shfl, forms, planes, &ms[0]);
   }
-  if (!rc) rc = pick(c, &c->tune.plane_waves, {1, 2, 3, 6}, planes, &ms[1]);
-  // 4, 5: the overlap product S (split-K width; tensor cores or FP64 in a mixed context)
+  // the two-stage passes fill the resident blocks whatever the knob says: it is timed
+  // as it stands there
+  if (!rc)
+    rc = c->ops.two_runs(c) ? pick(c, &c->tune.plane_waves, {c->tune.plane_waves}, planes, &ms[1])
+                            : pick(c, &c->tune.plane_waves, {1, 2, 3, 6}, planes, &ms[1]);
+  // 4: the overlap product S (split-K width)
   auto ovl = [&]() -> int {
     return pc_overlap_launch(c, d_psi, d_psi, S, S, 2 * c->npts, c->d_wpt, 1.0, 0.0, smat, S);
   };
   if (!rc) rc = pick(c, &c->tune.pc_split, {1, 2}, ovl, &ms[3]);
-  if (!rc && c->precision == CPSTEP_PREC_MIXED && c->tc_ok) rc = pick(c, &c->tc_ok, {1, 0}, ovl, &ms[4]);
-  // 6, 3: the EES pass: G space or NL-grid FFTs (mixed on the tensor cores), then
-  // the FFT path's blocks per SM if it runs
+  // the EES pass with atom forces, as a step runs it
+  if (c->nl.on) al(&fat, 3 * (size_t)std::max(1, c->atoms.natm));
+  auto ees = [&]() -> int {
+    CPSTEP_CUDA_TRY(cudaMemsetAsync(force, 0, sizeof(double) * 2 * ncoef, c->stream));
+    return nl_run(c, d_psi, d_occ, force, en, fat);
+  };
+  // 5: tensor cores or FP64 in a mixed context: the products that the choice decides,
+  // the EES pass among them (G space runs on the tensor cores only)
+  const int keep = c->tune.ees_gspace;
+  c->tune.ees_gspace = 1;
+  if (!rc && c->precision == CPSTEP_PREC_MIXED && c->tc_ok)
+    rc = pick(c, &c->tc_ok, {1, 0}, [&]() -> int {
+      if (int r = ovl()) return r;
+      if (int r = pc_backmul_launch(c, smat, S, d_psi, 2 * c->npts, force, 2 * c->npts, S, S,
+                                    2 * c->npts, 1.0, 0.0))
+        return r;
+      return c->nl.on ? ees() : CPSTEP_OK;
+    }, &ms[4]);
+  // 6, 3: G space or NL-grid FFTs where both are to be had, then the FFT path's
+  // blocks per SM if it runs
+  const bool gs = nl_in_gspace(c);
+  c->tune.ees_gspace = keep;
   if (!rc && c->nl.on) {
-    auto ees = [&]() -> int {
-      CPSTEP_CUDA_TRY(cudaMemsetAsync(force, 0, sizeof(double) * 2 * ncoef, c->stream));
-      return nl_run(c, d_psi, d_occ, force, en, nullptr);
-    };
-    const bool gs = c->nl.gspace_ok && c->precision == CPSTEP_PREC_MIXED && c->tc_ok;
     if (gs) rc = pick(c, &c->tune.ees_gspace, {1, 0}, ees, &ms[5]);
-    if (!rc && !(gs && c->tune.ees_gspace)) rc = pick(c, &c->tune.nl_blocks, {3, 6, 12}, ees, &ms[2]);
+    if (!rc && !nl_in_gspace(c)) rc = pick(c, &c->tune.nl_blocks, {3, 6, 12}, ees, &ms[2]);
   }
   if (!rc) rc = cudaStreamSynchronize(c->stream) == cudaSuccess ? CPSTEP_OK : CPSTEP_ERR_CUDA;
   cudaFree(rho);
@@ -156,6 +176,7 @@ int cpstep_autotune(cpstep_ctx* c, const double* d_psi, const double* d_occ, dou
   cudaFree(eke);
   cudaFree(smat);
   cudaFree(en);
+  cudaFree(fat);
   graph_drop(c);
   if (ms_out)
     for (int k = 0; k < CPSTEP_NTUNE; ++k) ms_out[k] = ms[k];

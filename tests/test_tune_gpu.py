@@ -59,3 +59,29 @@ def test_autotune_choices_and_step(precision):
     finally:
         ctx.close()
         ref.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_autotune_times_what_runs(precision):
+    """The non-local form is timed in both precisions; the blocks of the NL-grid
+    passes are picked only where those run, and the plane passes' block counts only
+    where a form reads them (48^3: the two-stage one does not)."""
+    if not cuda_ok():
+        pytest.skip("no CUDA device")
+    sysm, ctx, occ = _setup(precision)
+    try:
+        before = ctx.tune_get()
+        choice, ms = ctx.autotune(sysm.psi(), occ)
+        assert ms["ees_gspace"] > 0
+        if choice["ees_gspace"]:
+            assert choice["nl_blocks"] == before["nl_blocks"] and ms["nl_blocks"] == 0
+        else:
+            assert ms["nl_blocks"] > 0
+        if choice["plane_shfl"] == 2 or (precision == "fp64" and choice["plane_shfl"] == 1):
+            assert choice["plane_waves"] == before["plane_waves"]
+        # the choice that ran is not slower than the other one
+        ctx.tune_set({"ees_gspace": 0})
+        again, ms0 = ctx.autotune(sysm.psi(), occ)
+        assert again["ees_gspace"] == choice["ees_gspace"] and ms0["ees_gspace"] > 0
+    finally:
+        ctx.close()
