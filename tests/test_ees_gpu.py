@@ -152,15 +152,26 @@ def test_mixed_step_with_nonlocal(nlsys, nlstep):
     assert np.max(np.abs(f - fr)) <= 1e-5
 
 
-@pytest.mark.parametrize("states,atoms,keep", [
-    (1, {"O": 1, "H": 2}, None), (31, {"O": 3, "H": 5}, None), (33, {"O": 11, "H": 22}, None),
-    (65, {"O": 2, "H": 3}, (1, 0)), (130, {"O": 9, "H": 0}, None), (64, {"O": 16, "H": 17}, (0, 0))])
-def test_fp64_gspace_matches_grid_form(states, atoms, keep):
+def _launches(ctx, psi, occ):
+    """Kernels of one non-local pass."""
+    from openatom_b200 import _lib
+    n0 = _lib.lib().cpstep_launch_count()
+    ctx.ees_nonlocal(psi, occ)
+    return _lib.lib().cpstep_launch_count() - n0
+
+
+@pytest.mark.parametrize("states,atoms,keep,gspace", [
+    (1, {"O": 1, "H": 2}, None, True), (31, {"O": 3, "H": 5}, None, True),
+    (33, {"O": 11, "H": 22}, None, True), (65, {"O": 2, "H": 3}, (1, 0), False),
+    (65, {"O": 33, "H": 40}, (1, 0), True), (130, {"O": 9, "H": 0}, None, True),
+    (64, {"O": 16, "H": 17}, (0, 0), True)])
+def test_fp64_gspace_matches_grid_form(states, atoms, keep, gspace):
     """FP64 contexts: the G-space products against the NL-grid transforms at the
     edges of their tiles (32, 64, 128 states; 32 atoms; a ragged last point
     tile), with a type without channels or with one only, and forces added to
     what is there.  Both are FP64 sums of the same terms: 1e-11 of the largest
-    entry."""
+    entry.  `gspace`: whether choice 1 runs the G-space form (one channel and few
+    atoms do not), told by the kernels of a pass."""
     if not cuda_ok():
         pytest.skip("no CUDA device")
     import torch
@@ -174,7 +185,7 @@ def test_fp64_gspace_matches_grid_form(states, atoms, keep):
                                             dtype=torch.float64, device="cuda"))
     f0 = 0.1 * psi.flip(0).contiguous()
     occ = 1.0 + torch.arange(states, dtype=torch.float64, device="cuda") % 2
-    out = []
+    out, n = [], []
     for form in (1, 0):
         ctx = StepContext(s.layout, states, precision="fp64")
         try:
@@ -183,10 +194,12 @@ def test_fp64_gspace_matches_grid_form(states, atoms, keep):
             ctx.tune_set({"ees_gspace": form})
             f, e, fa = ctx.ees_nonlocal(psi, occ, fpsi=f0.clone())
             out.append((e[7:8].cpu().numpy(), f.cpu().numpy(), fa.cpu().numpy()))
+            n.append(_launches(ctx, psi, occ))
             f2, e2, _ = ctx.ees_nonlocal(psi, occ, fpsi=f0.clone(), forces=False)
             assert bool((f2 == f).all()) and bool((e2[7] == e[7]).all())
         finally:
             ctx.close()
+    assert (n[0] < n[1]) == gspace and (gspace or n[0] == n[1])
     for a, b in zip(*out):
         assert np.max(np.abs(b)) > 0.0
         assert np.max(np.abs(a - b)) <= 1e-11 * np.max(np.abs(b))
@@ -353,14 +366,6 @@ def test_mixed_atom_forces_do_not_lose_with_states():
     assert max(err.values()) <= 1.3 * err[256], err
 
 
-def _launches(ctx, psi, occ):
-    """Kernels of one non-local pass."""
-    from openatom_b200 import _lib
-    n0 = _lib.lib().cpstep_launch_count()
-    ctx.ees_nonlocal(psi, occ)
-    return _lib.lib().cpstep_launch_count() - n0
-
-
 @pytest.mark.parametrize("states,gspace", [(1, False), (8, False), (64, True), (128, True)])
 def test_fp64_form_follows_the_states(states, gspace):
     """195 atoms: the G-space products pay for whole tiles of states, so few states
@@ -387,3 +392,44 @@ def test_fp64_form_follows_the_states(states, gspace):
         assert (n < ngrid) == gspace and (gspace or n == ngrid)
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+def test_three_types_with_projectors(precision):
+    """Three types with projectors, two of them the same element: the mixed pass takes
+    the types two at a time, with psi's transposed levels kept from the first pair.
+    The sums are those of the two-type system in another order: FP64 to 1e-11 of the
+    largest entry, mixed to the module's 1e-5, and the mixed pass to FP64 as well."""
+    if not cuda_ok():
+        pytest.skip("no CUDA device")
+    import copy
+    import torch
+    from openatom_b200.context import StepContext
+    from openatom_b200.system import System
+    s = System(12.0, 25.0, 37, {"O": 9, "H": 20}, nfft=40, seed=5)
+    t = copy.copy(s)
+    t.typ = np.array(s.typ)
+    t.typ[np.nonzero(t.typ == 0)[0][::2]] = 2
+    t.tab = dict(s.tab)
+    for k in ("q", "vps", "gzvps"):
+        t.tab[k] = np.concatenate([s.tab[k], s.tab[k][:1]])
+    t.channels = s.channels + [dict(c, type=2) for c in s.channels if c["type"] == 0]
+    psi = s.psi()
+    occ = 1.0 + torch.arange(37, dtype=torch.float64, device="cuda") % 2
+    out = []
+    for system, prec in ((s, "fp64"), (s, precision), (t, precision)):
+        ctx = StepContext(s.layout, 37, precision=prec)
+        try:
+            ctx.set_atoms(system)
+            ctx.set_nonlocal(system)
+            f, e, fa = ctx.ees_nonlocal(psi, occ, fpsi=0.1 * psi)
+            out.append((e[7:8].cpu().numpy(), f.cpu().numpy(), fa.cpu().numpy()))
+            f2, e2, _ = ctx.ees_nonlocal(psi, occ, fpsi=0.1 * psi, forces=False)
+            assert bool((f2 == f).all()) and bool((e2[7] == e[7]).all())
+            assert ctx.device_errors() == 0
+        finally:
+            ctx.close()
+    tol = 1e-11 if precision == "fp64" else 1e-5
+    for a, b, c in zip(*out):
+        assert np.max(np.abs(c - b)) <= tol * np.max(np.abs(b)) and np.max(np.abs(b)) > 0.0
+        assert np.max(np.abs(c - a)) <= tol * np.max(np.abs(a))

@@ -140,8 +140,7 @@ def test_adjointness_of_the_two_transforms(system, ctx):
 @pytest.mark.parametrize("form", [0, 1, 2])
 def test_plane_pass_forms_match_oracle(system, form):
     """Density and V.psi in a mixed context with each plane-pass form: 0
-    shared-memory Stockham, 1 register shuffles, 2 the two-stage form of
-    fft_p16.cuh (grids 32, 64, 128; the others run form 1 there)."""
+    shared-memory Stockham, 1 register shuffles, 2 the two-stage form."""
     import torch
     from oracle import fftpath as OF
     from openatom_b200.context import StepContext
@@ -169,9 +168,9 @@ def test_plane_pass_forms_match_oracle(system, form):
 
 @pytest.mark.parametrize("form", [0, 2])
 def test_plane_pass_forms_n200(form):
-    """The 200^3 grid (the largest benchmark system's): V.psi in a mixed context
-    with the shared-memory Stockham form (0) and the two-stage 20 x 10 form of
-    fft_t20.cuh (2; the density pass runs form 0 there), against the oracle."""
+    """The 200^3 grid (the largest benchmark system's): density and V.psi in a mixed
+    context with the shared-memory Stockham form (0) and the two-stage 20 x 10 form
+    (2), against the oracle."""
     if not cuda_ok():
         pytest.skip("no CUDA device")
     import torch
@@ -211,7 +210,9 @@ def test_two_stage_planes_match_stockham(grid, box, states, precision):
     """Every grid of the two-stage P x Q passes (form 2) against the shared-memory
     Stockham passes (form 0): one state and many (blocks over several planes and
     several blocks per plane), empty and ragged rounds of line tasks.  Both are
-    transforms of the same rounding order: the oracle tests' tolerances."""
+    transforms of the same rounding order: the oracle tests' tolerances.  That form 2
+    ran is told by its other rounding; 200^3 in FP64 has no two-stage form and runs
+    form 0 both times."""
     if not cuda_ok():
         pytest.skip("no CUDA device")
     import torch
@@ -234,6 +235,9 @@ def test_two_stage_planes_match_stockham(grid, box, states, precision):
         for a, b in zip(*out):
             assert bool(torch.isfinite(a).all())
             assert relerr(a.cpu().numpy(), b.cpu().numpy()) < TOL[precision]
+        two = not (precision == "fp64" and grid == 200)
+        assert torch.equal(out[0][0], out[1][0]) != two
+        assert torch.equal(out[0][1], out[1][1]) != two
     finally:
         ctx.close()
 
