@@ -1,4 +1,4 @@
-// Two-stage line FFT for N = 16 R with R | 16 (N = 32, 64, 128): R threads
+// Two-stage line FFT for N = 16 R with R | 16 (the FP32 V.psi pass runs N = 128): R threads
 // hold one line, 16 elements each, and exchange once through a per-line
 // shared-memory scratch of N + N/16 elements.
 //

@@ -989,9 +989,9 @@ k_xy_bwd_p16(const cplx<float>* __restrict__ pen, const float* __restrict__ vks,
 // ---------------------------------------------------------------------------
 // K2 (MODE 0) and K3 (MODE 1) in the two-stage P x Q form of fft_two.cuh, over
 // the block's (plane, state) items (p16_item_start); blockIdx.y: the row split
-// of MODE 0.  MODE 0 adds occ psi^2 in FP64 registers per plane and writes one
-// partial plane per (block, plane touched) as k_xy_fwd_p16; MODE 1 as
-// k_xy_bwd_p16.
+// of MODE 0.  MODE 0 adds occ psi^2 in FP64 registers over the block's items of a
+// plane and writes one partial plane per (block, plane touched): segment q of its
+// item range at out[b segs + q], summed by k_rho_reduce_items; MODE 1 as k_xy_bwd_p16.
 template <typename T, int N, int MODE>
 __global__ void __launch_bounds__(TwoShape<T, N, MODE == 0>::THREADS, TwoShape<T, N, MODE == 0>::minb())
 k_two(const cplx<T>* __restrict__ pen, const T* __restrict__ vks, cplx<T>* __restrict__ pen_out,
@@ -2011,7 +2011,9 @@ struct StateFft {
 
   // whether the two-stage P x Q plane passes (k_two) run this size; in FP64 as form 1
   // too, whose shuffles lost on every grid (128 states of 128^3, density / V.psi:
-  // 1425/2606 against 720/1440 us)
+  // 1425/2606 against 720/1440 us).  Where a caller's own layout is so wide that a plane
+  // does not fit beside the scratch (128^3 in FP64 from about 50 planes of x), the
+  // shuffle or Stockham form runs.
   static constexpr bool two_built = TwoCfg<N>::ok && !(sizeof(T) == 8 && N == 200);
   static bool two_fits(const cpstep_ctx* c, const FftJob& j) {
     if constexpr (two_built)
@@ -2248,8 +2250,8 @@ struct StateFft {
     // N = 128 in FP32: the lane-group form of fft_p16.cuh, with V_KS in vector loads
     // (64 states: 492 us against 498 us)
     if constexpr (N == 128 && sizeof(T) == 4) {
-      const size_t smem = P16Shape<N>::bytes(j.g.nplane_x, j.g.nlines);
-      if (c->tune.shfl == 2 && smem <= 227 * 1024) {
+      if (c->tune.shfl == 2) {  // 168 KB at the widest sphere (64 planes of x, 8192 lines)
+        const size_t smem = P16Shape<N>::bytes(j.g.nplane_x, j.g.nlines);
         if (int rc = set_smem(k_xy_bwd_p16<N>, smem)) return rc;
         if (int rc = resident_blocks(c, k_xy_bwd_p16<N>, P16_THREADS, smem, &c->p16_blocks_k3))
           return rc;
@@ -2258,8 +2260,7 @@ struct StateFft {
             reinterpret_cast<cplx<float>*>(j.pen_b), j.g, tws<float>(c).x, occ, c->nstates);
         shfl_done = true;
       }
-    }
-    if (!shfl_done && two_fits(c, j)) {
+    } else if (two_fits(c, j)) {
       if (int rc = two_vpsi(c, j, vt, occ)) return rc;
       shfl_done = true;
     }
