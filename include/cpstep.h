@@ -280,8 +280,10 @@ CPSTEP_API int cpstep_dgemm(cpstep_ctx* ctx, char transa, char transb, int m, in
  * cp_lowdin.C:180-265) and the Ortho chare iteration (orthog_ctrl/ortho.C:
  * 153-269, :862-985): A = I, B = S/2, C = 3I - A B, B <- B C / 2,
  * A <- C A / 2 until rms(dA) <= tol or max_iter (reference: 1e-15, 10;
- * ortho.h:86-87).  mode bit 0: FP32 iteration followed by an FP64
- * correction that restores T^T (S/2) T = I to FP64 rounding; bit 1: scale
+ * ortho.h:86-87).  mode bit 0: for a looser tol: the iteration also stops where
+ * its update stops falling, and a correction restores T^T (S/2) T = I to FP64
+ * rounding (the iteration runs in FP64 in both modes).  tol >= 1 runs no
+ * iteration: T = A = I, scaled and corrected as the mode says.  bit 1: scale
  * by a Gershgorin bound of the spectrum first (converges for eig(S/2) >= 2,
  * where the reference's iteration diverges).  Blocks the host until done.
  * Returns CPSTEP_ERR_NOCONV (T still written) where the reference aborts.

@@ -881,10 +881,7 @@ static int ees_sep_run(cpstep_ctx* c) {
   return CPSTEP_OK;
 }
 
-// The EES pass in G space (see k_ees_sep): per type, the forward sums as one
-// tensor-core product of psi with conj(dyp) S, the glue, and the psi force as
-// one back-multiply with the same matrix.
-// the types with projectors
+// The types with projectors.
 static std::vector<int> nl_types(const cpstep_ctx* c) {
   std::vector<int> tl;
   for (int t = 0; t < c->atoms.ntyp; ++t)
@@ -892,7 +889,10 @@ static std::vector<int> nl_types(const cpstep_ctx* c) {
   return tl;
 }
 
-// The mixed pass in G space: separable transforms and S rows of every atom,
+// The mixed pass in G space (see k_ees_sep): per type the sums Z as one tensor-core
+// product of psi with conj(dyp) S, from Z the psi force as the product with the same
+// matrix and the atom forces as one with psi.  In four parts: separable transforms
+// and S rows of every atom,
 static int ees_gspace_tables(cpstep_ctx* c) {
   NlData& n = c->nl;
   const int S = c->nstates, natm = n.natm, ntyp = c->atoms.ntyp;

@@ -387,7 +387,8 @@ static int ensure(cpstep_ctx* c, double** p, size_t* have, size_t need) {
 }
 
 // T = (S/2)^(-1/2); S, T device [n][n] FP64 (symmetric, so row/column-major agree).
-// mixed: FP32 iteration + FP64 Newton step; scale: Gershgorin spectral scaling.
+// mixed: the iteration to a looser tolerance, then the correction; scale: Gershgorin
+// spectral scaling.
 int ortho_tmat(cpstep_ctx* c, const double* S, double* T, int n, int mixed, int scale,
                double tol, int max_iter, int* iters_out, double* rms_out, int check_host) {
   using namespace orth;

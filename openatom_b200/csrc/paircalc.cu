@@ -14,7 +14,9 @@
 //
 // All three run on the FP64 tensor units; the overlap is split over K (the
 // reference's numChunks K-split, pcCommManager.C:165-172) with a fixed-order
-// reduction of the partial tiles, so results are deterministic.
+// reduction of the partial tiles, so results are deterministic.  The overlap that
+// allocates nothing (cpstep_pc_overlap_noalloc) keeps its own scalar kernel,
+// k_overlap_part, whose splits fit the fixed buffer.
 #include <algorithm>
 #include <mutex>
 #include <cuda.h>
