@@ -392,6 +392,9 @@ CPSTEP_API int cpstep_gga_functional(cpstep_ctx* ctx, const double* d_rho, doubl
  *   Z' = 2 vnorm/vol occ Z (eesEnergyAtmForcRchare) -> NL R->G -> d_fpsi +=
  *   -w conj(dyp projPsiG') (eesPsiForcGspace).  d_energies[E_NL] is written,
  *   d_fatm[natm][3] (may be NULL) accumulated, d_fpsi accumulated.
+ * A later cpstep_set_atoms with as many atoms keeps the channels, for the new
+ * atoms' types; another number of atoms, or fewer types than the channels name,
+ * makes the pass and the step return CPSTEP_ERR_STATE.
  */
 CPSTEP_API int cpstep_nl_grid_size(int kmax, double scale, int n_interp);
 CPSTEP_API int cpstep_set_nonlocal(cpstep_ctx* ctx, int nkf, int n_interp, int nchan,
@@ -404,6 +407,8 @@ CPSTEP_API int cpstep_set_nonlocal(cpstep_ctx* ctx, int nkf, int n_interp, int n
  * cpstep_set_nonlocal_sf: channels as cpstep_set_nonlocal, each l = 0, m = 0,
  *   at most one per type; replaces an EES set-up (and cpstep_set_nonlocal
  *   replaces this one).  The step then adds this path's energy and forces.
+ *   Made for the atoms set at the time: other types or another number of them
+ *   make the pass and the step return CPSTEP_ERR_STATE.
  * cpstep_sf_nonlocal: for all states, d_energies[NL] = sum_s occ_s sum_a
  *   vnorm_a/vol z_a^2, d_fpsi -= sum_a z'_a S_a, d_fatm (if not NULL) += the
  *   atom forces; z'_a = 2 vnorm_a/vol z_a (no occupation factor in the
