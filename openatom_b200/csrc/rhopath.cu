@@ -991,6 +991,8 @@ int atoms_set(cpstep_ctx* c, int natm, int ntyp, const int* typ, const double* p
   cudaFree(a.ex); cudaFree(a.ey); cudaFree(a.ez); cudaFree(a.ezt); cudaFree(a.rank);
   cudaFree(a.fpart); cudaFree(a.pos);
   a = AtomData();
+  cudaFree(c->d_ion_e); cudaFree(c->d_force_atoms);  // per atom, made again on first use
+  c->d_ion_e = c->d_force_atoms = nullptr;
   if (ntyp > CPSTEP_MAX_TYPES || natm > rho::kMaxAtoms) {
     cpstep_set_error("atoms: %d types / %d atoms exceed the limits %d / %d", ntyp, natm,
                      CPSTEP_MAX_TYPES, rho::kMaxAtoms);
@@ -1049,9 +1051,8 @@ int atoms_set(cpstep_ctx* c, int natm, int ntyp, const int* typ, const double* p
   CPSTEP_LAUNCH_CHECK();
   if (!c->d_hmati) CPSTEP_CUDA_TRY(cudaMalloc(&c->d_hmati, sizeof(double) * 9));
   CPSTEP_CUDA_TRY(cudaMemcpy(c->d_hmati, c->hmati, sizeof(double) * 9, cudaMemcpyHostToDevice));
-  if ((rc = nl_follow_atoms(c))) return rc;  // the non-local pass's tables follow their types,
-  if (c->eloc.on) return eesloc_alloc(c);    // the EES form's the atoms
-  return CPSTEP_OK;
+  if (c->eloc.on && (rc = eesloc_alloc(c))) return rc;  // the EES form's tables follow the atoms,
+  return nl_follow_atoms(c);                            // the non-local pass's their types
 }
 
 static rho::Atoms atoms_view(const cpstep_ctx* c) {

@@ -50,6 +50,42 @@ def test_ion_forces_match_oracle(isys):
         ctx.close()
 
 
+def test_more_atoms_after_a_first_use(isys):
+    """set_atoms with more atoms once the per-atom scratch has been made for fewer:
+    forces and energies of the ions and of a host-buffer step are those of a context
+    that saw these atoms only."""
+    import copy
+    import ctypes
+    import torch
+    from openatom_b200 import _lib
+    from openatom_b200.context import StepContext
+    s = isys
+    few = copy.copy(s)
+    few.pos, few.typ, few.natm = s.pos[:5], s.typ[:5], 5
+    occ = torch.ones(s.nstates, dtype=torch.float64, device="cuda")
+    out = []
+    for systems in ((few, s), (s,)):
+        ctx = StepContext(s.layout, s.nstates, precision="fp64")
+        try:
+            ctx.set_cp_mass(25.0, 30.0)
+            ctx.set_constraint("ortho_t", 1.0)
+            for t in systems:
+                ctx.set_atoms(t)
+                f, e = ctx.ion_forces()
+                psi = s.psi()
+                v = torch.zeros_like(psi)
+                eh, fh = np.zeros(_lib.NENERGY), np.zeros((t.natm, 3))
+                _lib.call("cpstep_cp_step_host", ctx._h, _lib.ptr(psi), _lib.ptr(v), _lib.ptr(occ),
+                          5.0, 1, None, ctypes.c_void_p(eh.ctypes.data),
+                          ctypes.c_void_p(fh.ctypes.data))
+            out.append([f.cpu().numpy(), e[11].cpu().numpy(), eh[:9], fh])
+        finally:
+            ctx.close()
+    assert out[0][0].shape == (s.natm, 3)
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
+
+
 def test_atoms_integrate_matches_oracle_and_moves_the_context(isys):
     import torch
     from oracle import ions as OI
